@@ -17,6 +17,7 @@
 
 #include "../../include/hydroexa_gb300.h"
 #include "hx_dual.cuh"
+#include "hx_pair.cuh"
 
 namespace hx {
 

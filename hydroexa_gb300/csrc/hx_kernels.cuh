@@ -30,26 +30,40 @@ namespace hx {
 template <class T, class = void> struct InteriorFetch : std::false_type {};
 template <class T> struct InteriorFetch<T, std::void_t<decltype(T::kInterior)>> : std::bool_constant<T::kInterior> {};
 
-template <class R, int TXv = TX, int TYv = TY> struct HydroSmem {
+// V holds velocities: R, or float pairs in the FP64 fast form (TileSmem), whose slopes are then halved.
+template <class R, int TXv = TX, int TYv = TY, class V = R> struct HydroSmem {
+    static_assert(sizeof(V) == sizeof(R), "the layout does not depend on V");
     static constexpr int GX = TXv + 4, GY = TYv + 4;
-    R z[GY][GX], eta[GY][GX], u[GY][GX], v[GY][GX];
-    R sxe[TYv][TXv + 2], sxu[TYv][TXv + 2], sxv[TYv][TXv + 2];  // x-slopes of tile columns -1..TX
-    R sye[TYv + 2][TXv], syu[TYv + 2][TXv], syv[TYv + 2][TXv];  // y-slopes of tile rows -1..TY
-    R fx[4][TYv][TXv + 1];                                      // x faces: F0, FL1, FR1, F2
-    R fy[4][TYv + 1][TXv];                                      // y faces: F0, F1, FL2, FR2
+    R z[GY][GX], eta[GY][GX];
+    V u[GY][GX], v[GY][GX];
+    R sxe[TYv][TXv + 2];
+    V sxu[TYv][TXv + 2], sxv[TYv][TXv + 2];  // x-slopes of tile columns -1..TX
+    R sye[TYv + 2][TXv];
+    V syu[TYv + 2][TXv], syv[TYv + 2][TXv];  // y-slopes of tile rows -1..TY
+    // faces: mass flux, normal momentum flux seen by the lower and the upper cell, transverse momentum flux
+    V fxm[TYv][TXv + 1];
+    R fxl[TYv][TXv + 1], fxr[TYv][TXv + 1];
+    V fxt[TYv][TXv + 1];
+    V fym[TYv + 1][TXv];
+    R fyl[TYv + 1][TXv], fyr[TYv + 1][TXv];
+    V fyt[TYv + 1][TXv];
     unsigned char nod[GY][GX];                                  // NODATA predicate of each grown-tile cell
     R kc[4];  // dt/dx, dt/dy, 1/dx, 1/dy: computed once per tile, not once per cell
 };
+
+template <class R, bool FAST> constexpr bool kPairs = FAST && std::is_same_v<R, double>;
+template <class R, bool FAST, int TXv = TX, int TYv = TY>
+using TileSmem = HydroSmem<R, TXv, TYv, std::conditional_t<kPairs<R, FAST>, F2, R>>;
 
 // One hydrostatic face (src/solvers/HydrostaticRoe.cpp:218-396).  L and R are
 // the cells on either side; sX are the cells' slopes along the face normal.
 template <class R, bool FAST, int DIR, bool REC = false>
 __device__ __forceinline__ void hydro_face(bool wall, R zL, R zR, R eL, R eR, R seL, R seR, R uL, R uR, R suL, R suR,
-                                           R vL, R vR, R svL, R svR, R& F0, R& Fa, R& Fb, R& Fc,
+                                           R vL, R vR, R svL, R svR, R& Fm, R& Fl, R& Fr, R& Ft,
                                            RoeRecVals* rv = nullptr) {
     // wall: either side is NODATA (HydrostaticRoe.cpp:237-245)
     if (wall) {
-        F0 = R(0); Fa = R(0); Fb = R(0); Fc = R(0);
+        Fm = Fl = Fr = Ft = R(0);
         return;
     }
     R zf;
@@ -95,23 +109,207 @@ __device__ __forceinline__ void hydro_face(bool wall, R zL, R zR, R eL, R eR, R 
     } else {
         roe_hydrostatic_fast<R, DIR, REC>(hLs, uLf, vLf, hRs, uRf, vRf, f0, f1, f2, rv);
     }
-    // hydrostatic pressure correction, rotated with the normal
-    F0 = f0;
+    // hydrostatic pressure correction on the normal momentum
+    Fm = f0;
+    const R fn = (DIR == 0) ? f1 : f2;
+    Ft = (DIR == 0) ? f2 : f1;
     if constexpr (!FAST) {
-        const R pL = Cst<R>::half_g * (hLu * hLu - hLs * hLs);
-        const R pR = Cst<R>::half_g * (hRu * hRu - hRs * hRs);
-        if (DIR == 0) { Fa = f1 + pL; Fb = f1 + pR; Fc = f2; }
-        else { Fa = f1; Fb = f2 + pL; Fc = f2 + pR; }
+        Fl = fn + Cst<R>::half_g * (hLu * hLu - hLs * hLs);
+        Fr = fn + Cst<R>::half_g * (hRu * hRu - hRs * hRs);
     } else {
         // one add: the face-bed side's flux is the normal-momentum flux itself (adding its +0 correction
         // would change only a -0 flux into +0)
         (void)hLu;
         (void)hRu;
-        const R fn = (DIR == 0) ? f1 : f2, fw = fma(Cst<R>::half_g, pW, fn);
-        if (DIR == 0) { Fa = lhigh ? fn : fw; Fb = lhigh ? fw : fn; Fc = f2; }
-        else { Fa = f1; Fb = lhigh ? fn : fw; Fc = lhigh ? fw : fn; }
+        const R fw = fma(Cst<R>::half_g, pW, fn);
+        Fl = lhigh ? fn : fw;
+        Fr = lhigh ? fw : fn;
     }
 }
+
+// ---------------------------------------------------------------------------
+// The FP64 fast form's cell velocities, slopes and Roe flux (hx_pair.cuh).
+// ---------------------------------------------------------------------------
+// Velocities of a cell: (qx, qy) / h where h is above the division tolerance.
+template <class R> __device__ __forceinline__ void cell_velocity(R h, R qx, R qy, R& u, R& v) {
+    const R rh = gt_bits(h, Cst<R>::tol12_bits) ? rcp_nr(h) : R(0);
+    u = qx * rh;
+    v = qy * rh;
+}
+__device__ __forceinline__ void cell_velocity(double h, double qx, double qy, F2& u, F2& v) {
+    const bool wet = gt_bits(h, Cst<double>::tol12_bits);
+    F2 d = f2_of(h);
+    d.h = wet ? d.h : 1.f;
+    const float y0 = f_rcp(d.h), y = __fmaf_rn(y0, __fmaf_rn(-d.h, y0, 1.f), y0);
+    u = f2_sel(wet, f2_div(f2_of(qx), d, y));
+    v = f2_sel(wet, f2_div(f2_of(qy), d, y));
+}
+
+// Half the van Leer slope, dm dp / (dm + dp) where the differences have one sign (van_leer_slope), as
+// dm (dp / (dm + dp)): the quotient lies in (0, 1), so nothing leaves the float range.  rs, if given,
+// receives 1 / (dm + dp) (0 where the slope is 0 by a branch).
+__device__ __forceinline__ F2 half_slope_of(F2 dm, F2 dp, F2* rs) {
+    if (rs) *rs = F2{0.f, 0.f};
+    if (fabsf(dp.h) <= 1e-12f || __fmul_rn(dm.h, dp.h) <= 0.f) return F2{0.f, 0.f};
+    const F2 S = f2_add(dm, dp);
+    const float y = f_rcp(S.h);
+    if (rs) *rs = f2_rcp(S);
+    return f2_mul(dm, f2_div(dp, S, y));
+}
+__device__ __forceinline__ F2 half_slope(F2 qm, F2 q, F2 qp, F2* rs = nullptr) {
+    return half_slope_of(f2_sub(q, qm), f2_sub(qp, q), rs);
+}
+// The free surface's slope stays in FP64: the pressure that balances the bed follows from it.
+__device__ __forceinline__ double half_slope(double qm, double q, double qp, F2* rs = nullptr) {
+    if (rs) {
+        double r;
+        const double s = van_leer_slope_rs(qm, q, qp, r);
+        *rs = f2_of(r);
+        return 0.5 * s;
+    }
+    return 0.5 * van_leer_slope<double, true>(qm, q, qp);
+}
+
+// The flux of roe_hydrostatic_fast for states beyond the pair form's range (depths from 2^32 m, speeds from
+// 2^24 m/s, NaN and infinities), in FP64 throughout.  Not inlined: no ordinary face comes here.
+template <int DIR, bool REC>
+__device__ __noinline__ void roe_hydrostatic_far(double hi, double ui, double vi, double hj, double uj, double vj,
+                                                 double* F, RoeRecVals* rv) {
+    roe_hydrostatic_fast<double, DIR, REC>(hi, ui, vi, hj, uj, vj, F[0], F[1], F[2], rv);
+}
+// roe_hydrostatic_fast with velocities and every dissipation term in float pairs: the mass flux Fm, the
+// normal momentum flux Fn and the transverse one Ft (all along +x, +y).  What stays in FP64: the
+// jump dh = hj - hi, exact where the depths are close, so that the dissipation scales with it; the hydrostatic
+// pressure (g/4)(hi^2 + hj^2), which a lake at rest balances against the bed; the final sums.
+//
+// The dissipation is arranged so that nothing cancels at a high Froude number (thin fast flow, where the
+// wave strengths are large against their sum).  With Roe's averages, d(hu) = u dh + m for m = si sj du, so
+//   A = a2 + a0 = dh / 2,   B = a2 - a0 = m / (2 c)          (a0, a2: half the wave strengths)
+// and, the signs of l0 = u - c and l2 = u + c known (no entropy fix here),
+//   |l0| a0 + |l2| a2       = u P + c Q
+//   |l0| a0 l0 + |l2| a2 l2 = (u^2 + c^2) P + 2 u c Q
+// with (P, Q) = sgn(u)(A, B) for supercritical flow, where c B = m / 2 needs no division, and (B, A) for
+// subcritical flow.  The contact wave's |u| a1 c = |u| si sj dv / 2.  The reference's guards 1e-12 in the
+// denominators si + sj and 2 c enter to first order: um = u (1 - tol12 / (si + sj)), 1 / (2 c + tol12) =
+// (1 - tol12 / (2 c)) / (2 c), the second order being below 1e-18.
+//
+// Measured on the 8192^2 FP64 level: 24.6 -> 9.2 ms a step, the FP64 instructions of a cell's update 190 -> 55;
+// error of four steps against 64-bit arithmetic 8.9e-16 -> 5.8e-16 (2-norm).  A first version that kept the wave
+// strengths l2 dh - d(hu), l0 dh - d(hu) in pairs lost 2^-48 (|u| / c)^2 of thin fast flow and was 5% slower.
+template <int DIR, bool REC = false>
+__device__ __forceinline__ void roe_hydrostatic_pair(double hi, F2 ui, F2 vi, double hj, F2 uj, F2 vj, F2& Fm,
+                                                     double& Fn, F2& Ft, RoeRecVals* rv = nullptr) {
+    using C = Cst<double>;
+    const bool wi = ge_bits(hi, C::toldry_bits), wj = ge_bits(hj, C::toldry_bits);
+    hi = wi ? hi : 0.0;
+    hj = wj ? hj : 0.0;
+    const F2 uni = f2_sel(wi, DIR == 0 ? ui : vi), uti = f2_sel(wi, DIR == 0 ? vi : f2_neg(ui));
+    const F2 unj = f2_sel(wj, DIR == 0 ? uj : vj), utj = f2_sel(wj, DIR == 0 ? vj : f2_neg(uj));
+    const F2 Hi = f2_of(hi), Hj = f2_of(hj), dh = f2_of(__dadd_rn(hj, -hi));
+    float r;
+    const F2 si = f2_sqrt(Hi, r), sj = f2_sqrt(Hj, r);
+    {
+        const unsigned top = (1023u + 32u) << 20;  // depths are non-negative here; NaN and inf are above
+        const bool in = (unsigned)__double2hiint(hi) < top && (unsigned)__double2hiint(hj) < top &&
+                        fabsf(uni.h) < 0x1p24f && fabsf(uti.h) < 0x1p24f && fabsf(unj.h) < 0x1p24f &&
+                        fabsf(utj.h) < 0x1p24f;
+        // the entropy fixes, ruled out in float where a sign is certain (roe_hydrostatic_fast)
+        const float ci = __fmul_rn(3.13209195f, si.h), cj = __fmul_rn(3.13209195f, sj.h);
+        const float mi = 0x1p-16f * (fabsf(uni.h) + ci), mj = 0x1p-16f * (fabsf(unj.h) + cj);
+        const bool rule0 = (uni.h - ci >= mi) || (unj.h - cj <= -mj);
+        const bool rule2 = (uni.h + ci >= mi) || (unj.h + cj <= -mj);
+        if (!(in && rule0 && rule2)) {
+            double F[3];
+            roe_hydrostatic_far<DIR, REC>(hi, f64_of(ui), f64_of(vi), hj, f64_of(uj), f64_of(vj), F, rv);
+            Fm = f2_of(F[0]);
+            Fn = F[1 + DIR];
+            Ft = f2_of(F[2 - DIR]);
+            return;
+        }
+    }
+    const F2 hs = f2_add(Hi, Hj);
+    const bool hmb = hs.h > 2e-6f;
+    // c^2 = g hm: (g / 2)(hi + hj), floored at g toldry
+    F2 ghm = f2_mul(F2{4.905f, (float)(4.905 - (double)4.905f)}, hs);
+    if (!hmb) ghm = F2{9.81e-6f, (float)(9.81e-6 - (double)9.81e-6f)};
+    const F2 cm = f2_sqrt(ghm, r);
+    const F2 rc = f2_norm(r, __fmul_rn(r, __fmaf_rn(-cm.l, r, __fmaf_rn(-cm.h, r, 1.f))));  // 1 / cm
+    const float tc = __fmul_rn(0.5e-12f, rc.h);                                            // tol12 / (2 c)
+    const F2 rs = f2_rcp(f2_add(f2_add(si, sj), F2{1e-12f, 0.f}));
+    const F2 um = f2_mul(f2_add(f2_mul_raw(uni, si), f2_mul_raw(unj, sj)), rs);
+    const F2 vm = f2_mul(f2_add(f2_mul_raw(uti, si), f2_mul_raw(utj, sj)), rs);
+    const float ts = __fmul_rn(__fmul_rn(1e-12f, rs.h), dh.h);  // dh tol12 / (si + sj)
+    const F2 ss = f2_half(f2_mul(si, sj));
+    F2 m = f2_mul(ss, f2_sub(unj, uni)), mv = f2_mul(ss, f2_sub(utj, uti));  // halved
+    m.l = __fmaf_rn(0.5f * um.h, ts, m.l);  // the averages' guard: -(um - u) dh / 2
+    mv.l = __fmaf_rn(0.5f * vm.h, ts, mv.l);
+    F2 A = f2_half(dh), cB = m;
+    A.l = __fmaf_rn(-tc, A.h, A.l);
+    cB.l = __fmaf_rn(-tc, cB.h, cB.l);
+    // the signs of um - cm and um + cm, certain in float where they differ and irrelevant where they do not
+    const bool super = fabsf(um.h) > cm.h;
+    F2 P, cQ;
+    {
+        const F2 B = f2_mul(cB, rc), cA = f2_mul(cm, A);
+        const int s = __float_as_int(um.h) & (int)0x80000000;
+        P.h = super ? __int_as_float(__float_as_int(A.h) ^ s) : B.h;
+        P.l = super ? __int_as_float(__float_as_int(A.l) ^ s) : B.l;
+        cQ.h = super ? __int_as_float(__float_as_int(cB.h) ^ s) : cA.h;
+        cQ.l = super ? __int_as_float(__float_as_int(cB.l) ^ s) : cA.l;
+        if constexpr (REC) {
+            const F2 l0 = f2_sub(um, cm), l2 = f2_add(um, cm);
+            const float h = __fmul_rn(0.25f, rc.h);  // 1 / (4 cm + 2 tol12)
+            rv->si = f64_of(si); rv->sj = f64_of(sj); rv->cm = f64_of(cm); rv->rs = f64_of(rs);
+            rv->hrden = f64_of(f2_norm(h, __fmaf_rn(0.25f, rc.l, -__fmul_rn(h, tc))));
+            rv->hrcm = 0.5 * f64_of(rc);
+            rv->um = f64_of(um); rv->vm = f64_of(vm); rv->l0 = f64_of(l0); rv->l2 = f64_of(l2);
+            rv->a0h = 0.5 * f64_of(f2_sub(A, B)); rv->a2h = 0.5 * f64_of(f2_add(A, B));
+            rv->a1h = f64_of(f2_mul(mv, rc));
+            rv->fl = (wi ? RR_WI : 0u) | (wj ? RR_WJ : 0u) | (hmb ? RR_HM : 0u);
+        }
+    }
+    const F2 qi = f2_mul(Hi, uni), qj = f2_mul(Hj, unj);
+    const F2 w = f2_add(f2_mul_raw(um, P), cQ);
+    const F2 wl = f2_add(f2_mul_raw(f2_add(f2_mul_raw(um, um), ghm), P),
+                         f2_mul_raw(F2{um.h + um.h, um.l + um.l}, cQ));
+    const F2 d0 = f2_sub(f2_half(f2_add(qi, qj)), w);
+    const F2 d1 = f2_sub(f2_half(f2_add(f2_mul_raw(qi, uni), f2_mul_raw(qj, unj))), wl);
+    const F2 d2 = f2_sub(f2_half(f2_add(f2_mul_raw(qi, uti), f2_mul_raw(qj, utj))),
+                         f2_add(f2_mul_raw(w, vm), f2_mul_raw(f2_abs(um), mv)));
+    Fm = d0;
+    Fn = __fma_rn(0.5 * C::half_g, __fma_rn(hj, hj, __dmul_rn(hi, hi)), f64_of(d1));
+    Ft = DIR == 0 ? d2 : f2_neg(d2);
+}
+
+// hydro_face of the FP64 fast form: velocities in pairs, half slopes (seL ... svR).
+template <class R, bool FAST, int DIR, bool REC = false>
+__device__ __forceinline__ void hydro_face(bool wall, double zL, double zR, double eL, double eR, double seL,
+                                           double seR, F2 uL, F2 uR, F2 suL, F2 suR, F2 vL, F2 vR, F2 svL, F2 svR,
+                                           F2& Fm, double& Fl, double& Fr, F2& Ft, RoeRecVals* rv = nullptr) {
+    if (wall) {
+        Fm = Ft = F2{0.f, 0.f};
+        Fl = Fr = 0.0;
+        return;
+    }
+    const double etaLf = __dadd_rn(eL, seL), etaRf = __dadd_rn(eR, -seR);
+    const bool lhigh = !(okey(zL) < okey(zR));  // the left bed is the face bed: its pressure correction is +0
+    const double eH = lhigh ? etaLf : etaRf, zf = lhigh ? zL : zR;
+    const double eW = lhigh ? etaRf : etaLf, zW = lhigh ? zR : zL;
+    const double hH = max0_i(__dadd_rn(eH, -zf));
+    const double hWu = max0_i(__dadd_rn(eW, -zW)), hWs = max0_i(__dadd_rn(eW, -zf));
+    const double pW = __dmul_rn(__dadd_rn(hWu, -hWs), __dadd_rn(hWu, hWs));
+    double fn;
+    roe_hydrostatic_pair<DIR, REC>(lhigh ? hH : hWs, f2_add(uL, suL), f2_add(vL, svL), lhigh ? hWs : hH,
+                                   f2_sub(uR, suR), f2_sub(vR, svR), Fm, fn, Ft, rv);
+    const double fw = __fma_rn(Cst<double>::half_g, pW, fn);
+    Fl = lhigh ? fn : fw;
+    Fr = lhigh ? fw : fn;
+}
+// Fluxes and their differences as the update and the face arrays take them.
+template <class R> __device__ __forceinline__ R flux_of(R f) { return f; }
+__device__ __forceinline__ double flux_of(F2 f) { return f64_of(f); }
+template <class R> __device__ __forceinline__ R flux_diff(R a, R b) { return a - b; }
+__device__ __forceinline__ double flux_diff(F2 a, F2 b) { return f64_of(f2_sub(a, b)); }
 
 // dt of a step of the device time loop.  A collapse (min CFL bound < 1e-12,
 // HydrostaticRoe.cpp:77-80) is carried forward as a flag in the next
@@ -515,7 +713,7 @@ struct NoHooks {
 template <class R, bool FAST, int TXv, int TYv, int NTv, class Src, bool LINEAR = false, class Div = NoDiv,
           class Rec = NoRec, class UO = Cells3<R>, class NP = Plane<R>, class Hooks = NoHooks, class Sync = BlockSync,
           bool EPI = false>
-__device__ __forceinline__ void hydro_tile_body(HydroSmem<R, TXv, TYv>& S, const Src& src, const UO& uo,
+__device__ __forceinline__ void hydro_tile_body(TileSmem<R, FAST, TXv, TYv>& S, const Src& src, const UO& uo,
                                                 const NP& nplane, const Cells3W<R>& out, const FaceOut<R>& fo,
                                                 const IBox& vb, int x0, int y0, R dt, R dx, R dy, DtAccum* dt_out,
                                                 unsigned* status, unsigned* post_flags = nullptr,
@@ -551,12 +749,10 @@ __device__ __forceinline__ void hydro_tile_body(HydroSmem<R, TXv, TYv>& S, const
                 R hh, zz, qx, qy;
                 src.fetch_in(x0 + c - 2, y0 + r - 2, hh, zz, qx, qy);
                 const R hp = max0_i(hh);
-                const R rh = gt_bits(hp, Cst<R>::tol12_bits) ? rcp_nr(hp) : R(0);
                 S.nod[r][c] = is_nodata(zz) ? 1 : 0;
                 S.z[r][c] = zz;
                 S.eta[r][c] = hp + zz;
-                S.u[r][c] = qx * rh;
-                S.v[r][c] = qy * rh;
+                cell_velocity(hp, qx, qy, S.u[r][c], S.v[r][c]);
             }
         }
     }
@@ -573,22 +769,18 @@ __device__ __forceinline__ void hydro_tile_body(HydroSmem<R, TXv, TYv>& S, const
         } else if (src.inside(gi, gj)) {
             src.fetch(gi, gj, e, zz, qx, qy, nn);
         }
-        R hp, uu, vv;
+        R hp;
         if constexpr (!FAST) {
             hp = max0(e - zz);  // HydrostaticRoe.cpp:498
-            uu = (hp > Cst<R>::tol12) ? qx / hp : R(0);
-            vv = (hp > Cst<R>::tol12) ? qy / hp : R(0);
+            S.u[r][c] = (hp > Cst<R>::tol12) ? qx / hp : R(0);
+            S.v[r][c] = (hp > Cst<R>::tol12) ? qy / hp : R(0);
         } else {
             hp = stored ? max0_i(e) : max0_i(e - zz);
-            const R rh = gt_bits(hp, Cst<R>::tol12_bits) ? rcp_nr(hp) : R(0);
-            uu = qx * rh;
-            vv = qy * rh;
+            cell_velocity(hp, qx, qy, S.u[r][c], S.v[r][c]);
         }
         S.nod[r][c] = is_nodata(zz) ? 1 : 0;
         S.z[r][c] = zz;
         S.eta[r][c] = hp + zz;  // HydrostaticRoe.cpp:257-260
-        S.u[r][c] = uu;
-        S.v[r][c] = vv;
     }
     hooks.after_load();
     sy.bar();
@@ -597,15 +789,19 @@ __device__ __forceinline__ void hydro_tile_body(HydroSmem<R, TXv, TYv>& S, const
     auto xslopes = [&](int row, int col) {  // tile cell (col, row), col in -1..TXv
         const int r = row + 2, c = col + 2;
         if constexpr (Rec::on) {
-            double rs0, rs1, rs2;
-            const double s0 = van_leer_slope_rs(S.eta[r][c - 1], S.eta[r][c], S.eta[r][c + 1], rs0);
-            const double s1 = van_leer_slope_rs(S.u[r][c - 1], S.u[r][c], S.u[r][c + 1], rs1);
-            const double s2 = van_leer_slope_rs(S.v[r][c - 1], S.v[r][c], S.v[r][c + 1], rs2);
+            F2 rs0, rs1, rs2;
+            const double s0 = half_slope(S.eta[r][c - 1], S.eta[r][c], S.eta[r][c + 1], &rs0);
+            const F2 s1 = half_slope(S.u[r][c - 1], S.u[r][c], S.u[r][c + 1], &rs1);
+            const F2 s2 = half_slope(S.v[r][c - 1], S.v[r][c], S.v[r][c + 1], &rs2);
             S.sxe[row][col + 1] = s0; S.sxu[row][col + 1] = s1; S.sxv[row][col + 1] = s2;
             const int gi = x0 + col, gj = y0 + row;
-            rec.put_sx(col, TXv, gi, gj, 0, s0, rs0);
-            rec.put_sx(col, TXv, gi, gj, 1, s1, rs1);
-            rec.put_sx(col, TXv, gi, gj, 2, s2, rs2);
+            rec.put_sx(col, TXv, gi, gj, 0, 2.0 * s0, f64_of(rs0));
+            rec.put_sx(col, TXv, gi, gj, 1, 2.0 * f64_of(s1), f64_of(rs1));
+            rec.put_sx(col, TXv, gi, gj, 2, 2.0 * f64_of(s2), f64_of(rs2));
+        } else if constexpr (kPairs<R, FAST>) {
+            S.sxe[row][col + 1] = half_slope(S.eta[r][c - 1], S.eta[r][c], S.eta[r][c + 1]);
+            S.sxu[row][col + 1] = half_slope(S.u[r][c - 1], S.u[r][c], S.u[r][c + 1]);
+            S.sxv[row][col + 1] = half_slope(S.v[r][c - 1], S.v[r][c], S.v[r][c + 1]);
         } else {
             S.sxe[row][col + 1] = van_leer_slope<R, FAST>(S.eta[r][c - 1], S.eta[r][c], S.eta[r][c + 1]);
             S.sxu[row][col + 1] = van_leer_slope<R, FAST>(S.u[r][c - 1], S.u[r][c], S.u[r][c + 1]);
@@ -615,15 +811,19 @@ __device__ __forceinline__ void hydro_tile_body(HydroSmem<R, TXv, TYv>& S, const
     auto yslopes = [&](int row, int col) {  // row in -1..TYv
         const int r = row + 2, c = col + 2;
         if constexpr (Rec::on) {
-            double rs0, rs1, rs2;
-            const double s0 = van_leer_slope_rs(S.eta[r - 1][c], S.eta[r][c], S.eta[r + 1][c], rs0);
-            const double s1 = van_leer_slope_rs(S.u[r - 1][c], S.u[r][c], S.u[r + 1][c], rs1);
-            const double s2 = van_leer_slope_rs(S.v[r - 1][c], S.v[r][c], S.v[r + 1][c], rs2);
+            F2 rs0, rs1, rs2;
+            const double s0 = half_slope(S.eta[r - 1][c], S.eta[r][c], S.eta[r + 1][c], &rs0);
+            const F2 s1 = half_slope(S.u[r - 1][c], S.u[r][c], S.u[r + 1][c], &rs1);
+            const F2 s2 = half_slope(S.v[r - 1][c], S.v[r][c], S.v[r + 1][c], &rs2);
             S.sye[row + 1][col] = s0; S.syu[row + 1][col] = s1; S.syv[row + 1][col] = s2;
             const int gi = x0 + col, gj = y0 + row;
-            rec.put_sy(row, TYv, gi, gj, 0, s0, rs0);
-            rec.put_sy(row, TYv, gi, gj, 1, s1, rs1);
-            rec.put_sy(row, TYv, gi, gj, 2, s2, rs2);
+            rec.put_sy(row, TYv, gi, gj, 0, 2.0 * s0, f64_of(rs0));
+            rec.put_sy(row, TYv, gi, gj, 1, 2.0 * f64_of(s1), f64_of(rs1));
+            rec.put_sy(row, TYv, gi, gj, 2, 2.0 * f64_of(s2), f64_of(rs2));
+        } else if constexpr (kPairs<R, FAST>) {
+            S.sye[row + 1][col] = half_slope(S.eta[r - 1][c], S.eta[r][c], S.eta[r + 1][c]);
+            S.syu[row + 1][col] = half_slope(S.u[r - 1][c], S.u[r][c], S.u[r + 1][c]);
+            S.syv[row + 1][col] = half_slope(S.v[r - 1][c], S.v[r][c], S.v[r + 1][c]);
         } else {
             S.sye[row + 1][col] = van_leer_slope<R, FAST>(S.eta[r - 1][c], S.eta[r][c], S.eta[r + 1][c]);
             S.syu[row + 1][col] = van_leer_slope<R, FAST>(S.u[r - 1][c], S.u[r][c], S.u[r + 1][c]);
@@ -645,43 +845,36 @@ __device__ __forceinline__ void hydro_tile_body(HydroSmem<R, TXv, TYv>& S, const
 
     // --- C: faces.  The x face at the left of each cell and the y face below
     // it, then the right column and the top row. ------------------------------
+    using V = std::conditional_t<kPairs<R, FAST>, F2, R>;
     auto xface = [&](int fi, int fj) {
         const int r = fj + 2, cl = fi + 1, cr = fi + 2;
-        R F0, Fa, Fb, Fc;
+        V Fm, Ft;
+        R Fl, Fr;
         const bool wall = S.nod[r][cl] | S.nod[r][cr];
+        RoeRecVals rv;
+        hydro_face<R, FAST, 0, Rec::on>(wall, S.z[r][cl], S.z[r][cr], S.eta[r][cl], S.eta[r][cr], S.sxe[fj][fi],
+                                        S.sxe[fj][fi + 1], S.u[r][cl], S.u[r][cr], S.sxu[fj][fi], S.sxu[fj][fi + 1],
+                                        S.v[r][cl], S.v[r][cr], S.sxv[fj][fi], S.sxv[fj][fi + 1], Fm, Fl, Fr, Ft, &rv);
         if constexpr (Rec::on) {
-            RoeRecVals rv;
-            hydro_face<R, FAST, 0, true>(wall, S.z[r][cl], S.z[r][cr], S.eta[r][cl], S.eta[r][cr], S.sxe[fj][fi],
-                                         S.sxe[fj][fi + 1], S.u[r][cl], S.u[r][cr], S.sxu[fj][fi], S.sxu[fj][fi + 1],
-                                         S.v[r][cl], S.v[r][cr], S.sxv[fj][fi], S.sxv[fj][fi + 1], F0, Fa, Fb, Fc,
-                                         &rv);
             if (!wall) rec.put_x(x0 + fi, y0 + fj, rv, fi == TXv);
-        } else {
-            hydro_face<R, FAST, 0>(wall, S.z[r][cl], S.z[r][cr], S.eta[r][cl], S.eta[r][cr], S.sxe[fj][fi],
-                                   S.sxe[fj][fi + 1], S.u[r][cl], S.u[r][cr], S.sxu[fj][fi], S.sxu[fj][fi + 1],
-                                   S.v[r][cl], S.v[r][cr], S.sxv[fj][fi], S.sxv[fj][fi + 1], F0, Fa, Fb, Fc);
         }
-        S.fx[0][fj][fi] = F0; S.fx[1][fj][fi] = Fa; S.fx[2][fj][fi] = Fb; S.fx[3][fj][fi] = Fc;
-        fo.store_x(x0 + fi, y0 + fj, vb, F0, Fa, Fb, Fc, fi == TXv);
+        S.fxm[fj][fi] = Fm; S.fxl[fj][fi] = Fl; S.fxr[fj][fi] = Fr; S.fxt[fj][fi] = Ft;
+        if (fo.on || fo.mean) fo.store_x(x0 + fi, y0 + fj, vb, flux_of(Fm), Fl, Fr, flux_of(Ft), fi == TXv);
     };
     auto yface = [&](int fi, int fj) {
         const int c = fi + 2, rl = fj + 1, rr = fj + 2;
-        R F0, Fa, Fb, Fc;
+        V Fm, Ft;
+        R Fl, Fr;
         const bool wall = S.nod[rl][c] | S.nod[rr][c];
+        RoeRecVals rv;
+        hydro_face<R, FAST, 1, Rec::on>(wall, S.z[rl][c], S.z[rr][c], S.eta[rl][c], S.eta[rr][c], S.sye[fj][fi],
+                                        S.sye[fj + 1][fi], S.u[rl][c], S.u[rr][c], S.syu[fj][fi], S.syu[fj + 1][fi],
+                                        S.v[rl][c], S.v[rr][c], S.syv[fj][fi], S.syv[fj + 1][fi], Fm, Fl, Fr, Ft, &rv);
         if constexpr (Rec::on) {
-            RoeRecVals rv;
-            hydro_face<R, FAST, 1, true>(wall, S.z[rl][c], S.z[rr][c], S.eta[rl][c], S.eta[rr][c], S.sye[fj][fi],
-                                         S.sye[fj + 1][fi], S.u[rl][c], S.u[rr][c], S.syu[fj][fi], S.syu[fj + 1][fi],
-                                         S.v[rl][c], S.v[rr][c], S.syv[fj][fi], S.syv[fj + 1][fi], F0, Fa, Fb, Fc,
-                                         &rv);
             if (!wall) rec.put_y(x0 + fi, y0 + fj, rv, fj == TYv);
-        } else {
-            hydro_face<R, FAST, 1>(wall, S.z[rl][c], S.z[rr][c], S.eta[rl][c], S.eta[rr][c], S.sye[fj][fi],
-                                   S.sye[fj + 1][fi], S.u[rl][c], S.u[rr][c], S.syu[fj][fi], S.syu[fj + 1][fi],
-                                   S.v[rl][c], S.v[rr][c], S.syv[fj][fi], S.syv[fj + 1][fi], F0, Fa, Fb, Fc);
         }
-        S.fy[0][fj][fi] = F0; S.fy[1][fj][fi] = Fa; S.fy[2][fj][fi] = Fb; S.fy[3][fj][fi] = Fc;
-        fo.store_y(x0 + fi, y0 + fj, vb, F0, Fa, Fb, Fc, fj == TYv);
+        S.fym[fj][fi] = Fm; S.fyl[fj][fi] = Fl; S.fyr[fj][fi] = Fr; S.fyt[fj][fi] = Ft;
+        if (fo.on || fo.mean) fo.store_y(x0 + fi, y0 + fj, vb, flux_of(Fm), flux_of(Ft), Fl, Fr, fj == TYv);
     };
     for (int k = t; k < CELLS; k += NTv) {
         const int tx = k % TXv, ty = k / TXv;
@@ -725,12 +918,12 @@ __device__ __forceinline__ void hydro_tile_body(HydroSmem<R, TXv, TYv>& S, const
         const int tx = k % TXv, ty = k / TXv;
         const int gi = x0 + tx, gj = y0 + ty;
         if (gi > vb.hi0 || gj > vb.hi1) continue;
-        const R dx0 = S.fx[0][ty][tx + 1] - S.fx[0][ty][tx];
-        const R dx1 = S.fx[1][ty][tx + 1] - S.fx[2][ty][tx];
-        const R dx2 = S.fx[3][ty][tx + 1] - S.fx[3][ty][tx];
-        const R dy0 = S.fy[0][ty + 1][tx] - S.fy[0][ty][tx];
-        const R dy1 = S.fy[1][ty + 1][tx] - S.fy[1][ty][tx];
-        const R dy2 = S.fy[2][ty + 1][tx] - S.fy[3][ty][tx];
+        const R dx0 = flux_diff(S.fxm[ty][tx + 1], S.fxm[ty][tx]);
+        const R dx1 = S.fxl[ty][tx + 1] - S.fxr[ty][tx];
+        const R dx2 = flux_diff(S.fxt[ty][tx + 1], S.fxt[ty][tx]);
+        const R dy0 = flux_diff(S.fym[ty + 1][tx], S.fym[ty][tx]);
+        const R dy1 = flux_diff(S.fyt[ty + 1][tx], S.fyt[ty][tx]);
+        const R dy2 = S.fyl[ty + 1][tx] - S.fyr[ty][tx];
         if constexpr (Div::on) {  // the flux differences only: the update waits for dt
             div.st(gi, gj, dx0, dx1, dx2, dy0, dy1, dy2);
             continue;
@@ -793,10 +986,10 @@ template <class R, bool FAST, class Src, int TXH = TX, int TYH = TY, bool EPI = 
 __global__ void __launch_bounds__(TXH * TYH, min_ctas(TXH * TYH))
     k_hydro_tile(Src src, Cells3<R> uo, Plane<R> nplane, Cells3W<R> out, FaceOut<R> fo, IBox vb, StepCtl<R> ctl,
                  EpiOut<R> epi) {
-    static_assert(!EPI || sizeof(HydroSmem<R, TXH, TYH>) >= 4 * TXH * TYH * sizeof(double),
+    static_assert(!EPI || sizeof(TileSmem<R, FAST, TXH, TYH>) >= 4 * TXH * TYH * sizeof(double),
                   "the epilogue's block sums reuse the tile arrays");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    HydroSmem<R, TXH, TYH>& S = *reinterpret_cast<HydroSmem<R, TXH, TYH>*>(smem_raw);
+    TileSmem<R, FAST, TXH, TYH>& S = *reinterpret_cast<TileSmem<R, FAST, TXH, TYH>*>(smem_raw);
     R dt;
     if (!resolve_dt(ctl, dt)) return;
     step_bookkeeping(ctl, dt);
@@ -1039,7 +1232,7 @@ __global__ void __launch_bounds__(kPN, 1)
                     EpiOut<double> epi) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char* base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);  // 128-byte aligned
-    HydroSmem<double, kPX, kPY>& S = *reinterpret_cast<HydroSmem<double, kPX, kPY>*>(base);
+    TileSmem<double, FAST, kPX, kPY>& S = *reinterpret_cast<TileSmem<double, FAST, kPX, kPY>*>(base);
     PersistOwn* own = reinterpret_cast<PersistOwn*>(base + sizeof(HydroSmem<double, kPX, kPY>));
     PersistStaging* st = reinterpret_cast<PersistStaging*>(&S.sxe[0][0]);
     double dt = 0.0;
@@ -1156,7 +1349,7 @@ __global__ void __launch_bounds__(kPN, 1)
     k_boxlevel_persist(BoxSetSrc src, const int* __restrict__ tiles, int ntiles, StepCtl<double> ctl) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char* base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);  // 128-byte aligned
-    HydroSmem<double, kPX, kPY>& S = *reinterpret_cast<HydroSmem<double, kPX, kPY>*>(base);
+    TileSmem<double, FAST, kPX, kPY>& S = *reinterpret_cast<TileSmem<double, FAST, kPX, kPY>*>(base);
     PersistOwn* own = reinterpret_cast<PersistOwn*>(base + sizeof(HydroSmem<double, kPX, kPY>));
     PersistStaging* st = reinterpret_cast<PersistStaging*>(&S.sxe[0][0]);
     double dt;
@@ -1256,7 +1449,7 @@ template <class R, bool FAST, int TXH = TX, int TYH = TY>
 __global__ void __launch_bounds__(TXH * TYH, min_ctas(TXH * TYH))
     k_hydro_div(LevelSrc<R> src, Cells3<R> uo, Plane<R> nplane, DivOut<R> div, IBox vb, R dx, R dy) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    HydroSmem<R, TXH, TYH>& S = *reinterpret_cast<HydroSmem<R, TXH, TYH>*>(smem_raw);
+    TileSmem<R, FAST, TXH, TYH>& S = *reinterpret_cast<TileSmem<R, FAST, TXH, TYH>*>(smem_raw);
     FaceOut<R> fo{};
     Cells3W<R> none{};
     hydro_tile_body<R, FAST, TXH, TYH, TXH * TYH, LevelSrc<R>, false, DivOut<R>>(
@@ -1296,7 +1489,7 @@ __global__ void __launch_bounds__(NT) k_hydro_update(Cells3<R> uo, DivOut<R> div
 template <bool FAST>
 __global__ void __launch_bounds__(NT) k_boxlevel_hydro(BoxSetSrc base, const int* tiles, StepCtl<double> ctl) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    HydroSmem<double>& S = *reinterpret_cast<HydroSmem<double>*>(smem_raw);
+    TileSmem<double, FAST>& S = *reinterpret_cast<TileSmem<double, FAST>*>(smem_raw);
     double dt;
     if (!resolve_dt(ctl, dt)) return;
     step_bookkeeping(ctl, dt);
@@ -1418,15 +1611,15 @@ __global__ void __launch_bounds__(NT, 4) k_ensemble_hydro(const EnsInstance<R>* 
         DtAccum* dout = &I.slots[(step + 1) % 3];
         switch (I.shape) {
             case HX_TILE_16x16:
-                hydro_tile_body<R, FAST, 16, 16, NT>(*reinterpret_cast<HydroSmem<R, 16, 16>*>(smem_raw), src, uo, np,
+                hydro_tile_body<R, FAST, 16, 16, NT>(*reinterpret_cast<TileSmem<R, FAST, 16, 16>*>(smem_raw), src, uo, np,
                                                      out, fo, vb, bx * 16, by * 16, dt, I.dx, I.dy, dout, I.status);
                 break;
             case HX_TILE_64x4:
-                hydro_tile_body<R, FAST, 64, 4, NT>(*reinterpret_cast<HydroSmem<R, 64, 4>*>(smem_raw), src, uo, np,
+                hydro_tile_body<R, FAST, 64, 4, NT>(*reinterpret_cast<TileSmem<R, FAST, 64, 4>*>(smem_raw), src, uo, np,
                                                     out, fo, vb, bx * 64, by * 4, dt, I.dx, I.dy, dout, I.status);
                 break;
             default:
-                hydro_tile_body<R, FAST, 32, 8, NT>(*reinterpret_cast<HydroSmem<R, 32, 8>*>(smem_raw), src, uo, np,
+                hydro_tile_body<R, FAST, 32, 8, NT>(*reinterpret_cast<TileSmem<R, FAST, 32, 8>*>(smem_raw), src, uo, np,
                                                     out, fo, vb, bx * 32, by * 8, dt, I.dx, I.dy, dout, I.status);
         }
     }
@@ -1465,7 +1658,7 @@ __global__ void __launch_bounds__(32 * 32, 1) k_ensemble_big(const EnsInstance<R
         FaceOut<R> fo{};
         fo.on = 0;
         const IBox vb{0, 0, I.nx - 1, I.ny - 1};
-        hydro_tile_body<R, FAST, 32, 32, 32 * 32>(*reinterpret_cast<HydroSmem<R, 32, 32>*>(smem_raw), src, uo, np,
+        hydro_tile_body<R, FAST, 32, 32, 32 * 32>(*reinterpret_cast<TileSmem<R, FAST, 32, 32>*>(smem_raw), src, uo, np,
                                                    out, fo, vb, bx * 32, by * 32, dt, I.dx, I.dy,
                                                    &I.slots[(step + 1) % 3], I.status);
     }
@@ -1789,7 +1982,15 @@ __global__ void k_points(int method, long n, const R* __restrict__ st, const R* 
         } else {
             const R ui = q[0] > R(0) ? q[1] / q[0] : R(0), vi = q[0] > R(0) ? q[2] / q[0] : R(0);
             const R uj = q[3] > R(0) ? q[4] / q[3] : R(0), vj = q[3] > R(0) ? q[5] / q[3] : R(0);
-            if (ydir) roe_hydrostatic_fast<R, 1>(q[0], ui, vi, q[3], uj, vj, f0, f1, f2);
+            if constexpr (kPairs<R, FAST>) {
+                F2 m, t;
+                R fn;
+                if (ydir) roe_hydrostatic_pair<1>(q[0], f2_of(ui), f2_of(vi), q[3], f2_of(uj), f2_of(vj), m, fn, t);
+                else roe_hydrostatic_pair<0>(q[0], f2_of(ui), f2_of(vi), q[3], f2_of(uj), f2_of(vj), m, fn, t);
+                f0 = f64_of(m);
+                f1 = ydir ? f64_of(t) : fn;
+                f2 = ydir ? fn : f64_of(t);
+            } else if (ydir) roe_hydrostatic_fast<R, 1>(q[0], ui, vi, q[3], uj, vj, f0, f1, f2);
             else roe_hydrostatic_fast<R, 0>(q[0], ui, vi, q[3], uj, vj, f0, f1, f2);
         }
         out[3 * p] = f0; out[3 * p + 1] = f1; out[3 * p + 2] = f2;
@@ -1815,7 +2016,7 @@ __global__ void __launch_bounds__(AX * AY, min_ctas(AX * AY)) k_adj_forward(Leve
                                                      Cells3W<double> out, IBox vb, StepCtl<double> ctl,
                                                      const double* dt_fixed, unsigned* post_flags, AdjRecord rec) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    HydroSmem<double, AX, AY>& S = *reinterpret_cast<HydroSmem<double, AX, AY>*>(smem_raw);
+    TileSmem<double, FAST, AX, AY>& S = *reinterpret_cast<TileSmem<double, FAST, AX, AY>*>(smem_raw);
     double dt;
     if (dt_fixed) {
         dt = *dt_fixed;
@@ -1842,7 +2043,7 @@ __global__ void __launch_bounds__(AX * AY, min_ctas(AX * AY)) k_adj_forward_rec(
                                                          Cells3W<double> out, IBox vb, double dx, double dy,
                                                          const double* dt_fixed, unsigned* post_flags, FaceRec rec) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    HydroSmem<double, AX, AY>& S = *reinterpret_cast<HydroSmem<double, AX, AY>*>(smem_raw);
+    TileSmem<double, FAST, AX, AY>& S = *reinterpret_cast<TileSmem<double, FAST, AX, AY>*>(smem_raw);
     FaceOut<double> fo{};
     fo.on = 0;
     static_assert(FAST, "face records are kept for the fast form");
@@ -1856,7 +2057,7 @@ __global__ void __launch_bounds__(AX * AY, min_ctas(AX * AY)) k_adj_forward_line
                                                             Cells3W<double> out, IBox vb, double dx, double dy,
                                                             const double* dt_fixed) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    HydroSmem<double, AX, AY>& S = *reinterpret_cast<HydroSmem<double, AX, AY>*>(smem_raw);
+    TileSmem<double, FAST, AX, AY>& S = *reinterpret_cast<TileSmem<double, FAST, AX, AY>*>(smem_raw);
     FaceOut<double> fo{};
     fo.on = 0;
     hydro_tile_body<double, FAST, AX, AY, AX * AY, LevelSrc<double>, true>(

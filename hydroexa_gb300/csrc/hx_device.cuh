@@ -17,6 +17,7 @@
 
 #include "../../include/hydroexa_gb300.h"
 #include "hx_dual.cuh"
+#include "hx_ieee.cuh"
 #include "hx_pair.cuh"
 
 namespace hx {
@@ -171,6 +172,23 @@ __host__ __device__ __forceinline__ int okey(float x) {
 template <class R> __host__ __device__ __forceinline__ R smax_i(R a, R b) { return okey(a) < okey(b) ? b : a; }
 // max of two non-negative values
 template <class R> __host__ __device__ __forceinline__ R nnmax_i(R a, R b) { return sbits(a) < sbits(b) ? b : a; }
+
+// Comparisons of the exact form on the integer pipe, NaN included: false for a NaN, as the FP64 comparison is.
+// x >= c for c > 0, x > 0, and (0 < x) ? x : 0 (max0).
+__device__ __forceinline__ bool ge_num(double x, long long cb) {
+    return (unsigned long long)(sbits(x) - cb) <= (unsigned long long)(0x7FF0000000000000ll - cb);
+}
+__device__ __forceinline__ double max0_num(double x) { return ge_num(x, 1ll) ? x : 0.0; }
+
+// Division and square root of the exact form: IEEE rounded, for doubles off the FP64 pipe (hx_ieee.cuh).
+template <class R> __device__ __forceinline__ R ieee_quot(R a, R b) {
+    if constexpr (sizeof(R) == 8) return ieee_div(a, b);
+    else return a / b;
+}
+template <class R> __device__ __forceinline__ R ieee_root(R x) {
+    if constexpr (sizeof(R) == 8) return ieee_sqrt(x);
+    else return sqrt(x);
+}
 
 // The double holding a normal float exactly, built on the integer pipe.
 __host__ __device__ __forceinline__ double f64_widen(float f) {
@@ -368,6 +386,22 @@ __device__ __forceinline__ double van_leer_div2(double p, double S) {
     const double s0 = ok ? f64_of_f32_scaled(hf, ks + 1, sg) : 0.0;
     const double t = fma(-s0h, S, p);  // p - s0h S
     return fma(r2, t, s0);
+}
+
+// Half of it, p / S, by the same steps.
+__device__ __forceinline__ double van_leer_half_div(double p, double S) {
+    const unsigned hp = (unsigned)__double2hiint(p), lp = (unsigned)__double2loint(p);
+    const unsigned hS = (unsigned)__double2hiint(S), lS = (unsigned)__double2loint(S);
+    const int ep = (int)((hp >> 20) & 0x7FFu), eS = (int)((hS >> 20) & 0x7FFu);
+    const float mp = __int_as_float((int)(0x3F800000u | ((hp & 0xFFFFFu) << 3) | (lp >> 29)));
+    const float mS = __int_as_float((int)(0x3F800000u | ((hS & 0xFFFFFu) << 3) | (lS >> 29)));
+    const float rf = f_rcp(mS), hf = mp * rf;
+    const unsigned sg = hS & 0x80000000u;
+    const double r = f64_of_f32_scaled(rf, 1023 - eS, sg);
+    const int ks = ep - eS;
+    const bool ok = (ep != 0) & ((int)((unsigned)__float_as_int(hf) >> 23) + 896 + ks >= 1);
+    const double s0 = ok ? f64_of_f32_scaled(hf, ks, sg) : 0.0;
+    return __fma_rn(r, __fma_rn(-s0, S, p), s0);
 }
 
 // ----------------------------------------------------------------------------
@@ -800,11 +834,11 @@ __device__ __forceinline__ void dt_cell_contrib(R h, R hu, R hv, bool nod, R dx,
     if (nod) { flags |= DTF_NODATA; return; }
     if constexpr (!FAST) {
         if (!(h > Cst<R>::tol12)) { flags |= DTF_DRY; return; }
-        const R u = hu / h, v = hv / h;
-        const R c = sqrt(Cst<R>::g * h);
+        const R u = ieee_quot(hu, h), v = ieee_quot(hv, h);
+        const R c = ieee_root(Cst<R>::g * h);
         const R sx = fabs(u) + c;
         const R sy = fabs(v) + c;
-        rate = sx / dx + sy / dy;
+        rate = ieee_quot(sx, dx) + ieee_quot(sy, dy);
         mv = smax(fabs(u), fabs(v));
     } else {
         if (!gt_bits(h, Cst<R>::tol12_bits)) { flags |= DTF_DRY; return; }

@@ -50,6 +50,15 @@ template <class R, int TXv = TX, int TYv = TY, class V = R> struct HydroSmem {
     unsigned char nod[GY][GX];                                  // NODATA predicate of each grown-tile cell
     R kc[4];  // dt/dx, dt/dy, 1/dx, 1/dy: computed once per tile, not once per cell
 };
+template <class R, bool FAST> constexpr bool kIeee = !FAST && std::is_same_v<R, double>;
+// In the exact FP64 form the fluxes are kept doubled (hydro_face_ieee), so dt/dx and dt/dy are halved.
+template <class R, bool FAST> __device__ __forceinline__ void tile_constants(R* kc, R dt, R dx, R dy) {
+    constexpr R F = kIeee<R, FAST> ? R(0.5) : R(1);
+    kc[0] = F * (dt / dx);
+    kc[1] = F * (dt / dy);
+    kc[2] = R(1) / dx;
+    kc[3] = R(1) / dy;
+}
 
 template <class R, bool FAST> constexpr bool kPairs = FAST && std::is_same_v<R, double>;
 template <class R, bool FAST, int TXv = TX, int TYv = TY>
@@ -147,27 +156,35 @@ __device__ __forceinline__ void cell_velocity(double h, double qx, double qy, F2
 
 // Half the van Leer slope, dm dp / (dm + dp) where the differences have one sign (van_leer_slope), as
 // dm (dp / (dm + dp)): the quotient lies in (0, 1), so nothing leaves the float range.  rs, if given,
-// receives 1 / (dm + dp) (0 where the slope is 0 by a branch).
-__device__ __forceinline__ F2 half_slope_of(F2 dm, F2 dp, F2* rs) {
-    if (rs) *rs = F2{0.f, 0.f};
-    if (fabsf(dp.h) <= 1e-12f || __fmul_rn(dm.h, dp.h) <= 0.f) return F2{0.f, 0.f};
-    const F2 S = f2_add(dm, dp);
-    const float y = f_rcp(S.h);
-    if (rs) *rs = f2_rcp(S);
-    return f2_mul(dm, f2_div(dp, S, y));
-}
+// receives 1 / (dm + dp) (0 where the slope is 0 by a branch).  The lanes of a warp stay together (a branch
+// per lane splits the warp, and what follows may then issue once for each part).
 __device__ __forceinline__ F2 half_slope(F2 qm, F2 q, F2 qp, F2* rs = nullptr) {
-    return half_slope_of(f2_sub(q, qm), f2_sub(qp, q), rs);
+    const F2 dm = f2_sub(q, qm), dp = f2_sub(qp, q);
+    const bool slope = !((fabsf(dp.h) <= 1e-12f) | (__fmul_rn(dm.h, dp.h) <= 0.f));
+    F2 s{0.f, 0.f};
+    if (rs) *rs = s;
+    const unsigned lanes = __activemask();
+    if (__any_sync(lanes, slope)) {
+        const F2 S = f2_add(dm, dp);
+        s = f2_sel(slope, f2_mul(dm, f2_div(dp, S, f_rcp(S.h))));
+        if (rs) *rs = f2_sel(slope, f2_rcp(S));
+    }
+    return s;
 }
 // The free surface's slope stays in FP64: the pressure that balances the bed follows from it.
 __device__ __forceinline__ double half_slope(double qm, double q, double qp, F2* rs = nullptr) {
-    if (rs) {
-        double r;
-        const double s = van_leer_slope_rs(qm, q, qp, r);
-        *rs = f2_of(r);
-        return 0.5 * s;
+    const double dm = __dadd_rn(q, -qm), dp = __dadd_rn(qp, -q);
+    const double p = __dmul_rn(dm, dp);
+    const bool slope = !abs_le_bits(dp, Cst<double>::tol12_bits) & pos_i(p);
+    double s = 0.0;
+    if (rs) *rs = F2{0.f, 0.f};
+    const unsigned lanes = __activemask();
+    if (__any_sync(lanes, slope)) {
+        const double S = __dadd_rn(dm, dp), t = van_leer_half_div(p, S);
+        s = slope ? t : 0.0;
+        if (rs) *rs = f2_sel(slope, f2_of(rcp_nr(S)));
     }
-    return 0.5 * van_leer_slope<double, true>(qm, q, qp);
+    return s;
 }
 
 // The flux of roe_hydrostatic_fast for states beyond the pair form's range (depths from 2^32 m, speeds from
@@ -185,16 +202,18 @@ __device__ __noinline__ void roe_hydrostatic_far(double hi, double ui, double vi
 // The dissipation is arranged so that nothing cancels at a high Froude number (thin fast flow, where the
 // wave strengths are large against their sum).  With Roe's averages, d(hu) = u dh + m for m = si sj du, so
 //   A = a2 + a0 = dh / 2,   B = a2 - a0 = m / (2 c)          (a0, a2: half the wave strengths)
-// and, the signs of l0 = u - c and l2 = u + c known (no entropy fix here),
+// and, without an entropy fix, the signs of l0 = u - c and l2 = u + c being known,
 //   |l0| a0 + |l2| a2       = u P + c Q
 //   |l0| a0 l0 + |l2| a2 l2 = (u^2 + c^2) P + 2 u c Q
 // with (P, Q) = sgn(u)(A, B) for supercritical flow, where c B = m / 2 needs no division, and (B, A) for
-// subcritical flow.  The contact wave's |u| a1 c = |u| si sj dv / 2.  The reference's guards 1e-12 in the
+// subcritical flow.  (A face with a fixed speed, where u is near c, forms its two wave strengths.)  The contact
+// wave's |u| a1 c = |u| si sj dv / 2.  The reference's guards 1e-12 in the
 // denominators si + sj and 2 c enter to first order: um = u (1 - tol12 / (si + sj)), 1 / (2 c + tol12) =
 // (1 - tol12 / (2 c)) / (2 c), the second order being below 1e-18.
 //
-// Measured on the 8192^2 FP64 level: 24.6 -> 9.2 ms a step, the FP64 instructions of a cell's update 190 -> 55;
-// error of four steps against 64-bit arithmetic 8.9e-16 -> 5.8e-16 (2-norm).  A first version that kept the wave
+// Measured on the 8192^2 FP64 level: 24.6 -> 8.8 ms a step, the FP64 instructions of a cell's update 190 -> 50;
+// error of four steps against 64-bit arithmetic 8.9e-16 -> 5.8e-16 (2-norm).  The entropy-fixed faces in pairs too
+// (in FP64 out of line at first: 9.2 ms).  A first version that kept the wave
 // strengths l2 dh - d(hu), l0 dh - d(hu) in pairs lost 2^-48 (|u| / c)^2 of thin fast flow and was 5% slower.
 template <int DIR, bool REC = false>
 __device__ __forceinline__ void roe_hydrostatic_pair(double hi, F2 ui, F2 vi, double hj, F2 uj, F2 vj, F2& Fm,
@@ -210,15 +229,10 @@ __device__ __forceinline__ void roe_hydrostatic_pair(double hi, F2 ui, F2 vi, do
     const F2 si = f2_sqrt(Hi, r), sj = f2_sqrt(Hj, r);
     {
         const unsigned top = (1023u + 32u) << 20;  // depths are non-negative here; NaN and inf are above
-        const bool in = (unsigned)__double2hiint(hi) < top && (unsigned)__double2hiint(hj) < top &&
-                        fabsf(uni.h) < 0x1p24f && fabsf(uti.h) < 0x1p24f && fabsf(unj.h) < 0x1p24f &&
-                        fabsf(utj.h) < 0x1p24f;
-        // the entropy fixes, ruled out in float where a sign is certain (roe_hydrostatic_fast)
-        const float ci = __fmul_rn(3.13209195f, si.h), cj = __fmul_rn(3.13209195f, sj.h);
-        const float mi = 0x1p-16f * (fabsf(uni.h) + ci), mj = 0x1p-16f * (fabsf(unj.h) + cj);
-        const bool rule0 = (uni.h - ci >= mi) || (unj.h - cj <= -mj);
-        const bool rule2 = (uni.h + ci >= mi) || (unj.h + cj <= -mj);
-        if (!(in && rule0 && rule2)) {
+        const bool in = ((unsigned)__double2hiint(hi) < top) & ((unsigned)__double2hiint(hj) < top) &
+                        (fabsf(uni.h) < 0x1p24f) & (fabsf(uti.h) < 0x1p24f) & (fabsf(unj.h) < 0x1p24f) &
+                        (fabsf(utj.h) < 0x1p24f);
+        if (!in) {
             double F[3];
             roe_hydrostatic_far<DIR, REC>(hi, f64_of(ui), f64_of(vi), hj, f64_of(uj), f64_of(vj), F, rv);
             Fm = f2_of(F[0]);
@@ -248,7 +262,9 @@ __device__ __forceinline__ void roe_hydrostatic_pair(double hi, F2 ui, F2 vi, do
     cB.l = __fmaf_rn(-tc, cB.h, cB.l);
     // the signs of um - cm and um + cm, certain in float where they differ and irrelevant where they do not
     const bool super = fabsf(um.h) > cm.h;
-    F2 P, cQ;
+    F2 P, cQ, w, wl;
+    F2 l0, l2;
+    bool fix0 = false, fix2 = false;
     {
         const F2 B = f2_mul(cB, rc), cA = f2_mul(cm, A);
         const int s = __float_as_int(um.h) & (int)0x80000000;
@@ -256,22 +272,57 @@ __device__ __forceinline__ void roe_hydrostatic_pair(double hi, F2 ui, F2 vi, do
         P.l = super ? __int_as_float(__float_as_int(A.l) ^ s) : B.l;
         cQ.h = super ? __int_as_float(__float_as_int(cB.h) ^ s) : cA.h;
         cQ.l = super ? __int_as_float(__float_as_int(cB.l) ^ s) : cA.l;
+        w = f2_add(f2_mul_raw(um, P), cQ);
+        wl = f2_add(f2_mul_raw(f2_add(f2_mul_raw(um, um), ghm), P), f2_mul_raw(F2{um.h + um.h, um.l + um.l}, cQ));
+        F2 a0 = f2_half(f2_sub(A, B)), a2 = f2_half(f2_add(A, B));
+        // the entropy fixes, ruled out in float where a sign is certain (roe_hydrostatic_fast)
+        const float ci = __fmul_rn(3.13209195f, si.h), cj = __fmul_rn(3.13209195f, sj.h);
+        const float mi = 0x1p-16f * (fabsf(uni.h) + ci), mj = 0x1p-16f * (fabsf(unj.h) + cj);
+        const bool rule0 = (uni.h - ci >= mi) | (unj.h - cj <= -mj);
+        const bool rule2 = (uni.h + ci >= mi) | (unj.h + cj <= -mj);
+        if (REC || !(rule0 && rule2)) {
+            l0 = f2_sub(um, cm);
+            l2 = f2_add(um, cm);
+        }
+        if (!(rule0 && rule2)) {
+            constexpr F2 kSqrtG{3.1320919526731650f, (float)(3.1320919526731650 - (double)3.1320919526731650f)};
+            const F2 Ci = f2_mul(kSqrtG, si), Cj = f2_mul(kSqrtG, sj);
+            F2 ei = f2_sub(uni, Ci), ej = f2_sub(unj, Cj);
+            fix0 = !rule0 && ei.h < 0.f && ej.h > 0.f;
+            if (fix0) {
+                const F2 d = f2_sub(ej, ei);
+                l0 = f2_div(f2_mul(ei, f2_sub(ej, l0)), d, f_rcp(d.h));
+            }
+            ei = f2_add(uni, Ci);
+            ej = f2_add(unj, Cj);
+            fix2 = !rule2 && ei.h < 0.f && ej.h > 0.f;
+            if (fix2) {
+                const F2 d = f2_sub(ej, ei);
+                l2 = f2_div(f2_mul(ej, f2_sub(l2, ei)), d, f_rcp(d.h));
+            }
+            if (fix0 || fix2) {  // the wave strengths of the fixed speeds: (l2 - u) dh - m, (u - l0) dh + m
+                const F2 q = f2_half(rc), m2{m.h + m.h, m.l + m.l};
+                const F2 hd = f2_half(F2{q.h, __fmaf_rn(-tc, q.h, q.l)});  // 1 / (4 c + 2 tol12)
+                a0 = f2_mul(f2_sub(f2_mul_raw(f2_sub(l2, um), dh), m2), hd);
+                a2 = f2_mul(f2_add(f2_mul_raw(f2_sub(um, l0), dh), m2), hd);
+                const F2 w0 = f2_mul(f2_abs(l0), a0), w2 = f2_mul(f2_abs(l2), a2);
+                w = f2_add(w0, w2);
+                wl = f2_add(f2_mul_raw(w0, l0), f2_mul_raw(w2, l2));
+            }
+        }
         if constexpr (REC) {
-            const F2 l0 = f2_sub(um, cm), l2 = f2_add(um, cm);
             const float h = __fmul_rn(0.25f, rc.h);  // 1 / (4 cm + 2 tol12)
             rv->si = f64_of(si); rv->sj = f64_of(sj); rv->cm = f64_of(cm); rv->rs = f64_of(rs);
             rv->hrden = f64_of(f2_norm(h, __fmaf_rn(0.25f, rc.l, -__fmul_rn(h, tc))));
             rv->hrcm = 0.5 * f64_of(rc);
             rv->um = f64_of(um); rv->vm = f64_of(vm); rv->l0 = f64_of(l0); rv->l2 = f64_of(l2);
-            rv->a0h = 0.5 * f64_of(f2_sub(A, B)); rv->a2h = 0.5 * f64_of(f2_add(A, B));
+            rv->a0h = f64_of(a0); rv->a2h = f64_of(a2);
             rv->a1h = f64_of(f2_mul(mv, rc));
-            rv->fl = (wi ? RR_WI : 0u) | (wj ? RR_WJ : 0u) | (hmb ? RR_HM : 0u);
+            rv->fl = (wi ? RR_WI : 0u) | (wj ? RR_WJ : 0u) | (hmb ? RR_HM : 0u) | (fix0 ? RR_FIX0 : 0u) |
+                     (fix2 ? RR_FIX2 : 0u);
         }
     }
     const F2 qi = f2_mul(Hi, uni), qj = f2_mul(Hj, unj);
-    const F2 w = f2_add(f2_mul_raw(um, P), cQ);
-    const F2 wl = f2_add(f2_mul_raw(f2_add(f2_mul_raw(um, um), ghm), P),
-                         f2_mul_raw(F2{um.h + um.h, um.l + um.l}, cQ));
     const F2 d0 = f2_sub(f2_half(f2_add(qi, qj)), w);
     const F2 d1 = f2_sub(f2_half(f2_add(f2_mul_raw(qi, uni), f2_mul_raw(qj, unj))), wl);
     const F2 d2 = f2_sub(f2_half(f2_add(f2_mul_raw(qi, uti), f2_mul_raw(qj, utj))),
@@ -305,6 +356,199 @@ __device__ __forceinline__ void hydro_face(bool wall, double zL, double zR, doub
     Fl = lhigh ? fn : fw;
     Fr = lhigh ? fw : fn;
 }
+// ---------------------------------------------------------------------------
+// The exact FP64 form's slopes and face: the reference's operations and
+// rounding, with divisions, roots and decisions off the FP64 pipe.
+// ---------------------------------------------------------------------------
+static __device__ __noinline__ double half_slope_generic(double qm, double q, double qp) {
+    return 0.5 * van_leer_slope<double, false>(qm, q, qp);
+}
+// Half the van Leer slope as hydro_face takes it, 0.5 * van_leer_slope: with r = dm / dp > 0 the halves of
+// (r + |r|) / (1 + |r|) * dp, every factor of two being exact here, are (r / (1 + r)) dp; r <= 0 gives a zero
+// of dp's sign.  Differences that are not finite or whose quotient leaves 2^+-400 take the formula itself.
+// The lanes of a warp stay together: the quotients run for all of them where one needs them.
+__device__ __forceinline__ double half_slope_ieee(double qm, double q, double qp) {
+    const double dm = q - qm, dp = qp - q;
+    const unsigned hm = (unsigned)__double2hiint(dm), hp = (unsigned)__double2hiint(dp);
+    const unsigned em = hm & 0x7FF00000u, ep = hp & 0x7FF00000u;
+    const bool flat = abs_le_bits(dp, Cst<double>::tol12_bits);
+    const bool zero = ((hm & 0x7FFFFFFFu) | (unsigned)__double2loint(dm)) == 0u;
+    const bool odd = ep == 0x7FF00000u || em == 0x7FF00000u || (!zero && em - ep + (400u << 20) > (800u << 20));
+    const bool slope = !flat && !zero && (int)(hm ^ hp) >= 0;
+    double s = __hiloint2double(flat ? 0 : (int)(hp & 0x80000000u), 0);
+    const unsigned lanes = __activemask();
+    if (__any_sync(lanes, slope)) {
+        const double r = ieee_div<false>(dm, dp);
+        const double t = ieee_div<false>(r, 1.0 + r) * dp;
+        s = slope ? t : s;
+    }
+    if (odd && !flat) s = half_slope_generic(qm, q, qp);
+    return s;
+}
+
+// zero, or of magnitude within 2^+-250
+__device__ __forceinline__ bool exact_range(double x) {
+    const unsigned t = (unsigned)__double2hiint(x) & 0x7FFFFFFFu;
+    return (t - (773u << 20) < (500u << 20)) | ((t | (unsigned)__double2loint(x)) == 0u);
+}
+// u' = RN(RN(h u) / h) with p = RN(h u): the velocity the reference's flux rebuilds from the face momentum.
+// rem = p - h u is exact (fma), below one place of p; u' is u unless |rem| is more than half of h's product
+// with the last place of u, and then its neighbour on rem's side (it cannot be halfway, nor two places off).
+// RN(h u') is p itself, except perhaps where p is a power of two and u' not u: odd.  Operands are in the
+// range the caller checks.
+__device__ __forceinline__ double rebuilt_velocity(double h, double u, double& p, bool& odd) {
+    p = h * u;
+    const double rem = __fma_rn(-h, u, p);
+    const unsigned uh = (unsigned)__double2hiint(u);
+    const unsigned long long half =  // h ulp(u)
+        ((unsigned long long)((unsigned)__double2hiint(h) + (uh & 0x7FF00000u) - (1075u << 20)) << 32) |
+        (unsigned)__double2loint(h);
+    const unsigned long long r2 =  // 2 |rem|
+        ((unsigned long long)(((unsigned)__double2hiint(rem) & 0x7FFFFFFFu) + 0x100000u) << 32) |
+        (unsigned)__double2loint(rem);
+    const bool move = (r2 > half) & ((uh & 0x7FF00000u) != 0u);
+    odd |= move & ((((unsigned)__double2hiint(p) & 0xFFFFFu) | (unsigned)__double2loint(p)) == 0u);
+    const int to = ((int)(uh ^ (unsigned)__double2hiint(rem)) >> 31) | 1;
+    return __longlong_as_double(__double_as_longlong(u) + (move ? to : 0));
+}
+static __device__ __noinline__ double2 cell_velocity_generic(double h, double qx, double qy) {
+    return {qx / h, qy / h};
+}
+// (qx, qy) / h, IEEE rounded, where h is above the division tolerance, else 0.
+__device__ __forceinline__ void cell_velocity_ieee(double h, double qx, double qy, double& u, double& v) {
+    const bool wet = gt_bits(h, Cst<double>::tol12_bits);
+    const IeeeDivisor d = ieee_divisor(wet ? h : 1.0);
+    u = wet ? ieee_div<false>(qx, d) : 0.0;
+    v = wet ? ieee_div<false>(qy, d) : 0.0;
+    if (wet && !(exact_range(qx) && exact_range(qy) && d.e < ((1023u + 200u) << 20))) {
+        const double2 q = cell_velocity_generic(h, qx, qy);
+        u = q.x;
+        v = q.y;
+    }
+}
+// The entropy-fixed speeds of a face whose signs float cannot tell (roe_hydrostatic_exact).  Not inlined, but on
+// wet/dry fronts some lane of a third of the warps comes here: roots and quotients stay off the FP64 pipe.
+static __device__ __noinline__ void sonic_fix_exact(double hi, double uni, double hj, double unj, double& l0,
+                                                    double& l2) {
+    const double ci = ieee_sqrt(Cst<double>::g * hi), cj = ieee_sqrt(Cst<double>::g * hj);
+    double ei = uni - ci, ej = unj - cj;
+    if (neg_i(ei) && pos_i(ej)) l0 = ieee_div(ei * (ej - l0), ej - ei);
+    ei = uni + ci;
+    ej = unj + cj;
+    if (neg_i(ei) && pos_i(ej)) l2 = ieee_div(ej * (l2 - ei), ej - ei);
+}
+static __device__ __noinline__ void hydro_face_generic(int dir, double zL, double zR, double eL, double eR, double seL,
+                                                       double seR, double uL, double uR, double suL, double suR,
+                                                       double vL, double vR, double svL, double svR, double* F) {
+    // the slopes come halved: 2 s is exact (or infinite, as s then is)
+    if (dir == 0)
+        hydro_face<double, false, 0>(false, zL, zR, eL, eR, 2.0 * seL, 2.0 * seR, uL, uR, 2.0 * suL, 2.0 * suR, vL, vR,
+                                     2.0 * svL, 2.0 * svR, F[0], F[1], F[2], F[3]);
+    else
+        hydro_face<double, false, 1>(false, zL, zR, eL, eR, 2.0 * seL, 2.0 * seR, uL, uR, 2.0 * suL, 2.0 * suR, vL, vR,
+                                     2.0 * svL, 2.0 * svR, F[0], F[1], F[2], F[3]);
+    for (int k = 0; k < 4; ++k) F[k] *= 2.0;
+}
+
+// hydro_face of the exact FP64 form: the reference's values bit for bit, from half slopes, with every flux
+// doubled (each of the reference's factors 0.5 is exact and moves out of the sums; the update's dt/dx is halved
+// instead).  Of the face's ~250 FP64 pipe slots in the compiler's sequences 72 additions and products remain:
+// five quotients and three roots run on the integer pipe (hx_ieee.cuh), the four velocities that the
+// reference rebuilds as (h u) / h follow from one fma each, and comparisons are taken on bit patterns.  Values
+// whose products could leave the normal range (speeds outside 2^+-250, depths from 2^200, beds that are
+// not finite) take the formula itself.
+//
+// Measured: the step of a 2047 x 1531 level 4.9 -> 1.64 ms, of a 256^2 level 163 -> 49 us, 186 FP64 instructions
+// per cell (all of them additions and products).  No term of the range check branches on its own: with && and ||
+// the compiler split the warp on dry sides and rebuilt velocities and issued the FP64 instructions after it
+// once for each part (252 per cell, 2.35 ms).
+template <int DIR>
+__device__ __forceinline__ void hydro_face_ieee(bool wall, double zL, double zR, double eL, double eR, double seL,
+                                                double seR, double uL, double uR, double suL, double suR, double vL,
+                                                double vR, double svL, double svR, double& Fm, double& Fl, double& Fr,
+                                                double& Ft) {
+    using C = Cst<double>;
+    if (wall) {
+        Fm = Fl = Fr = Ft = 0.0;
+        return;
+    }
+    const double etaLf = eL + seL, etaRf = eR - seR;
+    const double uLf = uL + suL, uRf = uR - suR;
+    const double vLf = vL + svL, vRf = vR - svR;
+    const bool lhigh = !(okey(zL) < okey(zR));  // the left bed is the face bed: its pressure correction is +0
+    const double eH = lhigh ? etaLf : etaRf, zf = lhigh ? zL : zR;
+    const double eW = lhigh ? etaRf : etaLf, zW = lhigh ? zR : zL;
+    const double hH = max0_num(eH - zf);
+    const double hWu = max0_num(eW - zW), hWs = max0_num(eW - zf);
+    double hi = lhigh ? hH : hWs, hj = lhigh ? hWs : hH;
+    const bool wi = ge_bits(hi, C::toldry_bits), wj = ge_bits(hj, C::toldry_bits);
+    const double dry = DIR == 0 ? 0.0 : -0.0;  // the rotated tangential velocity of a dry side
+    const double Hi = wi ? hi : 0.0, Hj = wj ? hj : 0.0;
+    double pi, pj, ri, rj;  // h uni, h uti on either side
+    bool odd = false;
+    const double uni = rebuilt_velocity(Hi, wi ? (DIR == 0 ? uLf : vLf) : 0.0, pi, odd);
+    const double uti = rebuilt_velocity(Hi, wi ? (DIR == 0 ? vLf : -uLf) : dry, ri, odd);
+    const double unj = rebuilt_velocity(Hj, wj ? (DIR == 0 ? uRf : vRf) : 0.0, pj, odd);
+    const double utj = rebuilt_velocity(Hj, wj ? (DIR == 0 ? vRf : -uRf) : dry, rj, odd);
+    {
+        const unsigned top = (1023u + 200u) << 20, fin = 0x7FF00000u;
+        // (bitwise: a branch per term would split the warp around the FP64 instructions)
+        const bool in = !odd & (!wi | (exact_range(uLf) & exact_range(vLf))) &
+                        (!wj | (exact_range(uRf) & exact_range(vRf))) & ((unsigned)__double2hiint(hi) < top) &
+                        ((unsigned)__double2hiint(hj) < top) & ((unsigned)__double2hiint(hWu) < top) &
+                        (((unsigned)__double2hiint(zL) & 0x7FFFFFFFu) < fin) &
+                        (((unsigned)__double2hiint(zR) & 0x7FFFFFFFu) < fin);
+        if (!in) {
+            double F[4];
+            hydro_face_generic(DIR, zL, zR, eL, eR, seL, seR, uL, uR, suL, suR, vL, vR, svL, svR, F);
+            Fm = F[0]; Fl = F[1]; Fr = F[2]; Ft = F[3];
+            return;
+        }
+    }
+    hi = Hi;
+    hj = Hj;
+    const double si = ieee_sqrt<false>(hi), sj = ieee_sqrt<false>(hj);
+    const double hs = hi + hj;
+    const double cm = ieee_sqrt<false>(gt_bits(hs, C::toldry2_bits) ? C::half_g * hs : C::g_toldry);
+    const IeeeDivisor sden = ieee_divisor(si + sj + C::tol12);
+    const double um = ieee_div<false>(uni * si + unj * sj, sden);
+    const double vm = ieee_div<false>(uti * si + utj * sj, sden);
+    double l0 = um - cm, l2 = um + cm;
+    {  // the entropy fixes, ruled out in float where a sign is certain (roe_hydrostatic_fast)
+        const float ui32 = f32_lead(uni), uj32 = f32_lead(unj);
+        const float ci32 = 3.13209195f * f32_lead(si), cj32 = 3.13209195f * f32_lead(sj);
+        const float mi = 0x1p-16f * (fabsf(ui32) + ci32), mj = 0x1p-16f * (fabsf(uj32) + cj32);
+        const bool rule0 = (ui32 - ci32 >= mi) | (uj32 - cj32 <= -mj);
+        const bool rule2 = (ui32 + ci32 >= mi) | (uj32 + cj32 <= -mj);
+        if (!(rule0 & rule2)) sonic_fix_exact(hi, uni, hj, unj, l0, l2);
+    }
+    const IeeeDivisor den = ieee_divisor(__fma_rn(2.0, cm, C::tol12));  // 2 cm is exact
+    const double dh = hj - hi, dhu = pj - pi, dhv = rj - ri;
+    const double a0 = ieee_div<false>(l2 * dh - dhu, den);
+    const double a1 = ieee_div<false>(dhv - vm * dh, cm);
+    const double a2 = ieee_div<false>(dhu - l0 * dh, den);
+    const double w0 = fabs(l0) * a0, w1 = fabs(um) * a1, w2 = fabs(l2) * a2;
+    Fm = (pi + pj) - w0 - w2;
+    const double f1 = (pi * uni + C::half_g * hi * hi + pj * unj + C::half_g * hj * hj) - w0 * l0 - w2 * l2;
+    const double f2 = (pi * uti + pj * utj) - w0 * vm - w1 * cm - w2 * vm;
+    Ft = DIR == 0 ? f2 : -f2;
+    const double fw = f1 + C::g * (hWu * hWu - hWs * hWs);
+    // adding the other side's +0 correction turns a -0 into +0
+    const double fn = __double_as_longlong(f1) == (long long)0x8000000000000000ull ? 0.0 : f1;
+    Fl = lhigh ? fn : fw;
+    Fr = lhigh ? fw : fn;
+}
+// The face of an arithmetic form.
+template <class R, bool FAST, int DIR, bool REC, class V>
+__device__ __forceinline__ void hydro_face_of(bool wall, R zL, R zR, R eL, R eR, R seL, R seR, V uL, V uR, V suL, V suR,
+                                              V vL, V vR, V svL, V svR, V& Fm, R& Fl, R& Fr, V& Ft, RoeRecVals* rv) {
+    if constexpr (kIeee<R, FAST>)
+        hydro_face_ieee<DIR>(wall, zL, zR, eL, eR, seL, seR, uL, uR, suL, suR, vL, vR, svL, svR, Fm, Fl, Fr, Ft);
+    else
+        hydro_face<R, FAST, DIR, REC>(wall, zL, zR, eL, eR, seL, seR, uL, uR, suL, suR, vL, vR, svL, svR, Fm, Fl, Fr,
+                                      Ft, rv);
+}
+
 // Fluxes and their differences as the update and the face arrays take them.
 template <class R> __device__ __forceinline__ R flux_of(R f) { return f; }
 __device__ __forceinline__ double flux_of(F2 f) { return f64_of(f); }
@@ -360,6 +604,15 @@ template <class R> struct ScreenCell {
     bool nod = false, live = false;
 };
 
+template <class R> __device__ __forceinline__ R exact_quot(R a, R b) {
+    if constexpr (std::is_same_v<R, double>) return ieee_div(a, b);
+    else return a / b;
+}
+template <class R> __device__ __forceinline__ R exact_root(R x) {
+    if constexpr (std::is_same_v<R, double>) return ieee_sqrt(x);
+    else return sqrt(x);
+}
+
 template <class R, bool FAST, bool LINEAR, class NP = Plane<R>>
 __device__ __forceinline__ void step_cell(R o0, R o1, R o2, R dx0, R dx1, R dx2, R dy0, R dy1, R dy2, R cx, R cy,
                                           R dt, const NP& nplane, const Cells3W<R>& out, int gi, int gj,
@@ -376,24 +629,31 @@ __device__ __forceinline__ void step_cell(R o0, R o1, R o2, R dx0, R dx1, R dx2,
     const R hh = un[0];
     bool wet, rough;
     if constexpr (FAST) wet = ge_bits(hh, Cst<R>::toldry_bits);
+    else if constexpr (kIeee<R, FAST>) wet = ge_num(hh, Cst<R>::toldry_bits);
     else wet = hh >= Cst<R>::toldry;
     if (wet) {
         const R nv = nplane.ld(gi, gj);
-        const R nsq = nv * nv;
+        R nsq = R(0);
+        if constexpr (sizeof(R) == 8 && !std::is_same_v<R, Dual>) {
+            // |n| below 0.9e-6: n^2 is not above tol12 (a smooth bed takes no FP64 instruction here)
+            if (!abs_le_bits(nv, 0x3EAE32F0EE144531ll)) nsq = nv * nv;
+        } else {
+            nsq = nv * nv;
+        }
         if constexpr (FAST) rough = gt_bits(nsq, Cst<R>::tol12_bits);
         else rough = nsq > Cst<R>::tol12;
         if (rough) {  // the friction factor needs a rough bed
             const R qx = un[1], qy = un[2];
             if constexpr (!FAST) {
-                const R inv_h = R(1.0) / hh;
+                const R inv_h = exact_quot(R(1.0), hh);
                 const R uu = qx * inv_h, vv = qy * inv_h;
-                const R modM = sqrt(uu * uu + vv * vv);
+                const R modM = exact_root(uu * uu + vv * vv);
                 if (modM > Cst<R>::tol12) {
                     pflags |= 1u;
                     const R h43 = hh * cbrt(hh);
-                    const R tt = dt * Cst<R>::g * nsq * modM / h43;
-                    const R ff = sqrt(R(1.0) + R(4.0) * tt);
-                    const R fac = R(2.0) / (R(1.0) + ff);
+                    const R tt = exact_quot(dt * Cst<R>::g * nsq * modM, h43);
+                    const R ff = exact_root(R(1.0) + R(4.0) * tt);
+                    const R fac = exact_quot(R(2.0), R(1.0) + ff);
                     un[1] = qx * fac;
                     un[2] = qy * fac;
                 }
@@ -729,10 +989,7 @@ __device__ __forceinline__ void hydro_tile_body(TileSmem<R, FAST, TXv, TYv>& S, 
     const int t = sy.tid();
     if (start_barrier) sy.bar();  // the previous tile of this block is done with S (else the caller synced)
     if (set_kc && t == 0) {  // read after the barriers below (a persistent caller sets them once)
-        S.kc[0] = dt / dx;
-        S.kc[1] = dt / dy;
-        S.kc[2] = R(1) / dx;
-        S.kc[3] = R(1) / dy;
+        tile_constants<R, FAST>(S.kc, dt, dx, dy);
     }
 
     // --- A: grown tile -> h rebuilt, eta = h + z, velocities -----------------
@@ -771,9 +1028,14 @@ __device__ __forceinline__ void hydro_tile_body(TileSmem<R, FAST, TXv, TYv>& S, 
         }
         R hp;
         if constexpr (!FAST) {
-            hp = max0(e - zz);  // HydrostaticRoe.cpp:498
-            S.u[r][c] = (hp > Cst<R>::tol12) ? qx / hp : R(0);
-            S.v[r][c] = (hp > Cst<R>::tol12) ? qy / hp : R(0);
+            if constexpr (kIeee<R, FAST>) {
+                hp = max0_num(e - zz);  // HydrostaticRoe.cpp:498
+                cell_velocity_ieee(hp, qx, qy, S.u[r][c], S.v[r][c]);
+            } else {
+                hp = max0(e - zz);
+                S.u[r][c] = (hp > Cst<R>::tol12) ? qx / hp : R(0);
+                S.v[r][c] = (hp > Cst<R>::tol12) ? qy / hp : R(0);
+            }
         } else {
             hp = stored ? max0_i(e) : max0_i(e - zz);
             cell_velocity(hp, qx, qy, S.u[r][c], S.v[r][c]);
@@ -802,6 +1064,10 @@ __device__ __forceinline__ void hydro_tile_body(TileSmem<R, FAST, TXv, TYv>& S, 
             S.sxe[row][col + 1] = half_slope(S.eta[r][c - 1], S.eta[r][c], S.eta[r][c + 1]);
             S.sxu[row][col + 1] = half_slope(S.u[r][c - 1], S.u[r][c], S.u[r][c + 1]);
             S.sxv[row][col + 1] = half_slope(S.v[r][c - 1], S.v[r][c], S.v[r][c + 1]);
+        } else if constexpr (kIeee<R, FAST>) {
+            S.sxe[row][col + 1] = half_slope_ieee(S.eta[r][c - 1], S.eta[r][c], S.eta[r][c + 1]);
+            S.sxu[row][col + 1] = half_slope_ieee(S.u[r][c - 1], S.u[r][c], S.u[r][c + 1]);
+            S.sxv[row][col + 1] = half_slope_ieee(S.v[r][c - 1], S.v[r][c], S.v[r][c + 1]);
         } else {
             S.sxe[row][col + 1] = van_leer_slope<R, FAST>(S.eta[r][c - 1], S.eta[r][c], S.eta[r][c + 1]);
             S.sxu[row][col + 1] = van_leer_slope<R, FAST>(S.u[r][c - 1], S.u[r][c], S.u[r][c + 1]);
@@ -824,6 +1090,10 @@ __device__ __forceinline__ void hydro_tile_body(TileSmem<R, FAST, TXv, TYv>& S, 
             S.sye[row + 1][col] = half_slope(S.eta[r - 1][c], S.eta[r][c], S.eta[r + 1][c]);
             S.syu[row + 1][col] = half_slope(S.u[r - 1][c], S.u[r][c], S.u[r + 1][c]);
             S.syv[row + 1][col] = half_slope(S.v[r - 1][c], S.v[r][c], S.v[r + 1][c]);
+        } else if constexpr (kIeee<R, FAST>) {
+            S.sye[row + 1][col] = half_slope_ieee(S.eta[r - 1][c], S.eta[r][c], S.eta[r + 1][c]);
+            S.syu[row + 1][col] = half_slope_ieee(S.u[r - 1][c], S.u[r][c], S.u[r + 1][c]);
+            S.syv[row + 1][col] = half_slope_ieee(S.v[r - 1][c], S.v[r][c], S.v[r + 1][c]);
         } else {
             S.sye[row + 1][col] = van_leer_slope<R, FAST>(S.eta[r - 1][c], S.eta[r][c], S.eta[r + 1][c]);
             S.syu[row + 1][col] = van_leer_slope<R, FAST>(S.u[r - 1][c], S.u[r][c], S.u[r + 1][c]);
@@ -852,14 +1122,17 @@ __device__ __forceinline__ void hydro_tile_body(TileSmem<R, FAST, TXv, TYv>& S, 
         R Fl, Fr;
         const bool wall = S.nod[r][cl] | S.nod[r][cr];
         RoeRecVals rv;
-        hydro_face<R, FAST, 0, Rec::on>(wall, S.z[r][cl], S.z[r][cr], S.eta[r][cl], S.eta[r][cr], S.sxe[fj][fi],
+        hydro_face_of<R, FAST, 0, Rec::on>(wall, S.z[r][cl], S.z[r][cr], S.eta[r][cl], S.eta[r][cr], S.sxe[fj][fi],
                                         S.sxe[fj][fi + 1], S.u[r][cl], S.u[r][cr], S.sxu[fj][fi], S.sxu[fj][fi + 1],
                                         S.v[r][cl], S.v[r][cr], S.sxv[fj][fi], S.sxv[fj][fi + 1], Fm, Fl, Fr, Ft, &rv);
         if constexpr (Rec::on) {
             if (!wall) rec.put_x(x0 + fi, y0 + fj, rv, fi == TXv);
         }
         S.fxm[fj][fi] = Fm; S.fxl[fj][fi] = Fl; S.fxr[fj][fi] = Fr; S.fxt[fj][fi] = Ft;
-        if (fo.on || fo.mean) fo.store_x(x0 + fi, y0 + fj, vb, flux_of(Fm), Fl, Fr, flux_of(Ft), fi == TXv);
+        if (fo.on || fo.mean) {
+            constexpr R F = kIeee<R, FAST> ? R(0.5) : R(1);
+            fo.store_x(x0 + fi, y0 + fj, vb, F * flux_of(Fm), F * Fl, F * Fr, F * flux_of(Ft), fi == TXv);
+        }
     };
     auto yface = [&](int fi, int fj) {
         const int c = fi + 2, rl = fj + 1, rr = fj + 2;
@@ -867,14 +1140,17 @@ __device__ __forceinline__ void hydro_tile_body(TileSmem<R, FAST, TXv, TYv>& S, 
         R Fl, Fr;
         const bool wall = S.nod[rl][c] | S.nod[rr][c];
         RoeRecVals rv;
-        hydro_face<R, FAST, 1, Rec::on>(wall, S.z[rl][c], S.z[rr][c], S.eta[rl][c], S.eta[rr][c], S.sye[fj][fi],
+        hydro_face_of<R, FAST, 1, Rec::on>(wall, S.z[rl][c], S.z[rr][c], S.eta[rl][c], S.eta[rr][c], S.sye[fj][fi],
                                         S.sye[fj + 1][fi], S.u[rl][c], S.u[rr][c], S.syu[fj][fi], S.syu[fj + 1][fi],
                                         S.v[rl][c], S.v[rr][c], S.syv[fj][fi], S.syv[fj + 1][fi], Fm, Fl, Fr, Ft, &rv);
         if constexpr (Rec::on) {
             if (!wall) rec.put_y(x0 + fi, y0 + fj, rv, fj == TYv);
         }
         S.fym[fj][fi] = Fm; S.fyl[fj][fi] = Fl; S.fyr[fj][fi] = Fr; S.fyt[fj][fi] = Ft;
-        if (fo.on || fo.mean) fo.store_y(x0 + fi, y0 + fj, vb, flux_of(Fm), flux_of(Ft), Fl, Fr, fj == TYv);
+        if (fo.on || fo.mean) {
+            constexpr R F = kIeee<R, FAST> ? R(0.5) : R(1);
+            fo.store_y(x0 + fi, y0 + fj, vb, F * flux_of(Fm), F * flux_of(Ft), F * Fl, F * Fr, fj == TYv);
+        }
     };
     for (int k = t; k < CELLS; k += NTv) {
         const int tx = k % TXv, ty = k / TXv;
@@ -925,7 +1201,8 @@ __device__ __forceinline__ void hydro_tile_body(TileSmem<R, FAST, TXv, TYv>& S, 
         const R dy1 = flux_diff(S.fyt[ty + 1][tx], S.fyt[ty][tx]);
         const R dy2 = S.fyl[ty + 1][tx] - S.fyr[ty][tx];
         if constexpr (Div::on) {  // the flux differences only: the update waits for dt
-            div.st(gi, gj, dx0, dx1, dx2, dy0, dy1, dy2);
+            constexpr R F = kIeee<R, FAST> ? R(0.5) : R(1);
+            div.st(gi, gj, F * dx0, F * dx1, F * dx2, F * dy0, F * dy1, F * dy2);
             continue;
         }
         const R o0 = uo.ld(0, gi, gj), o1 = uo.ld(1, gi, gj), o2 = uo.ld(2, gi, gj);
@@ -938,7 +1215,7 @@ __device__ __forceinline__ void hydro_tile_body(TileSmem<R, FAST, TXv, TYv>& S, 
         if (fold) screened_fold<NTv, 1, Sync, FAST>(&sc, dx, dy, idx, idy, rate, mv, flags, sy);
     }
     if (defer) {
-        if constexpr (FAST) {
+        if constexpr (FAST || kIeee<R, FAST>) {  // non-negative: the integer max is the max either form takes
             defer->rate = nnmax_i(defer->rate, rate);
             defer->mv = nnmax_i(defer->mv, mv);
         } else {
@@ -1256,10 +1533,7 @@ __global__ void __launch_bounds__(kPN, 1)
     ThreadFold<double>* tf = &own->fold[threadIdx.x];
     *tf = ThreadFold<double>{};
     if (threadIdx.x == 0) {  // the tile body's per-tile constants, the same for every tile of the launch
-        S.kc[0] = dt / ctl.dx;
-        S.kc[1] = dt / ctl.dy;
-        S.kc[2] = 1.0 / ctl.dx;
-        S.kc[3] = 1.0 / ctl.dy;
+        tile_constants<double, FAST>(S.kc, dt, ctl.dx, ctl.dy);
     }
     const FaceOut<double> fo{};
     unsigned parity = 0;
@@ -1362,10 +1636,7 @@ __global__ void __launch_bounds__(kPN, 1)
     ThreadFold<double>* tf = &own->fold[threadIdx.x];
     *tf = ThreadFold<double>{};
     if (threadIdx.x == 0) {  // the tile body's per-tile constants, the same for every tile of the launch
-        S.kc[0] = dt / ctl.dx;
-        S.kc[1] = dt / ctl.dy;
-        S.kc[2] = 1.0 / ctl.dx;
-        S.kc[3] = 1.0 / ctl.dy;
+        tile_constants<double, FAST>(S.kc, dt, ctl.dx, ctl.dy);
     }
     const FaceOut<double> fo{};
     const int nxt = 1 - src.phase;

@@ -1,6 +1,6 @@
 """The FP64 fast form's float-pair arithmetic where it can go wrong: thin fast flow (high Froude numbers), nearly
-equal states, one dry side, transcritical faces and speeds past the pair form's range (both in FP64 throughout),
-and whole steps on levels that hold such cells at every remainder of the tiles."""
+equal states, one dry side, transcritical faces (entropy-fixed wave strengths) and speeds past the pair form's range
+(in FP64 throughout), and whole steps on levels that hold such cells at every remainder of the tiles."""
 import numpy as np
 import pytest
 import torch
@@ -66,7 +66,7 @@ def roe_long_double(st, ydir):
 
 
 def fp64_faces(st, ydir):
-    """Faces the pair form leaves to FP64: past its range, or with a characteristic speed that may change sign."""
+    """Faces past the pair form's range, or with a characteristic speed that may change sign."""
     h = np.where(st[:, [0, 3]] >= 1e-6, st[:, [0, 3]], 0.0)
     q = np.where(ydir[:, None], st[:, [2, 5]], st[:, [1, 4]])
     u, c = np.where(h > 0, q / np.where(h > 0, h, 1.0), 0.0), np.sqrt(9.81 * h)
@@ -81,8 +81,8 @@ def fp64_faces(st, ydir):
 @pytest.mark.parametrize("kind", ["ordinary", "thin_fast", "near_equal", "one_dry", "transcritical", "far"])
 def test_pair_flux_against_extended_precision(cuda, hxlib, kind):
     """A flux is a sum of about 16 pair products and sums, each within 2^-46 of its terms: 2^-42 of their scale.
-    The FP64 path of transcritical and far faces (fp64_faces) takes one-step reciprocals (2^-42) in wave strengths that cancel
-    like the Froude number |u| / c, in some 16 terms."""
+    Transcritical and far faces (fp64_faces) form wave strengths that cancel like the Froude number |u| / c, from
+    one-step reciprocals (2^-42), in some 16 terms."""
     rng = np.random.default_rng(20)
     st = face_states(kind, 40000, rng)
     normals = np.zeros((len(st), 2))

@@ -147,11 +147,12 @@ template <class R> __device__ __forceinline__ void cell_velocity(R h, R qx, R qy
 }
 __device__ __forceinline__ void cell_velocity(double h, double qx, double qy, F2& u, F2& v) {
     const bool wet = gt_bits(h, Cst<double>::tol12_bits);
-    F2 d = f2_of(h);
+    F2 d = f2_of_rn(h);
     d.h = wet ? d.h : 1.f;
     const float y0 = f_rcp(d.h), y = __fmaf_rn(y0, __fmaf_rn(-d.h, y0, 1.f), y0);
-    u = f2_sel(wet, f2_div(f2_of(qx), d, y));
-    v = f2_sel(wet, f2_div(f2_of(qy), d, y));
+    // as near as a pair can be: the limiter of nearly equal velocities, and an adjoint through it, see this error
+    u = f2_sel(wet, f2_div_rn(f2_of_rn(qx), d, y));
+    v = f2_sel(wet, f2_div_rn(f2_of_rn(qy), d, y));
 }
 
 // Half the van Leer slope, dm dp / (dm + dp) where the differences have one sign (van_leer_slope), as

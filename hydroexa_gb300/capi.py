@@ -131,8 +131,9 @@ def _declare(L):
                                                                   POINTER(Array4I32), Box, P4, P4, c_void_p, c_void_p,
                                                                   c_int, c_void_p]
         getattr(L, f"hx_dt_reduce_box_{sfx}").argtypes = [P4, P4, Box, real, real, c_void_p, c_void_p]
-        getattr(L, f"hx_tag_box_{sfx}").argtypes = [c_int, P4, P4, POINTER(Array4I8), Box, real, real, real, real,
-                                                   real, real, ctypes.c_byte, c_void_p]
+        for form in ("box", "level"):
+            getattr(L, f"hx_tag_{form}_{sfx}").argtypes = [c_int, P4, P4, POINTER(Array4I8), Box, real, real, real,
+                                                          real, real, real, ctypes.c_byte, c_void_p]
         getattr(L, f"hx_masked_average_down_box_{sfx}").argtypes = [P4, P4, Box, c_int, c_int, c_int, c_int, c_int,
                                                                     real, real, c_void_p]
         getattr(L, f"hx_average_down_box_{sfx}").argtypes = [P4, P4, Box, c_int, c_int, c_int, c_int, c_int,
@@ -233,6 +234,7 @@ EXPORTED = [
     "hx_advance_box_hydrostatic_f64", "hx_advance_box_hydrostatic_f32", "hx_advance_box_roe_f64",
     "hx_advance_box_roe_f32", "hx_advance_box_hydrostatic_reflux_f64", "hx_advance_box_hydrostatic_reflux_f32",
     "hx_advance_box_roe_reflux_f64", "hx_advance_box_roe_reflux_f32", "hx_dt_reduce_box_f64", "hx_dt_reduce_box_f32", "hx_tag_box_f64", "hx_tag_box_f32",
+    "hx_tag_level_f64", "hx_tag_level_f32",
     "hx_masked_average_down_box_f64", "hx_masked_average_down_box_f32", "hx_average_down_box_f64",
     "hx_average_down_box_f32", "hx_derive_eta_box_f64",
     "hx_derive_eta_box_f32", "hx_diagnostics_work_bytes", "hx_diagnostics_box_f64", "hx_diagnostics_box_f32",

@@ -260,13 +260,14 @@ int dt_reduce_box(const A* U, const A* T, hx_box vb, R dx, R dy, hx_dt_accum* ac
 
 template <class R, class A>
 int tag_box(int method, const A* U, const A* T, hx_array4_i8* tags, hx_box vb, R dx, R dy, R time, R hth, R uth,
-            R zth, signed char setv, cudaStream_t st) {
+            R zth, signed char setv, bool clamp, cudaStream_t st) {
+    const int g = clamp ? 0 : 1;
     if (!box_ok(vb)) return HX_ERR_ARG;
     if (method != HX_METHOD_ROE && method != HX_METHOD_HYDROSTATIC_ROE) return fail(HX_ERR_ARG, "unknown method");
-    if (!covers(U, vb, 1, 3, "U") || !covers(T, vb, 1, 1, "T") || !covers(tags, vb, 0, 1, "tags")) return HX_ERR_ARG;
+    if (!covers(U, vb, g, 3, "U") || !covers(T, vb, g, 1, "T") || !covers(tags, vb, 0, 1, "tags")) return HX_ERR_ARG;
     return launched(launch_tag<R>(method, to_v4(*U), to_v4(*T), to_v4(*tags), ibox(vb), dx, dy, time, hth, uth, zth,
-                                  setv, st),
-                    "hx_tag_box");
+                                  setv, clamp, st),
+                    clamp ? "hx_tag_level" : "hx_tag_box");
 }
 
 template <class R, class A>
@@ -703,11 +704,19 @@ int hx_dt_reduce_box_f32(const hx_array4_f32* U, const hx_array4_f32* T, hx_box 
 }
 int hx_tag_box_f64(int method, const hx_array4_f64* U, const hx_array4_f64* T, hx_array4_i8* tags, hx_box vb,
                    double dx, double dy, double time, double h, double u, double z, signed char sv, hx_stream_t st) {
-    return tag_box<double>(method, U, T, tags, vb, dx, dy, time, h, u, z, sv, (cudaStream_t)st);
+    return tag_box<double>(method, U, T, tags, vb, dx, dy, time, h, u, z, sv, false, (cudaStream_t)st);
+}
+int hx_tag_level_f64(int method, const hx_array4_f64* U, const hx_array4_f64* T, hx_array4_i8* tags, hx_box vb,
+                     double dx, double dy, double time, double h, double u, double z, signed char sv, hx_stream_t st) {
+    return tag_box<double>(method, U, T, tags, vb, dx, dy, time, h, u, z, sv, true, (cudaStream_t)st);
 }
 int hx_tag_box_f32(int method, const hx_array4_f32* U, const hx_array4_f32* T, hx_array4_i8* tags, hx_box vb,
                    float dx, float dy, float time, float h, float u, float z, signed char sv, hx_stream_t st) {
-    return tag_box<float>(method, U, T, tags, vb, dx, dy, time, h, u, z, sv, (cudaStream_t)st);
+    return tag_box<float>(method, U, T, tags, vb, dx, dy, time, h, u, z, sv, false, (cudaStream_t)st);
+}
+int hx_tag_level_f32(int method, const hx_array4_f32* U, const hx_array4_f32* T, hx_array4_i8* tags, hx_box vb,
+                     float dx, float dy, float time, float h, float u, float z, signed char sv, hx_stream_t st) {
+    return tag_box<float>(method, U, T, tags, vb, dx, dy, time, h, u, z, sv, true, (cudaStream_t)st);
 }
 int hx_masked_average_down_box_f64(const hx_array4_f64* fine, hx_array4_f64* crse, hx_box cb, int scomp, int ccomp,
                                    int ncomp, int rx, int ry, double fv, double nodata, hx_stream_t st) {

@@ -20,7 +20,7 @@ namespace hx {
     template cudaError_t launch_dt_reduce<R, false>(const Cells3<R>&, const Plane<R>&, const IBox&, R, R,      \
                                                     DtAccum*, cudaStream_t);                                   \
     template cudaError_t launch_tag<R>(int, const V4<R>&, const V4<R>&, const V4<signed char>&, const IBox&, R, \
-                                       R, R, R, R, R, signed char, cudaStream_t);                              \
+                                       R, R, R, R, R, signed char, bool, cudaStream_t);                           \
     template cudaError_t launch_masked_avgdown<R>(const V4<R>&, const V4<R>&, const IBox&, int, int, int, int,  \
                                                   int, R, R, cudaStream_t);                                     \
     template cudaError_t launch_average_down<R>(const V4<R>&, const V4<R>&, const IBox&, int, int, int, int, int,  \

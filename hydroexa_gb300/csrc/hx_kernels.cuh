@@ -2082,49 +2082,116 @@ __global__ void __launch_bounds__(NT) k_dt_reduce(Cells3<R> U, Plane<R> Z, IBox 
 
 // ---------------------------------------------------------------------------
 // tag_cells_Impl (HydrostaticRoe.cpp:109-169 method 1; Roe.cpp:121-179 method 0).
+//
+// A cell is tagged when a gradient's length is above a threshold, so each length is first bounded in float from
+// the leading bits of the differences (h, z: exact differences; |u|: within 2^-18 of the two speeds) and only
+// cells whose bounds hold the threshold evaluate the reference's formula, whose 25 divisions and roots on the FP64
+// pipe bound the kernel before.  A regrid's tags and restrictions on 1024 x 896 cells: 0.49 -> 0.075 ms.  The tags
+// are those of the formula everywhere.  CLAMP: the views hold no ghosts; a neighbour outside a view is its edge
+// cell, which is the ghost of every boundary rule here (a wall's first ghost mirrors the edge cell, and the
+// momentum's sign does not enter).
 // ---------------------------------------------------------------------------
-template <class R>
+struct TagTh {
+    float h, u, z;        // thresholds in float, negative where float cannot decide (outside 1e-15 .. 1e15)
+    float i2dx, i2dy;     // 1 / (2 dx), 1 / (2 dy)
+};
+template <bool CLAMP, class T> __device__ __forceinline__ T tag_ld(const V4<T>& v, int i, int j, int c) {
+    if constexpr (CLAMP) {
+        i = i < v.lo0 ? v.lo0 : (i > v.hi0 ? v.hi0 : i);
+        j = j < v.lo1 ? v.lo1 : (j > v.hi1 ? v.hi1 : j);
+    }
+    return v.ld(i, j, c);
+}
+// 1: the length of (gx, gy), known within (ex, ey), is above th; 0: it is not; 2: undecided
+__device__ __forceinline__ int tag_screen(float gx, float gy, float ex, float ey, float th) {
+    const float ax = fabsf(gx), ay = fabsf(gy), t2 = th * th;
+    const float lx = fmaxf(ax - ex, 0.f), ly = fmaxf(ay - ey, 0.f), hx = ax + ex, hy = ay + ey;
+    const float lo = (lx * lx + ly * ly) * (1.f - 0x1p-15f), hi = (hx * hx + hy * hy) * (1.f + 0x1p-15f);
+    if (!(th > 0.f)) return 2;
+    return (lo > t2) & (hi < 1e30f) ? 1 : (hi < t2 ? 0 : 2);
+}
+__device__ __forceinline__ float tag_f32(double x) { return f32_lead(x); }
+__device__ __forceinline__ float tag_f32(float x) { return x; }
+__device__ __forceinline__ bool tag_thin(double h) { return sbits(h) < 0x3EB0C6F7A0B5ED8Dll; }  // h < 1e-6
+__device__ __forceinline__ bool tag_thin(float h) { return h < 1.0e-6f; }
+__device__ __forceinline__ bool bed_is(double z, double) { return sbits(z) == kNodataRoughBits; }  // z == -9999
+__device__ __forceinline__ bool bed_is(float z, float) { return z == -9999.0f; }
+
+template <class R, bool CLAMP>
+__device__ __noinline__ bool tag_formula(const V4<R>& U, const V4<R>& T, int i, int j, R dx, R dy, R h_th, R u_th,
+                                         R z_th, int ask) {
+    auto len = [&](R ex, R wx, R nx, R sx) -> R {
+        // the reference divides by the double 2.0 * dx and stores the quotient in Real
+        const R gx = (R)((double)(ex - wx) / (2.0 * (double)dx));
+        const R gy = (R)((double)(nx - sx) / (2.0 * (double)dy));
+        return sqrt(gx * gx + gy * gy);
+    };
+    auto umag = [&](int ii, int jj) -> R {
+        const R hh = tag_ld<CLAMP>(U, ii, jj, 0);
+        if (hh < R(1.0e-6)) return R(0);
+        const R uu = tag_ld<CLAMP>(U, ii, jj, 1) / hh, vv = tag_ld<CLAMP>(U, ii, jj, 2) / hh;
+        return sqrt(uu * uu + vv * vv);
+    };
+    bool tag = false;
+    if (ask & 1)
+        tag = len(tag_ld<CLAMP>(U, i + 1, j, 0), tag_ld<CLAMP>(U, i - 1, j, 0), tag_ld<CLAMP>(U, i, j + 1, 0),
+                  tag_ld<CLAMP>(U, i, j - 1, 0)) > h_th;
+    if (!tag && (ask & 2))
+        tag = len(tag_ld<CLAMP>(T, i + 1, j, 0), tag_ld<CLAMP>(T, i - 1, j, 0), tag_ld<CLAMP>(T, i, j + 1, 0),
+                  tag_ld<CLAMP>(T, i, j - 1, 0)) > z_th;
+    if (!tag && (ask & 4)) tag = len(umag(i + 1, j), umag(i - 1, j), umag(i, j + 1), umag(i, j - 1)) > u_th;
+    return tag;
+}
+
+template <class R, bool CLAMP>
 __global__ void __launch_bounds__(NT) k_tag(int method, V4<R> U, V4<R> T, V4<signed char> tags, IBox vb, R dx, R dy,
-                                            R time, R h_th, R u_th, R z_th, signed char set_value) {
+                                            R time, R h_th, R u_th, R z_th, TagTh f, signed char set_value) {
     const int i = vb.lo0 + blockIdx.x * TX + (threadIdx.x & (TX - 1));
     const int j = vb.lo1 + blockIdx.y * TY + threadIdx.x / TX;
     if (i > vb.hi0 || j > vb.hi1) return;
-    const R zE = T.ld(i + 1, j, 0), zW = T.ld(i - 1, j, 0), zN = T.ld(i, j + 1, 0), zS = T.ld(i, j - 1, 0);
+    const R zE = tag_ld<CLAMP>(T, i + 1, j, 0), zW = tag_ld<CLAMP>(T, i - 1, j, 0);
+    const R zN = tag_ld<CLAMP>(T, i, j + 1, 0), zS = tag_ld<CLAMP>(T, i, j - 1, 0);
     if (method == HX_METHOD_HYDROSTATIC_ROE) {
-        if (is_nodata(zE) || is_nodata(zW) || is_nodata(zN) || is_nodata(zS)) return;
+        if (is_nodata(zE) | is_nodata(zW) | is_nodata(zN) | is_nodata(zS)) return;
     } else {
-        if ((double)zE == -9999.0 || (double)zW == -9999.0 || (double)zN == -9999.0 || (double)zS == -9999.0) return;
+        if (bed_is(zE, zE) | bed_is(zW, zW) | bed_is(zN, zN) | bed_is(zS, zS)) return;
     }
-    bool tag = false;
-    {
-        // the reference divides by the double 2.0 * dx and stores the quotient in Real
-        const R dhdx = (R)((double)(U.ld(i + 1, j, 0) - U.ld(i - 1, j, 0)) / (2.0 * (double)dx));
-        const R dhdy = (R)((double)(U.ld(i, j + 1, 0) - U.ld(i, j - 1, 0)) / (2.0 * (double)dy));
-        if (sqrt(dhdx * dhdx + dhdy * dhdy) > h_th) tag = true;
+    const R hE = tag_ld<CLAMP>(U, i + 1, j, 0), hW = tag_ld<CLAMP>(U, i - 1, j, 0);
+    const R hN = tag_ld<CLAMP>(U, i, j + 1, 0), hS = tag_ld<CLAMP>(U, i, j - 1, 0);
+    int r = tag_screen(tag_f32(hE - hW) * f.i2dx, tag_f32(hN - hS) * f.i2dy, 0.f, 0.f, f.h);
+    int ask = r == 2 ? 1 : 0;
+    if (r != 1 && (double)time <= 1.0e-8) {
+        r = tag_screen(tag_f32(zE - zW) * f.i2dx, tag_f32(zN - zS) * f.i2dy, 0.f, 0.f, f.z);
+        ask |= r == 2 ? 2 : 0;
     }
-    auto umag = [&](int ii, int jj) -> R {
-        const R hh = U.ld(ii, jj, 0);
-        if (hh < R(1.0e-6)) return R(0);
-        const R uu = U.ld(ii, jj, 1) / hh, vv = U.ld(ii, jj, 2) / hh;
-        return sqrt(uu * uu + vv * vv);
-    };
-    if (!tag && (double)time <= 1.0e-8) {
-        const R dzdx = (R)((double)(zE - zW) / (2.0 * (double)dx));
-        const R dzdy = (R)((double)(zN - zS) / (2.0 * (double)dy));
-        if (sqrt(dzdx * dzdx + dzdy * dzdy) > z_th) tag = true;
+    if (r != 1) {
+        auto speed = [&](R h, int ii, int jj) -> float {
+            if (tag_thin(h)) return 0.f;
+            const float a = tag_f32(tag_ld<CLAMP>(U, ii, jj, 1)), b = tag_f32(tag_ld<CLAMP>(U, ii, jj, 2));
+            return fast_sqrt(a * a + b * b) * f_rcp(tag_f32(h));
+        };
+        const float uE = speed(hE, i + 1, j), uW = speed(hW, i - 1, j), uN = speed(hN, i, j + 1), uS = speed(hS, i, j - 1);
+        // (1e-12: squares below the float range)
+        r = tag_screen((uE - uW) * f.i2dx, (uN - uS) * f.i2dy, (0x1p-18f * (uE + uW) + 1e-12f) * f.i2dx,
+                       (0x1p-18f * (uN + uS) + 1e-12f) * f.i2dy, f.u);
+        ask |= r == 2 ? 4 : 0;
     }
-    if (!tag) {
-        const R uE = umag(i + 1, j), uW = umag(i - 1, j), uN = umag(i, j + 1), uS = umag(i, j - 1);
-        const R dudx = (R)((double)(uE - uW) / (2.0 * (double)dx));
-        const R dudy = (R)((double)(uN - uS) / (2.0 * (double)dy));
-        if (sqrt(dudx * dudx + dudy * dudy) > u_th) tag = true;
-    }
-    if (tag) tags.ref(i, j, 0) = set_value;
+    if (r != 1 && ask && tag_formula<R, CLAMP>(U, T, i, j, dx, dy, h_th, u_th, z_th, ask)) r = 1;
+    if (r == 1) tags.ref(i, j, 0) = set_value;
 }
 
 // ---------------------------------------------------------------------------
 // masked_avgdown_with_vol over a coarse box (MaskedAverageDown.H:64-104).
 // ---------------------------------------------------------------------------
+// (double)fabs(x) > 1e-3, false for a NaN, on the bit pattern (a float is above the double 1e-3 from 0.001f on).
+__device__ __forceinline__ bool apart_1em3(double x) {
+    const long long b = sbits(x) & 0x7FFFFFFFFFFFFFFFll;
+    return (b > 0x3F50624DD2F1A9FCll) & (b <= 0x7FF0000000000000ll);
+}
+__device__ __forceinline__ bool apart_1em3(float x) {
+    const int b = sbits(x) & 0x7FFFFFFF;
+    return (b >= 0x3A83126F) & (b <= 0x7F800000);
+}
 template <class R>
 __global__ void __launch_bounds__(NT) k_masked_avgdown(V4<R> fine, V4<R> crse, IBox cb, int scomp, int ccomp,
                                                        int ncomp, int rx, int ry, R fv, R nodata) {
@@ -2137,13 +2204,13 @@ __global__ void __launch_bounds__(NT) k_masked_avgdown(V4<R> fine, V4<R> crse, I
         for (int jr = 0; jr < ry; ++jr)
             for (int ir = 0; ir < rx; ++ir) {
                 const R val = fine.ld(i * rx + ir, j * ry + jr, scomp + n);
-                if (!isnan(val) && (double)fabs(val - nodata) > 1e-3) {
+                if (apart_1em3(val - nodata)) {
                     ++nvalid;
                     cv += fv;
                     cd += val * fv;
                 }
             }
-        crse.ref(i, j, ccomp + n) = (nvalid * 2 >= rx * ry && cv > R(0)) ? cd / cv : nodata;
+        crse.ref(i, j, ccomp + n) = (nvalid * 2 >= rx * ry && cv > R(0)) ? ieee_quot(cd, cv) : nodata;
     }
 }
 
@@ -2614,8 +2681,13 @@ cudaError_t launch_points(int method, long n, const R* st, const R* aux, R* out,
 
 template <class R>
 cudaError_t launch_tag(int method, const V4<R>& U, const V4<R>& T, const V4<signed char>& tags, const IBox& vb, R dx,
-                       R dy, R time, R h_th, R u_th, R z_th, signed char set_value, cudaStream_t st) {
-    k_tag<R><<<tile_grid(vb, TX, TY), NT, 0, st>>>(method, U, T, tags, vb, dx, dy, time, h_th, u_th, z_th, set_value);
+                       R dy, R time, R h_th, R u_th, R z_th, signed char set_value, bool clamp, cudaStream_t st) {
+    auto f32 = [](double th) { return th >= 1e-15 && th <= 1e15 ? (float)th : -1.f; };
+    TagTh f{f32(h_th), f32(u_th), f32(z_th), (float)(0.5 / (double)dx), (float)(0.5 / (double)dy)};
+    const auto normal = [](float v) { return v >= 1e-15f && v <= 1e15f; };
+    if (!normal(f.i2dx) || !normal(f.i2dy)) f.h = f.u = f.z = -1.f;
+    auto k = clamp ? k_tag<R, true> : k_tag<R, false>;
+    k<<<tile_grid(vb, TX, TY), NT, 0, st>>>(method, U, T, tags, vb, dx, dy, time, h_th, u_th, z_th, f, set_value);
     return cudaGetLastError();
 }
 

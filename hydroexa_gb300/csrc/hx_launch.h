@@ -44,7 +44,7 @@ template <bool FAST> cudaError_t launch_rcp(long n, const double* x, double* y, 
 
 template <class R>
 cudaError_t launch_tag(int method, const V4<R>& U, const V4<R>& T, const V4<signed char>& tags, const IBox& vb, R dx,
-                       R dy, R time, R h_th, R u_th, R z_th, signed char set_value, cudaStream_t st);
+                       R dy, R time, R h_th, R u_th, R z_th, signed char set_value, bool clamp, cudaStream_t st);
 
 template <class R>
 cudaError_t launch_masked_avgdown(const V4<R>& fine, const V4<R>& crse, const IBox& cb, int scomp, int ccomp,

@@ -103,51 +103,20 @@ class BaseSolver:
     def tag_cells(self, tags: torch.Tensor, U: torch.Tensor, terrain: torch.Tensor, geom: Geometry, lev: int,
                   time: float, phys_params: PhysicsParameters, set_value: int = 2) -> None:
         """Tag the valid cells of a single-box level.  The one-cell ghost ring the
-        stencil reads is generated with the level's boundary rules (the
-        reference reads whatever its MultiFab ghosts hold)."""
-        Ug = _pad_state(U, geom)
-        Tg = _pad_terrain(terrain)
-        tg = torch.zeros((geom.ny + 2, geom.nx + 2), dtype=torch.int8, device=U.device)
-        tg[1:-1, 1:-1] = tags
+        stencil reads follows the level's boundary rules (the reference reads
+        whatever its MultiFab ghosts hold): each ghost holds its edge cell,
+        a wall's up to a momentum sign that the tags do not depend on."""
+        tg = tags if tags.dtype == torch.int8 and tags.is_contiguous() else tags.to(torch.int8).contiguous()
         R = ctypes.c_double if U.dtype == torch.float64 else ctypes.c_float
         sfx = "f64" if U.dtype == torch.float64 else "f32"
         th = (phys_params.h_grad_thresh[lev], phys_params.umag_grad_thresh[lev], phys_params.z_grad_thresh[lev])
-        rc = getattr(capi.lib(), f"hx_tag_box_{sfx}")(
-            self.method, ctypes.byref(array4(Ug, (-1, -1))), ctypes.byref(array4(Tg, (-1, -1))),
-            ctypes.byref(array4(tg, (-1, -1))), box((0, 0), (geom.nx - 1, geom.ny - 1)), R(geom.dx), R(geom.dy),
+        rc = getattr(capi.lib(), f"hx_tag_level_{sfx}")(
+            self.method, ctypes.byref(array4(U.contiguous())), ctypes.byref(array4(terrain.contiguous())),
+            ctypes.byref(array4(tg)), box((0, 0), (geom.nx - 1, geom.ny - 1)), R(geom.dx), R(geom.dy),
             R(time), *(R(x) for x in th), set_value, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
-        capi.check(rc, "hx_tag_box")
-        tags.copy_(tg[1:-1, 1:-1])
-
-
-def _mirror(a: torch.Tensor, dim: int, lo_rule: str, hi_rule: str) -> torch.Tensor:
-    def ghost(edge_idx, mirror_idx, rule):
-        if rule == "edge":
-            return a.narrow(dim, edge_idx, 1)
-        g = a.narrow(dim, mirror_idx, 1)
-        return -g if rule == "odd" else g
-    n = a.shape[dim]
-    return torch.cat([ghost(0, 0, lo_rule), a, ghost(n - 1, n - 1, hi_rule)], dim=dim)
-
-
-def _rule(code: int, kind: str) -> str:
-    if code != 0:
-        return "edge"
-    return "odd" if kind == "normal" else "even"
-
-
-def _pad_state(U, g: Geometry):
-    out = []
-    for c, (kx, ky) in enumerate((("scalar", "scalar"), ("normal", "tangential"), ("tangential", "normal"))):
-        p = _mirror(U[c], 1, _rule(g.bc_lo[0], kx), _rule(g.bc_hi[0], kx))
-        p = _mirror(p, 0, _rule(g.bc_lo[1], ky), _rule(g.bc_hi[1], ky))
-        out.append(p)
-    return torch.stack(out).contiguous()
-
-
-def _pad_terrain(T):
-    out = [_mirror(_mirror(T[c], 1, "edge", "edge"), 0, "edge", "edge") for c in range(T.shape[0])]
-    return torch.stack(out).contiguous()
+        capi.check(rc, "hx_tag_level")
+        if tg is not tags:
+            tags.copy_(tg)
 
 
 class Roe(BaseSolver):

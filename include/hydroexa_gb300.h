@@ -270,6 +270,16 @@ int hx_tag_box_f64(int method, const hx_array4_f64* U, const hx_array4_f64* T, h
 int hx_tag_box_f32(int method, const hx_array4_f32* U, const hx_array4_f32* T, hx_array4_i8* tags, hx_box valid,
                    float dx, float dy, float time, float h_thresh, float umag_thresh, float z_thresh,
                    signed char set_value, hx_stream_t stream);
+/*
+ * The same on a single-box level without ghosts: U and T cover the box, and a neighbour outside a view is the
+ * view's edge cell (the first ghost of every physical boundary rule; the momentum's sign does not enter).
+ */
+int hx_tag_level_f64(int method, const hx_array4_f64* U, const hx_array4_f64* T, hx_array4_i8* tags, hx_box valid,
+                     double dx, double dy, double time, double h_thresh, double umag_thresh, double z_thresh,
+                     signed char set_value, hx_stream_t stream);
+int hx_tag_level_f32(int method, const hx_array4_f32* U, const hx_array4_f32* T, hx_array4_i8* tags, hx_box valid,
+                     float dx, float dy, float time, float h_thresh, float umag_thresh, float z_thresh,
+                     signed char set_value, hx_stream_t stream);
 
 /*
  * NODATA-aware volume-weighted restriction of the coarse box crse_box

@@ -630,57 +630,165 @@ __host__ __device__ __forceinline__ void roe_hydrostatic_fast(R hi, R ui, R vi, 
 // guard (include/solvers/kernels/Roe.H:51-309), direction fixed at compile
 // time.  Outputs F, S-, S+ in global coordinates.
 // ----------------------------------------------------------------------------
-template <class R, bool FAST, int DIR>
-__host__ __device__ __forceinline__ void roe_classic(R hi, R hui, R hvi, R zi, R ni, R hj, R huj, R hvj, R zj, R nj, R dx,
-                                            R F[3], R Sm[3], R Sp[3]) {
-    using C = Cst<R>;
-    const R T12 = C::tol12, TD = C::toldry;
-    hi = (hi >= TD) ? hi : R(0);
-    hj = (hj >= TD) ? hj : R(0);
-    R si, sj, ui, vi, uj, vj;
-    if constexpr (!FAST) {
-        si = (hi > R(0)) ? sqrt(hi) : R(0);
-        sj = (hj > R(0)) ? sqrt(hj) : R(0);
-        ui = (hi > R(0)) ? hui / hi : R(0);
-        vi = (hi > R(0)) ? hvi / hi : R(0);
-        uj = (hj > R(0)) ? huj / hj : R(0);
-        vj = (hj > R(0)) ? hvj / hj : R(0);
+// FP64 (both forms): quotients and roots on the integer pipe, correctly rounded (hx_ieee.cuh), comparisons on bit
+// patterns, and the positivity guard's quotients only where float bounds cannot rule the guard out.  The exact
+// form's results are the formula's bit for bit.  The fast form contracts, forms the fluxes with the halves folded
+// in, and takes the friction's power from classic_rh43.
+// 0 + x: x, with -0 as +0.
+__device__ __forceinline__ float zero_plus(float x) { return 0.f + x; }
+__device__ __forceinline__ double zero_plus(double x) { return sbits(x) == (long long)0x8000000000000000ull ? 0.0 : x; }
+// x >= 0, x < 0, false for a NaN
+__device__ __forceinline__ bool cl_ge0(double x) { return ge_num(x, 0ll) | (sbits(x) == (long long)0x8000000000000000ull); }
+__device__ __forceinline__ bool cl_ge0(float x) { return x >= 0.f; }
+__device__ __forceinline__ bool cl_gt0(double x) { return ge_num(x, 1ll); }
+__device__ __forceinline__ bool cl_gt0(float x) { return x > 0.f; }
+__device__ __forceinline__ bool cl_lt0(double x) {
+    return (unsigned long long)sbits(x) - 0x8000000000000001ull < 0x7FF0000000000000ull;
+}
+__device__ __forceinline__ bool cl_lt0(float x) { return x < 0.f; }
+// |x| > tol12
+__device__ __forceinline__ bool cl_above12(double x) {
+    return (unsigned long long)((sbits(x) & 0x7FFFFFFFFFFFFFFFll) - (Cst<double>::tol12_bits + 1)) <=
+           (unsigned long long)(0x7FF0000000000000ll - (Cst<double>::tol12_bits + 1));
+}
+__device__ __forceinline__ bool cl_above12(float x) { return fabsf(x) > Cst<float>::tol12; }
+__device__ __forceinline__ bool cl_is0(double x) { return (sbits(x) << 1) == 0; }
+__device__ __forceinline__ bool cl_is0(float x) { return x == 0.f; }
+__device__ __forceinline__ bool cl_dry(double h) { return !ge_num(h, Cst<double>::toldry_bits); }
+__device__ __forceinline__ bool cl_dry(float h) { return !(h >= Cst<float>::toldry); }
+__device__ __forceinline__ bool cl_above_dry(double h) { return ge_num(h, Cst<double>::toldry_bits + 1); }
+__device__ __forceinline__ bool cl_above_dry(float h) { return h > Cst<float>::toldry; }
+// no roughness and averages whose squares stay finite: the friction term is a zero with um's sign
+__device__ __forceinline__ bool cl_no_friction(double nm, double um, double vm) {
+    const unsigned top = (1023u + 500u) << 20;
+    return ((sbits(nm) << 1) == 0) & (((unsigned)__double2hiint(um) & 0x7FFFFFFFu) < top) &
+           (((unsigned)__double2hiint(vm) & 0x7FFFFFFFu) < top);
+}
+__device__ __forceinline__ bool cl_no_friction(float, float, float) { return false; }
+__device__ __forceinline__ double cl_signed_zero(double x) { return __hiloint2double(__double2hiint(x) & (int)0x80000000, 0); }
+__device__ __forceinline__ float cl_signed_zero(float x) { return copysignf(0.f, x); }
+// a / d with the divisor unpacked once (doubles)
+struct ClassicDiv64 {
+    IeeeDivisor d;
+    __device__ __forceinline__ explicit ClassicDiv64(double b) : d(ieee_divisor(b)) {}
+    __device__ __forceinline__ double operator()(double a) const { return ieee_div(a, d); }
+};
+struct ClassicDiv32 {
+    float b;
+    __device__ __forceinline__ explicit ClassicDiv32(float x) : b(x) {}
+    __device__ __forceinline__ float operator()(float a) const { return a / b; }
+};
+// Whether the guard (hi1 < -toldry < toldry < hj3 or the other way round) can hold, from float estimates whose
+// error is below 2^-18 of the terms.
+__device__ __forceinline__ bool classic_guard_possible(double hi, double a0, double b0, double l0s, double hj, double a2,
+                                                       double b2, double l2s) {
+    const float h1 = f32_lead(hi), x1 = f32_lead(a0), q1 = f32_lead(b0) * f_rcp(f32_lead(l0s));
+    const float h3 = f32_lead(hj), x3 = f32_lead(a2), q3 = f32_lead(b2) * f_rcp(f32_lead(l2s));
+    const float s1 = h1 + x1 - q1, e1 = 0x1p-18f * (fabsf(h1) + fabsf(x1) + fabsf(q1));
+    const float s3 = h3 - x3 + q3, e3 = 0x1p-18f * (fabsf(h3) + fabsf(x3) + fabsf(q3));
+    return !((s1 - e1 > -0.9e-6f) & (s3 - e3 > -0.9e-6f));
+}
+__device__ __forceinline__ bool classic_guard_possible(float, float, float, float, float, float, float, float) {
+    return true;
+}
+
+// What the classic faces need of a cell, the same for its four faces: the depth (0 where dry), its square root and
+// the velocities.
+template <class R> struct ClassicCell {
+    R h, s, u, v, z, n;
+};
+template <class R, bool FAST>
+__device__ __forceinline__ void classic_cell(R h, R hu, R hv, R& s, R& u, R& v) {
+    const bool wet = !cl_dry(h);
+    const R hd = wet ? h : R(0);
+    if constexpr (FAST && sizeof(R) == 4) {
+        s = fast_sqrt(hd);
+        const R r = wet ? R(1) / hd : R(0);
+        u = hu * r;
+        v = hv * r;
     } else {
-        si = fast_sqrt(hi);
-        sj = fast_sqrt(hj);
-        const R ri = (hi > R(0)) ? R(1) / hi : R(0);
-        const R rj = (hj > R(0)) ? R(1) / hj : R(0);
-        ui = hui * ri; vi = hvi * ri; uj = huj * rj; vj = hvj * rj;
+        using Div = std::conditional_t<sizeof(R) == 8, ClassicDiv64, ClassicDiv32>;
+        s = wet ? ieee_root(hd) : R(0);
+        const Div q(wet ? hd : R(1));
+        u = wet ? q(hu) : R(0);
+        v = wet ? q(hv) : R(0);
     }
+}
+// The FP64 fast form's fluxes, sources apart: the same sums with the halves folded in and the contact wave's
+// w1 c = |u| (dhv - vm dh) / 2 without its division.
+template <class R>
+__device__ __forceinline__ void classic_flux_fast(R hi, R uni, R uti, R hj, R unj, R utj, R um, R vm, R l0, R l2, R a0,
+                                                  R a2, R dv, R& f0, R& f1, R& f2) {
+    const R qi = hi * uni, qj = hj * unj;
+    const R w0 = fabs(l0) * (R(0.5) * a0), w2 = fabs(l2) * (R(0.5) * a2), w = w0 + w2;
+    f0 = fma(R(0.5), qi + qj, -w);
+    const R c = fma(Cst<R>::half_g, fma(hj, hj, hi * hi), fma(qj, unj, qi * uni));
+    f1 = fma(R(0.5), c, -fma(w2, l2, w0 * l0));
+    f2 = fma(R(0.5), fma(-fabs(um), dv, fma(qj, utj, qi * uti)), -(w * vm));
+}
+// 1 / max(toldry, hm^(4/3)) for a wet mean depth: r = hm^(-1/3) by a third-order step from its float seed (error
+// ~e^3 / 6 for e below 2^-20: within the rounding), to the fourth power; 1 / toldry is the cap.
+__device__ __forceinline__ double classic_rh43(double hm) {
+    const double r = f64_widen(rcbrtf(f32_lead(hm)));
+    const double e = fma(-hm, r * r * r, 1.0);
+    const double q = fma(r, e * fma(2.0 / 9.0, e, 1.0 / 3.0), r);
+    const double q2 = q * q, q4 = q2 * q2;
+    return gt_bits(q4, 0x412E848000000000ll) ? 1.0e6 : q4;
+}
+__device__ __forceinline__ float classic_rh43(float hm) { return 1.0f / smax(Cst<float>::toldry, hm * cbrtf(hm)); }
+
+template <class R, bool FAST, int DIR>
+__device__ __forceinline__ void roe_classic(const ClassicCell<R>& ci_, const ClassicCell<R>& cj_, R dx, R F[3], R Sm[3],
+                                            R Sp[3]) {
+    using C = Cst<R>;
+    using Div = std::conditional_t<sizeof(R) == 8, ClassicDiv64, ClassicDiv32>;
+    constexpr bool F64 = FAST && sizeof(R) == 8;
+    const R T12 = C::tol12, TD = C::toldry;
+    const R hi = cl_dry(ci_.h) ? R(0) : ci_.h, hj = cl_dry(cj_.h) ? R(0) : cj_.h;
+    const R si = ci_.s, sj = cj_.s, ui = ci_.u, vi = ci_.v, uj = cj_.u, vj = cj_.v;
+    const R zi = ci_.z, zj = cj_.z, ni = ci_.n, nj = cj_.n;
     R uni, uti, unj, utj;
     if (DIR == 0) { uni = ui; uti = vi; unj = uj; utj = vj; }
     else { uni = vi; uti = -ui; unj = vj; utj = -uj; }
     const R hsum = hi + hj;
-    const R hm = (R(0.5) * hsum > TD) ? R(0.5) * hsum : TD;
-    const R cm = FAST ? fast_sqrt(C::g * hm) : sqrt(C::g * hm);
-    const R sden = si + sj + T12;
-    const R um = (uni * si + unj * sj) / sden;
-    const R vm = (uti * si + utj * sj) / sden;
+    const R half = R(0.5) * hsum;
+    const R hm = cl_above_dry(half) ? half : TD;
+    const R cm = FAST ? fast_sqrt(C::g * hm) : ieee_root(C::g * hm);
+    const Div sden(si + sj + T12);
+    const R um = sden(uni * si + unj * sj);
+    const R vm = sden(uti * si + utj * sj);
     R l0 = um - cm;
     const R l1 = um;
     R l2 = um + cm;
     {
-        R ci, cj;
-        if constexpr (!FAST) { ci = sqrt(C::g * hi); cj = sqrt(C::g * hj); }
-        else { ci = C::sqrt_g * si; cj = C::sqrt_g * sj; }
-        R ei = uni - ci, ej = unj - cj;
-        if (ei < R(0) && ej > R(0)) l0 = ei * (ej - l0) / (ej - ei);
-        ei = uni + ci;
-        ej = unj + cj;
-        if (ei < R(0) && ej > R(0)) l2 = ej * (l2 - ei) / (ej - ei);
+        // the fixes need e_i < 0 < e_j for e = u -+ c: in FP64 ruled out in float where a sign is certain (as in
+        // roe_hydrostatic_fast)
+        bool rule0 = false, rule2 = false;
+        if constexpr (sizeof(R) == 8) {
+            const float ui32 = f32_lead(uni), uj32 = f32_lead(unj);
+            const float ci32 = 3.13209195f * f32_lead(si), cj32 = 3.13209195f * f32_lead(sj);
+            const float mi = 0x1p-16f * (fabsf(ui32) + ci32), mj = 0x1p-16f * (fabsf(uj32) + cj32);
+            rule0 = (ui32 - ci32 >= mi) | (uj32 - cj32 <= -mj);
+            rule2 = (ui32 + ci32 >= mi) | (uj32 + cj32 <= -mj);
+        }
+        if (!(rule0 & rule2)) {
+            R ci, cj;
+            if constexpr (!FAST) { ci = ieee_root(C::g * hi); cj = ieee_root(C::g * hj); }
+            else { ci = C::sqrt_g * si; cj = C::sqrt_g * sj; }
+            R ei = uni - ci, ej = unj - cj;
+            if (cl_lt0(ei) && cl_gt0(ej)) l0 = ieee_quot(ei * (ej - l0), ej - ei);
+            ei = uni + ci;
+            ej = unj + cj;
+            if (cl_lt0(ei) && cl_gt0(ej)) l2 = ieee_quot(ej * (l2 - ei), ej - ei);
+        }
     }
-    const R den = R(2) * cm + T12;
+    const Div den(fma(R(2), cm, T12));  // 2 cm is exact
     const R dh = hj - hi;
     const R dhu = hj * unj - hi * uni;
     const R dhv = hj * utj - hi * uti;
-    const R a0 = (l2 * dh - dhu) / den;
-    const R a1 = (-vm * dh + dhv) / cm;
-    const R a2 = (-l0 * dh + dhu) / den;
+    const R a0 = den(l2 * dh - dhu);
+    const R dv = -vm * dh + dhv;
+    const R a2 = den(-l0 * dh + dhu);
 
     const R dz = zj - zi;
     const R di = hi + zi;
@@ -689,89 +797,111 @@ __host__ __device__ __forceinline__ void roe_classic(R hi, R hui, R hvi, R zi, R
     R thrust, tau;
     {
         const R ta = -C::g * hm * dz;
+        const bool up = cl_ge0(dz), down = cl_lt0(dz);
         R dzt;
-        if ((dz >= R(0)) && (di < zj)) dzt = hi;
-        else if ((dz < R(0)) && (dj < zi)) dzt = hj;
+        if (up & (F64 ? okey(di) < okey(zj) : di < zj)) dzt = hi;
+        else if (down & (F64 ? okey(dj) < okey(zi) : dj < zi)) dzt = hj;
         else dzt = dz;
-        const R hr = (dz >= R(0)) ? hi : hj;
+        const R hr = up ? hi : hj;
         const R tb = -C::g * (hr - R(0.5) * fabs(dzt)) * dzt;
-        thrust = ((dz * dd >= R(0)) && (um * dz > R(0))) ? smax(ta, tb) : tb;
+        thrust = (cl_ge0(dz * dd) & cl_gt0(um * dz)) ? (F64 ? smax_i(ta, tb) : smax(ta, tb)) : tb;
         const R nm = R(0.5) * (ni + nj);
-        if constexpr (!FAST) {
-            const R sf = (nm * nm * sqrt(um * um + vm * vm) * um) / smax(TD, hm * cbrt(hm));
-            tau = C::g * hm * sf * dx;
+        // the friction term vanishes when the face roughness is zero (the fast form skips its sign too)
+        if (F64 ? cl_is0(nm) : (FAST ? nm == R(0) : cl_no_friction(nm, um, vm))) {
+            tau = FAST ? R(0) : cl_signed_zero(um);
+        } else if constexpr (F64) {
+            tau = (nm * nm * ieee_root(fma(um, um, vm * vm)) * um) * classic_rh43(hm) * (C::g * hm * dx);
         } else {
-            // the friction term vanishes identically when the face roughness is zero
-            if (nm != R(0)) {
-                const R sf = (nm * nm * sqrt(um * um + vm * vm) * um) / smax(TD, hm * cbrt(hm));
-                tau = C::g * hm * sf * dx;
-            } else {
-                tau = R(0);
-            }
+            const R sf = ieee_quot(nm * nm * ieee_root(um * um + vm * vm) * um, smax(TD, hm * cbrt(hm)));
+            tau = C::g * hm * sf * dx;
         }
     }
-    R b0 = (thrust - tau) / den;
+    R b0 = den(thrust - tau);
     const R b1 = R(0);
     R b2 = -b0;
     {
-        const R l0s = (fabs(l0) > T12) ? l0 : (l0 >= R(0) ? T12 : -T12);
-        const R l2s = (fabs(l2) > T12) ? l2 : (l2 >= R(0) ? T12 : -T12);
-        const R hi1 = hi + a0 - (b0 / l0s);
-        const R hj3 = hj - a2 + (b2 / l2s);
-        R ml = fabs(l0);
-        ml = smax(ml, fabs(l1));
-        ml = smax(ml, fabs(l2));
-        const R ldt = dx / (ml + T12);
-        const R d1 = hi - hi1;
-        const R d1s = (fabs(d1) > T12) ? d1 : (d1 >= R(0) ? T12 : -T12);
-        const R d3 = hj - hj3;
-        const R d3s = (fabs(d3) > T12) ? d3 : (d3 >= R(0) ? T12 : -T12);
-        const bool g1 = (hi1 < -TD) && (hj3 > TD);
-        const bool g3 = (hi1 > TD) && (hj3 < -TD);
-        if (g1 || g3) {
-            const R dt1 = (dx * R(0.5) / l0s) * (hi / d1s);
-            const R dt3 = (dx * R(0.5) / l2s) * (hj / d3s);
-            if (g1 && (dt1 < ldt)) {
-                const R b1min = -(hi + a0) * fabs(l0);
-                const R b3min = -(hj - a2) * l2;
-                if (-b1min >= b3min) b0 = b1min;
-                b2 = -b0;
-            }
-            if (g3 && (dt3 < ldt)) {
-                const R b1min = -(hi + a0) * fabs(l0);
-                const R b3min = -(hj - a2) * l2;
-                if (-b3min >= b1min) b2 = b3min;
-                b0 = -b2;
+        const R l0s = cl_above12(l0) ? l0 : (cl_ge0(l0) ? T12 : -T12);
+        const R l2s = cl_above12(l2) ? l2 : (cl_ge0(l2) ? T12 : -T12);
+        if (classic_guard_possible(hi, a0, b0, l0s, hj, a2, b2, l2s)) {
+            const R hi1 = hi + a0 - ieee_quot(b0, l0s);
+            const R hj3 = hj - a2 + ieee_quot(b2, l2s);
+            const bool g1 = (hi1 < -TD) && (hj3 > TD);
+            const bool g3 = (hi1 > TD) && (hj3 < -TD);
+            if (g1 || g3) {
+                R ml = fabs(l0);
+                ml = smax(ml, fabs(l1));
+                ml = smax(ml, fabs(l2));
+                const R ldt = ieee_quot(dx, ml + T12);
+                const R d1 = hi - hi1;
+                const R d1s = (fabs(d1) > T12) ? d1 : (d1 >= R(0) ? T12 : -T12);
+                const R d3 = hj - hj3;
+                const R d3s = (fabs(d3) > T12) ? d3 : (d3 >= R(0) ? T12 : -T12);
+                const R dt1 = ieee_quot(dx * R(0.5), l0s) * ieee_quot(hi, d1s);
+                const R dt3 = ieee_quot(dx * R(0.5), l2s) * ieee_quot(hj, d3s);
+                if (g1 && (dt1 < ldt)) {
+                    const R b1min = -(hi + a0) * fabs(l0);
+                    const R b3min = -(hj - a2) * l2;
+                    if (-b1min >= b3min) b0 = b1min;
+                    b2 = -b0;
+                }
+                if (g3 && (dt3 < ldt)) {
+                    const R b1min = -(hi + a0) * fabs(l0);
+                    const R b3min = -(hj - a2) * l2;
+                    if (-b3min >= b1min) b2 = b3min;
+                    b0 = -b2;
+                }
             }
         }
     }
-    R f0 = R(0.5) * (hi * uni + hj * unj);
-    R f1 = R(0.5) * (hi * uni * uni + C::half_g * hi * hi + hj * unj * unj + C::half_g * hj * hj);
-    R f2 = R(0.5) * (hi * uni * uti + hj * unj * utj);
-    R m0 = 0, m1 = 0, m2 = 0, p0 = 0, p1 = 0, p2 = 0;
-    {
-        const R w = R(0.5) * fabs(l0) * a0;
-        f0 -= w; f1 -= w * l0; f2 -= w * vm;
-        if (l0 > R(0)) { m0 += b0; m1 += b0 * l0; m2 += b0 * vm; }
-        else if (l0 < R(0)) { p0 += b0; p1 += b0 * l0; p2 += b0 * vm; }
-    }
-    {
-        const R w = R(0.5) * fabs(l1) * a1;
-        f2 -= w * cm;
-        if (l1 > R(0)) { m2 += b1 * cm; }
-        else if (l1 < R(0)) { p2 += b1 * cm; }
-    }
-    {
-        const R w = R(0.5) * fabs(l2) * a2;
-        f0 -= w; f1 -= w * l2; f2 -= w * vm;
-        if (l2 > R(0)) { m0 += b2; m1 += b2 * l2; m2 += b2 * vm; }
-        else if (l2 < R(0)) { p0 += b2; p1 += b2 * l2; p2 += b2 * vm; }
-    }
-    F[0] = f0; Sm[0] = m0; Sp[0] = p0;
-    if (DIR == 0) {
-        F[1] = f1; F[2] = f2; Sm[1] = m1; Sm[2] = m2; Sp[1] = p1; Sp[2] = p2;
+    R f0, f1, f2;
+    if constexpr (F64) {
+        classic_flux_fast(hi, uni, uti, hj, unj, utj, um, vm, l0, l2, a0, a2, dv, f0, f1, f2);
     } else {
-        F[1] = -f2; F[2] = f1; Sm[1] = -m2; Sm[2] = m1; Sp[1] = -p2; Sp[2] = p1;
+        const R a1 = ieee_quot(dv, cm);
+        f0 = R(0.5) * (hi * uni + hj * unj);
+        f1 = R(0.5) * (hi * uni * uni + C::half_g * hi * hi + hj * unj * unj + C::half_g * hj * hj);
+        f2 = R(0.5) * (hi * uni * uti + hj * unj * utj);
+        {
+            const R w = R(0.5) * fabs(l0) * a0;
+            f0 -= w; f1 -= w * l0; f2 -= w * vm;
+        }
+        {
+            const R w = R(0.5) * fabs(l1) * a1;
+            f2 -= w * cm;
+        }
+        {
+            const R w = R(0.5) * fabs(l2) * a2;
+            f0 -= w; f1 -= w * l2; f2 -= w * vm;
+        }
+    }
+    // sources: b_k on the side wave k travels to (b1 = 0: the contact wave adds a zero)
+    const bool p0 = cl_gt0(l0), n0 = cl_lt0(l0), p1 = cl_gt0(l1), n1 = cl_lt0(l1), p2 = cl_gt0(l2), n2 = cl_lt0(l2);
+    const R s01 = b0 * l0, s02 = b0 * vm, s21 = b2 * l2, s22 = b2 * vm;
+    R m0, m1, m2, q0, q1, q2;
+    const unsigned lanes = __activemask();
+    if (__any_sync(lanes, (p0 & p2) | (n0 & n2) | bits_nonfinite(cm))) {  // 0 += x per wave, in the reference's order
+        const R s12 = b1 * cm;
+        auto sum = [](bool c0, R x0, bool c1, R x1, bool c2, R x2) -> R {
+            R m = R(0);
+            if (c0) m += x0;
+            if (c1) m += x1;
+            if (c2) m += x2;
+            return m;
+        };
+        m0 = sum(p0, b0, false, R(0), p2, b2); m1 = sum(p0, s01, false, R(0), p2, s21);
+        m2 = sum(p0, s02, p1, s12, p2, s22);
+        q0 = sum(n0, b0, false, R(0), n2, b2); q1 = sum(n0, s01, false, R(0), n2, s21);
+        q2 = sum(n0, s02, n1, s12, n2, s22);
+    } else {  // one wave to a side at most (every lane subcritical): its term, a -0 as +0
+        auto one = [](bool c0, R x0, bool c2, R x2) -> R { return zero_plus(c0 ? x0 : (c2 ? x2 : R(0))); };
+        m0 = one(p0, b0, p2, b2); m1 = one(p0, s01, p2, s21); m2 = one(p0, s02, p2, s22);
+        q0 = one(n0, b0, n2, b2); q1 = one(n0, s01, n2, s21); q2 = one(n0, s02, n2, s22);
+    }
+    F[0] = f0; Sm[0] = m0; Sp[0] = q0;
+    if (DIR == 0) {
+        F[1] = f1; F[2] = f2; Sm[1] = m1; Sm[2] = m2; Sp[1] = q1; Sp[2] = q2;
+    } else {
+        F[1] = -f2; F[2] = f1; Sm[1] = -m2; Sm[2] = m1; Sp[1] = -q2; Sp[2] = q1;
     }
 }
 

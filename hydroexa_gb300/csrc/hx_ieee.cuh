@@ -84,15 +84,10 @@ template <bool CHECKED = true> __device__ __forceinline__ double ieee_div(double
     if constexpr (!CHECKED) {
         return __hiloint2double((int)(ae != 0u ? vh : sg), (int)(ae != 0u ? vl : 0u));
     } else {
-        double v = __hiloint2double((int)vh, (int)vl);
-        const bool ok = ae - 0x00100000u < 0x7FE00000u && d.e - 0x00100000u < 0x7FE00000u &&
-                        ae - d.e + (1000u << 20) < (2000u << 20);
-        if (!ok) {
-            if ((ae | (ahi & 0xFFFFFu) | alo) == 0u && d.e - 0x00100000u < 0x7FE00000u)
-                v = __hiloint2double((int)sg, 0);
-            else
-                v = ieee_div_slow(a, d.b);
-        }
+        const bool dok = d.e - 0x00100000u < 0x7FE00000u, zero = (ae | (ahi & 0xFFFFFu) | alo) == 0u;
+        const bool ok = dok & (zero | ((ae - 0x00100000u < 0x7FE00000u) & (ae - d.e + (1000u << 20) < (2000u << 20))));
+        double v = __hiloint2double((int)(zero ? sg : vh), (int)(zero ? 0u : vl));
+        if (!ok) v = ieee_div_slow(a, d.b);
         return v;
     }
 }
@@ -136,8 +131,9 @@ template <bool CHECKED = true> __device__ __forceinline__ double ieee_sqrt(doubl
     if constexpr (!CHECKED) {
         return __hiloint2double((int)(hi != 0u ? vh : 0u), (int)(hi != 0u ? vl : 0u));
     } else {
-        double v = __hiloint2double((int)vh, (int)vl);
-        if (hi - 0x00100000u >= 0x7FE00000u) v = (hi | lo) == 0u ? 0.0 : ieee_sqrt_slow(x);
+        const bool zero = (hi | lo) == 0u;
+        double v = __hiloint2double((int)(zero ? 0u : vh), (int)(zero ? 0u : vl));
+        if (!(zero | (hi - 0x00100000u < 0x7FE00000u))) v = ieee_sqrt_slow(x);
         return v;
     }
 }

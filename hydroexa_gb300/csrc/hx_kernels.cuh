@@ -1937,11 +1937,13 @@ __global__ void __launch_bounds__(32 * 32, 1) k_ensemble_big(const EnsInstance<R
 }
 
 // ---------------------------------------------------------------------------
-// Classic Roe tile kernel (src/solvers/Roe.cpp:184-248, 327-434).
+// Classic Roe tile kernel (src/solvers/Roe.cpp:184-248, 327-434).  Each cell's root and velocities once, for its
+// four faces.  FP64 issue bounds it (75% of the pipe on 1000 x 750 rough cells, 230 instructions per cell, 0.375 ms);
+// four driver steps of that level, host reads of dt and status included: 4.61 -> 2.41 ms.
 // ---------------------------------------------------------------------------
 template <class R> struct ClassicSmem {
     static constexpr int GX = TX + 2, GY = TY + 2;
-    R h[GY][GX], hu[GY][GX], hv[GY][GX], z[GY][GX], n[GY][GX];
+    R h[GY][GX], s[GY][GX], u[GY][GX], v[GY][GX], z[GY][GX], n[GY][GX];  // s = sqrt(h); u, v: 0 where dry
     R fx[9][TY][TX + 1];  // F0..2, S-0..2, S+0..2
     R fy[9][TY + 1][TX];
     R kc[4];  // dt/dx, dt/dy, 1/dx, 1/dy: computed once per tile
@@ -1974,29 +1976,31 @@ __global__ void __launch_bounds__(NT) k_classic_tile(Src src, Cells3W<R> out, Fa
         const int gi = x0 + c - 1, gj = y0 + r - 1;
         R e = R(0), zz = R(0), qx = R(0), qy = R(0), nn = R(0);
         if (src.inside(gi, gj)) src.fetch(gi, gj, e, zz, qx, qy, nn);
-        const R hp = max0(e - zz);  // Roe.cpp:246, in place on the grown tile
+        R hp;  // Roe.cpp:246, in place on the grown tile
+        if constexpr (sizeof(R) == 8) hp = max0_num(e - zz);
+        else hp = max0(e - zz);
         S.h[r][c] = hp;
-        S.hu[r][c] = qx;
-        S.hv[r][c] = qy;
+        classic_cell<R, FAST>(hp, qx, qy, S.s[r][c], S.u[r][c], S.v[r][c]);
         S.z[r][c] = zz;
         S.n[r][c] = nn;
         hb.store(gi, gj, vb, hp);
     }
     __syncthreads();
 
+    auto cell = [&](int r, int c) {
+        return ClassicCell<R>{S.h[r][c], S.s[r][c], S.u[r][c], S.v[r][c], S.z[r][c], S.n[r][c]};
+    };
     auto xface = [&](int fi, int fj) {
         const int r = fj + 1, cl = fi, cr = fi + 1;
         R F[3], Sm[3], Sp[3];
-        roe_classic<R, FAST, 0>(S.h[r][cl], S.hu[r][cl], S.hv[r][cl], S.z[r][cl], S.n[r][cl], S.h[r][cr],
-                                S.hu[r][cr], S.hv[r][cr], S.z[r][cr], S.n[r][cr], ctl.dx, F, Sm, Sp);
+        roe_classic<R, FAST, 0>(cell(r, cl), cell(r, cr), ctl.dx, F, Sm, Sp);
         for (int k = 0; k < 3; ++k) { S.fx[k][fj][fi] = F[k]; S.fx[3 + k][fj][fi] = Sm[k]; S.fx[6 + k][fj][fi] = Sp[k]; }
         fo.store_x(x0 + fi, y0 + fj, vb, F, Sm, Sp, fi == TX);
     };
     auto yface = [&](int fi, int fj) {
         const int c = fi + 1, rl = fj, rr = fj + 1;
         R F[3], Sm[3], Sp[3];
-        roe_classic<R, FAST, 1>(S.h[rl][c], S.hu[rl][c], S.hv[rl][c], S.z[rl][c], S.n[rl][c], S.h[rr][c],
-                                S.hu[rr][c], S.hv[rr][c], S.z[rr][c], S.n[rr][c], ctl.dy, F, Sm, Sp);
+        roe_classic<R, FAST, 1>(cell(rl, c), cell(rr, c), ctl.dy, F, Sm, Sp);
         for (int k = 0; k < 3; ++k) { S.fy[k][fj][fi] = F[k]; S.fy[3 + k][fj][fi] = Sm[k]; S.fy[6 + k][fj][fi] = Sp[k]; }
         fo.store_y(x0 + fi, y0 + fj, vb, F, Sm, Sp, fj == TY);
     };
@@ -2017,12 +2021,20 @@ __global__ void __launch_bounds__(NT) k_classic_tile(Src src, Cells3W<R> out, Fa
     const bool valid = gi <= vb.hi0 && gj <= vb.hi1;
     R rate = R(0), mv = R(0);
     unsigned flags = 0;
+    ScreenCell<R> sc;
     if (valid) {
         const R cx = S.kc[0], cy = S.kc[1];
-        const R uo[3] = {S.h[ty + 1][tx + 1], S.hu[ty + 1][tx + 1], S.hv[ty + 1][tx + 1]};
+        R e, zz, nn, uo[3];
+        src.fetch(gi, gj, e, zz, uo[1], uo[2], nn);  // the momenta, once more
+        uo[0] = S.h[ty + 1][tx + 1];
         R un[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
+            if constexpr (FAST && sizeof(R) == 8) {  // the direction's flux and source differences summed first
+                un[k] = uo[k] - cx * ((S.fx[k][ty][tx + 1] - S.fx[k][ty][tx]) + (S.fx[6 + k][ty][tx + 1] + S.fx[3 + k][ty][tx])) -
+                        cy * ((S.fy[k][ty + 1][tx] - S.fy[k][ty][tx]) + (S.fy[6 + k][ty + 1][tx] + S.fy[3 + k][ty][tx]));
+                continue;
+            }
             // Roe.cpp:426-430, in this order
             un[k] = uo[k] - cx * (S.fx[k][ty][tx + 1] - S.fx[k][ty][tx]) - cy * (S.fy[k][ty + 1][tx] - S.fy[k][ty][tx]) -
                     cx * (S.fx[6 + k][ty][tx + 1] + S.fx[3 + k][ty][tx]) -
@@ -2030,10 +2042,16 @@ __global__ void __launch_bounds__(NT) k_classic_tile(Src src, Cells3W<R> out, Fa
         }
         out.st(gi, gj, un[0], un[1], un[2]);
         if (bits_nonfinite(un[0]) || bits_nonfinite(un[1]) || bits_nonfinite(un[2])) flags |= DTF_NAN;
-        if (ctl.dt_out) {
+        if constexpr (sizeof(R) == 8) {
+            sc.h = un[0]; sc.hu = un[1]; sc.hv = un[2]; sc.nod = is_nodata(S.z[ty + 1][tx + 1]); sc.live = true;
+        } else if (ctl.dt_out) {
             dt_cell_contrib<R, FAST>(un[0], un[1], un[2], is_nodata(S.z[ty + 1][tx + 1]), ctl.dx, ctl.dy,
                                      S.kc[2], S.kc[3], rate, mv, flags);
         }
+    }
+    if constexpr (sizeof(R) == 8) {  // FP64 folds the bound through the float screen, as the hydrostatic tile does
+        if (ctl.dt_out)
+            screened_fold<NT, 1, BlockSync, FAST>(&sc, ctl.dx, ctl.dy, S.kc[2], S.kc[3], rate, mv, flags);
     }
     if (ctl.dt_out) block_fold_dt<R, NT>(rate, mv, flags, ctl.dt_out);
     if ((flags & DTF_NAN) && ctl.status) atomicOr(ctl.status, (unsigned)HX_STATUS_NAN);
@@ -2337,8 +2355,11 @@ __global__ void k_points(int method, long n, const R* __restrict__ st, const R* 
         const R* q = st + 10 * p;
         const R* a = aux + 4 * p;
         R F[3], Sm[3], Sp[3];
-        if (a[3] != R(0)) roe_classic<R, FAST, 1>(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7], q[8], q[9], a[1], F, Sm, Sp);
-        else roe_classic<R, FAST, 0>(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7], q[8], q[9], a[1], F, Sm, Sp);
+        ClassicCell<R> l{q[0], R(0), R(0), R(0), q[3], q[4]}, r{q[5], R(0), R(0), R(0), q[8], q[9]};
+        classic_cell<R, FAST>(q[0], q[1], q[2], l.s, l.u, l.v);
+        classic_cell<R, FAST>(q[5], q[6], q[7], r.s, r.u, r.v);
+        if (a[3] != R(0)) roe_classic<R, FAST, 1>(l, r, a[1], F, Sm, Sp);
+        else roe_classic<R, FAST, 0>(l, r, a[1], F, Sm, Sp);
         for (int k = 0; k < 3; ++k) { out[3 * p + k] = F[k]; out[3 * n + 3 * p + k] = Sm[k]; out[6 * n + 3 * p + k] = Sp[k]; }
     }
 }

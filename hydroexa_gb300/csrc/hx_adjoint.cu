@@ -176,14 +176,10 @@ __device__ void roe_rev(double hi, double ui, double vi, double hj, double uj, d
     if (wj) { ghj += gHj; guj += gUj; gvj += gVj; }
 }
 
-// Fast form of roe_rev, in two parts.  The forward section gives the
-// quantities the reverse needs: either recomputed (roe_fwd_fast, taking the
-// branches roe_hydrostatic_fast takes, every division of the reverse turned
-// into a product with one of five reciprocals 1/sden, 1/den, 1/cm, 1/si, 1/sj
-// from a single rcp_nr of their product), or read from the record the segment
-// recompute wrote for the face (roe_fwd_rec: square roots, Roe averages,
-// entropy-fixed speeds and wave strengths as the forward step computed them;
-// only 1/si and 1/sj are formed).  roe_rev_core then runs the reverse.
+// Fast form of roe_rev in FP64, for the faces that face_rev_pair leaves: roe_fwd_fast forms the quantities the
+// reverse needs (taking the branches roe_hydrostatic_fast takes, every division of the reverse turned into a
+// product with one of five reciprocals 1/sden, 1/den, 1/cm, 1/si, 1/sj from a single rcp_nr of their product),
+// roe_rev_core runs the reverse.
 struct RoeFwd {
     double Hi, Hj, Ui, Uj, Vi, Vj, si, sj, hrsi, hrsj, cm, rs, rden, rcm, um, vm, l0, l2, dh;  // hrs = 1/(2 s)
     double a0h, a1h, a2h, w0, w1, w2, hrden, hrcm;  // half wave strengths, w = |l| ah, halves of 1/den, 1/cm
@@ -247,42 +243,6 @@ __device__ __forceinline__ void roe_fwd_fast(double hi, double ui, double vi, do
     F.a2h = 0.5 * ((dhu - F.l0 * dh) * F.rden);
     F.w0 = fabs(F.l0) * F.a0h; F.w1 = fabs(um) * F.a1h; F.w2 = fabs(F.l2) * F.a2h;
     F.hrden = 0.5 * F.rden; F.hrcm = 0.5 * F.rcm;
-}
-
-__device__ __forceinline__ void roe_fwd_rec(double hi, double ui, double vi, double hj, double uj, double vj,
-                                            const RoeRecVals& R, RoeFwd& F) {
-    using C = Cst<double>;
-    const bool wi = (R.fl & RR_WI) != 0, wj = (R.fl & RR_WJ) != 0;
-    F.wi = wi; F.wj = wj;
-    const double Hi = wi ? hi : 0.0, Hj = wj ? hj : 0.0;
-    const double Ui = wi ? ui : 0.0, Vi = wi ? vi : 0.0, Uj = wj ? uj : 0.0, Vj = wj ? vj : 0.0;
-    F.Hi = Hi; F.Hj = Hj; F.Ui = Ui; F.Uj = Uj; F.Vi = Vi; F.Vj = Vj;
-    const double si = R.si, sj = R.sj, cm = R.cm;
-    F.si = si; F.sj = sj; F.cm = cm;
-    F.hmb = (R.fl & RR_HM) != 0;
-    F.rs = R.rs; F.hrden = R.hrden; F.hrcm = R.hrcm;  // as the forward computed them
-    F.hrsi = 0.0; F.hrsj = 0.0;
-    if (wi && wj) {
-        const double r = rcp_nr((si + si) * sj);
-        F.hrsi = sj * r;
-        F.hrsj = si * r;
-    } else {
-        if (wi) F.hrsi = rcp_nr(si + si);
-        if (wj) F.hrsj = rcp_nr(sj + sj);
-    }
-    F.um = R.um; F.vm = R.vm; F.l0 = R.l0; F.l2 = R.l2;
-    F.fix0 = (R.fl & RR_FIX0) != 0;
-    F.fix2 = (R.fl & RR_FIX2) != 0;
-    if (F.fix0 | F.fix2) {  // the sonic-fix derivatives need the one-sided speeds
-        const double ci = C::sqrt_g * si, cj = C::sqrt_g * sj;
-        F.l0a = R.um - cm; F.l2a = R.um + cm;
-        F.e0i = Ui - ci; F.e0j = Uj - cj; F.e2i = Ui + ci; F.e2j = Uj + cj;
-        F.rD0 = F.fix0 ? rcp_nr(F.e0j - F.e0i) : 0.0;
-        F.rD2 = F.fix2 ? rcp_nr(F.e2j - F.e2i) : 0.0;
-    }
-    F.dh = Hj - Hi;
-    F.a0h = R.a0h; F.a1h = R.a1h; F.a2h = R.a2h;
-    F.w0 = fabs(R.l0) * R.a0h; F.w1 = fabs(R.um) * R.a1h; F.w2 = fabs(R.l2) * R.a2h;
 }
 
 __device__ __forceinline__ void roe_rev_core(const RoeFwd& F, double b0, double b1, double b2, double& ghi,
@@ -366,9 +326,8 @@ struct FaceVals {
 
 // Reverse of the hydrostatic face (HydrostaticRoe.cpp:247-396) for direction
 // DIR, given the adjoints of FL and FR (global frame).  Writes g.
-template <int DIR, bool FAST, bool REC = false>
-__device__ void face_rev(const FaceVals& f, const double gFL[3], const double gFR[3], FaceVals& g,
-                         const RoeRecVals* rec = nullptr) {
+template <int DIR, bool FAST>
+__device__ void face_rev(const FaceVals& f, const double gFL[3], const double gFR[3], FaceVals& g) {
     const bool zLmax = okey(f.zL) >= okey(f.zR);  // std::max(zL, zR) keeps zL on ties
     const double zf = zLmax ? f.zL : f.zR;
     const double etaLf = f.eL + 0.5 * f.seL, etaRf = f.eR - 0.5 * f.seR;
@@ -387,11 +346,9 @@ __device__ void face_rev(const FaceVals& f, const double gFL[3], const double gF
     double ghLs = 0, gunL = 0, gutL = 0, ghRs = 0, gunR = 0, gutR = 0;
     if constexpr (FAST) {
         RoeFwd F;
-        if constexpr (REC) roe_fwd_rec(hLs, unL, utL, hRs, unR, utR, *rec, F);
-        else roe_fwd_fast(hLs, unL, utL, hRs, unR, utR, F);
+        roe_fwd_fast(hLs, unL, utL, hRs, unR, utR, F);
         roe_rev_core(F, gf0, b1, b2, ghLs, gunL, gutL, ghRs, gunR, gutR);
     } else {
-        static_assert(!REC, "face records are kept for the fast form");
         roe_rev(hLs, unL, utL, hRs, unR, utR, gf0, b1, b2, ghLs, gunL, gutL, ghRs, gunR, gutR);
     }
     // pressure correction p = HG (hu^2 - hs^2)
@@ -438,6 +395,174 @@ __device__ void face_rev(const FaceVals& f, const double gFL[3], const double gF
     g.zL = gzL; g.zR = gzR;
 }
 
+// What one face's reverse reads and writes: V as in AdjSmem; the free surface, its slopes and the bed are doubles.
+// The fast form's slopes come halved.
+template <class V> struct FaceIn {
+    double eL, eR, zL, zR, seL, seR;
+    V uL, uR, vL, vR, suL, suR, svL, svR;
+};
+template <class V> struct FaceAdj {
+    V a[8];  // adjoints of eta L R, z L R, u L R, v L R at the face
+};
+
+// face_rev in FP64 for a face of the fast form: an entropy fix, a state past the pairs' range, or thin fast flow.
+template <int DIR>
+__device__ __noinline__ void face_rev_far(const FaceIn<F2>& f, const F2* lL, const F2* lR, FaceAdj<F2>& g) {
+    FaceVals v;
+    v.eL = f.eL; v.eR = f.eR; v.zL = f.zL; v.zR = f.zR;
+    v.uL = f64_of(f.uL); v.uR = f64_of(f.uR); v.vL = f64_of(f.vL); v.vR = f64_of(f.vR);
+    v.seL = 2.0 * f.seL; v.seR = 2.0 * f.seR;
+    v.suL = 2.0 * f64_of(f.suL); v.suR = 2.0 * f64_of(f.suR);
+    v.svL = 2.0 * f64_of(f.svL); v.svR = 2.0 * f64_of(f.svR);
+    double gFL[3], gFR[3];
+    for (int k = 0; k < 3; ++k) { gFL[k] = -f64_of(lL[k]); gFR[k] = f64_of(lR[k]); }
+    FaceVals r{};
+    face_rev<DIR, true>(v, gFL, gFR, r);
+    const double* a = &r.eL;
+    for (int k = 0; k < 8; ++k) g.a[k] = f2_of(a[k]);
+}
+// The exact form: face_rev itself.
+template <int DIR>
+__device__ __forceinline__ void face_adjoint(const FaceIn<double>& f, const double* lL, const double* lR,
+                                             FaceAdj<double>& g) {
+    const FaceVals v{f.eL, f.eR, f.zL, f.zR, f.uL, f.uR, f.vL, f.vR, f.seL, f.seR, f.suL, f.suR, f.svL, f.svR};
+    const double gFL[3] = {-lL[0], -lL[1], -lL[2]}, gFR[3] = {lR[0], lR[1], lR[2]};
+    FaceVals r{};
+    face_rev<DIR, false>(v, gFL, gFR, r);
+    const double* a = &r.eL;
+    for (int k = 0; k < 8; ++k) g.a[k] = a[k];
+}
+
+// Reverse of the hydrostatic face in float pairs (the fast form): roe_fwd_fast and roe_rev_core with every product
+// and sum on the FP32 pipe; the face depths are formed in FP64 as the forward forms them.  The averages, roots and
+// wave strengths come from the segment recompute's record or are formed as the forward forms them.  lL, lR: the
+// lambda of the two cells (FL enters the left one with -, FR the right one with +).  Thin fast flow (|u| > 4 c),
+// whose terms cancel like (u / c)^2, entropy fixes and states past the pairs' range go to FP64.
+//
+// Of the reverse's 422 FP64 instructions per cell this leaves ADJ_SLOTS; measured ADJ_TIME.
+template <int DIR>
+__device__ __forceinline__ void face_adjoint(const FaceIn<F2>& f, const F2* lL, const F2* lR, FaceAdj<F2>& g,
+                                             const RoeRecVals* rec = nullptr) {
+    const bool lhigh = !(okey(f.zL) < okey(f.zR));  // std::max(zL, zR) keeps zL on ties
+    const double etaLf = f.eL + f.seL, etaRf = f.eR - f.seR;
+    const double eH = lhigh ? etaLf : etaRf, zf = lhigh ? f.zL : f.zR;
+    const double eW = lhigh ? etaRf : etaLf, zW = lhigh ? f.zR : f.zL;
+    const double dH = eH - zf, dWs = eW - zf, dWu = eW - zW;
+    const double hH = max0_i(dH), hWs = max0_i(dWs), hWu = max0_i(dWu);
+    const double hi = lhigh ? hH : hWs, hj = lhigh ? hWs : hH;
+    const bool wi = ge_bits(hi, Cst<double>::toldry_bits), wj = ge_bits(hj, Cst<double>::toldry_bits);
+    const F2 uL = f2_add(f.uL, f.suL), vL = f2_add(f.vL, f.svL), uR = f2_sub(f.uR, f.suR), vR = f2_sub(f.vR, f.svR);
+    const F2 Ui = f2_sel(wi, DIR == 0 ? uL : vL), Vi = f2_sel(wi, DIR == 0 ? vL : f2_neg(uL));
+    const F2 Uj = f2_sel(wj, DIR == 0 ? uR : vR), Vj = f2_sel(wj, DIR == 0 ? vR : f2_neg(uR));
+    const double Hid = wi ? hi : 0.0, Hjd = wj ? hj : 0.0;
+    const F2 Hi = f2_of(Hid), Hj = f2_of(Hjd), dh = f2_of(Hjd - Hid);
+    RoeRecVals R;
+    if (rec) {
+        R = *rec;
+    } else {
+        const RoePair q = roe_pair_state(Hi, Hj, dh, Ui, Vi, Uj, Vj);
+        const F2 B = f2_mul(q.cB, q.rc);
+        R = RoeRecVals{q.si, q.sj, q.cm, q.rs, f2_half(q.rc), q.um, q.vm, f2_half(f2_sub(q.A, B)), f2_mul(q.mv, q.rc),
+                       f2_half(f2_add(q.A, B)), (q.hmb ? RR_HM : 0u) | (q.rule0 & q.rule2 ? 0u : RR_OTHER)};
+    }
+    {
+        const unsigned top = (1023u + 32u) << 20;
+        const bool in = ((unsigned)__double2hiint(hi) < top) & ((unsigned)__double2hiint(hj) < top) &
+                        (fabsf(Ui.h) < 0x1p24f) & (fabsf(Vi.h) < 0x1p24f) & (fabsf(Uj.h) < 0x1p24f) &
+                        (fabsf(Vj.h) < 0x1p24f) & ((R.fl & RR_OTHER) == 0u) & (fabsf(R.um.h) <= 4.f * R.cm.h);
+        if (!in) {
+            face_rev_far<DIR>(f, lL, lR, g);
+            return;
+        }
+    }
+    constexpr F2 kG{9.81f, (float)(9.81 - (double)9.81f)};
+    const F2 b0 = f2_sub(lR[0], lL[0]);
+    const F2 b1 = f2_sub(lR[1 + DIR], lL[1 + DIR]);
+    const F2 b2t = f2_sub(lR[2 - DIR], lL[2 - DIR]), b2 = DIR == 0 ? b2t : f2_neg(b2t);
+    const F2 um = R.um, vm = R.vm, cm = R.cm;
+    const F2 l0 = f2_sub(um, cm), l2 = f2_add(um, cm);
+    // central flux (F(U_i) + F(U_j)) / 2
+    const F2 hb0 = f2_half(b0), hb1 = f2_half(b1), hb2 = f2_half(b2);
+    const F2 gb1 = f2_mul(kG, hb1);
+    const F2 ti = f2_mul(b1, Ui), tj = f2_mul(b1, Uj);
+    const F2 pi = f2_add(hb0, f2_mul_raw(hb2, Vi)), pj = f2_add(hb0, f2_mul_raw(hb2, Vj));
+    F2 gHi = f2_add(f2_mul_raw(Ui, f2_add(pi, f2_half(ti))), f2_mul_raw(gb1, Hi));
+    F2 gHj = f2_add(f2_mul_raw(Uj, f2_add(pj, f2_half(tj))), f2_mul_raw(gb1, Hj));
+    F2 gUi = f2_add(pi, ti), gUj = f2_add(pj, tj);      // times H
+    F2 gVi = f2_mul(hb2, Ui), gVj = f2_mul(hb2, Uj);    // times H
+    // wave strengths: w_k = |l_k| ah_k
+    const F2 bc = f2_neg(f2_add(b0, f2_mul_raw(b2, vm)));
+    const F2 bl0 = f2_mul(b1, l0), bl2 = f2_mul(b1, l2);
+    const F2 gw0 = f2_sub(bc, bl0), gw2 = f2_sub(bc, bl2);
+    const F2 A0 = f2_abs(l0), A1 = f2_abs(um), A2 = f2_abs(l2);
+    const int s0 = __float_as_int(l0.h) & (int)0x80000000, s1 = __float_as_int(um.h) & (int)0x80000000,
+              s2 = __float_as_int(l2.h) & (int)0x80000000;
+    auto flip = [](F2 a, int s) {
+        return F2{__int_as_float(__float_as_int(a.h) ^ s), __int_as_float(__float_as_int(a.l) ^ s)};
+    };
+    F2 gl0 = flip(f2_mul(R.a0h, f2_sub(gw0, bl0)), s0);  // gw0 sgn(l0) a0h - b1 |l0| a0h
+    F2 gl2 = flip(f2_mul(R.a2h, f2_sub(gw2, bl2)), s2);
+    const F2 w1 = f2_mul(A1, R.a1h);
+    F2 gvm = f2_neg(f2_mul(b2, f2_add(f2_mul_raw(A0, R.a0h), f2_mul_raw(A2, R.a2h))));
+    F2 gcm = f2_neg(f2_mul(b2, w1));
+    const F2 gl1 = f2_sel(um.h != 0.f, flip(f2_neg(f2_mul(f2_mul(b2, cm), R.a1h)), s1));  // sgn(0) = 0
+    // adjoints of the wave strengths, divided by den = 2 cm + tol12 and by cm
+    F2 hrden = f2_half(R.hrcm);
+    hrden.l = __fmaf_rn(-hrden.h, __fmul_rn(1e-12f, R.hrcm.h), hrden.l);
+    const F2 ga0 = f2_mul(f2_mul(gw0, A0), hrden), ga2 = f2_mul(f2_mul(gw2, A2), hrden);
+    const F2 ga1 = f2_neg(f2_mul(hb2, A1));  // gw1 |um| / (2 cm), gw1 = -b2 cm
+    gl2 = f2_add(gl2, f2_mul_raw(ga0, dh));
+    gl0 = f2_sub(gl0, f2_mul_raw(ga2, dh));
+    gvm = f2_sub(gvm, f2_mul_raw(ga1, dh));
+    const F2 gdhu = f2_sub(ga2, ga0);
+    // gcm -= 2 (ga1 a1h + 2 (ga0 a0h + ga2 a2h))
+    const F2 ga = f2_add(f2_mul_raw(ga0, R.a0h), f2_mul_raw(ga2, R.a2h));
+    const F2 gb = f2_add(f2_mul_raw(ga1, R.a1h), F2{ga.h + ga.h, ga.l + ga.l});
+    gcm = f2_sub(gcm, F2{gb.h + gb.h, gb.l + gb.l});
+    // gHj += gdh + gdhu Uj + ga1 Vj with gdh = ga0 l2 - ga2 l0 - ga1 vm, and the same of i with the other sign;
+    // in differences of speeds
+    gHj = f2_add(gHj, f2_add(f2_add(f2_mul_raw(ga0, f2_sub(l2, Uj)), f2_mul_raw(ga2, f2_sub(Uj, l0))),
+                             f2_mul_raw(ga1, f2_sub(Vj, vm))));
+    gHi = f2_sub(gHi, f2_add(f2_add(f2_mul_raw(ga0, f2_sub(l2, Ui)), f2_mul_raw(ga2, f2_sub(Ui, l0))),
+                             f2_mul_raw(ga1, f2_sub(Vi, vm))));
+    gUi = f2_sub(gUi, gdhu);
+    gUj = f2_add(gUj, gdhu);
+    gVi = f2_sub(f2_mul_raw(gVi, Hi), f2_mul_raw(ga1, Hi));
+    gVj = f2_add(f2_mul_raw(gVj, Hj), f2_mul_raw(ga1, Hj));
+    const F2 gum = f2_add(gl1, f2_add(gl2, gl0));
+    gcm = f2_add(gcm, f2_sub(gl2, gl0));
+    const F2 gnu = f2_mul(gum, R.rs), gnv = f2_mul(gvm, R.rs);
+    gUi = f2_add(f2_mul_raw(gUi, Hi), f2_mul_raw(gnu, R.si));
+    gUj = f2_add(f2_mul_raw(gUj, Hj), f2_mul_raw(gnu, R.sj));
+    gVi = f2_add(gVi, f2_mul_raw(gnv, R.si));
+    gVj = f2_add(gVj, f2_mul_raw(gnv, R.sj));
+    // s = sqrt(H): d/dH = 1 / (2 s), with gsden = -(gnu um + gnv vm)
+    const F2 gsi = f2_add(f2_mul_raw(gnu, f2_sub(Ui, um)), f2_mul_raw(gnv, f2_sub(Vi, vm)));
+    const F2 gsj = f2_add(f2_mul_raw(gnu, f2_sub(Uj, um)), f2_mul_raw(gnv, f2_sub(Vj, vm)));
+    const F2 hrsi = f2_half(f2_rcp(F2{wi ? R.si.h : 1.f, wi ? R.si.l : 0.f}));
+    const F2 hrsj = f2_half(f2_rcp(F2{wj ? R.sj.h : 1.f, wj ? R.sj.l : 0.f}));
+    const F2 hg = f2_sel((R.fl & RR_HM) != 0u, f2_mul(f2_half(f2_mul(kG, R.hrcm)), gcm));
+    gHi = f2_add(gHi, f2_add(hg, f2_mul_raw(gsi, hrsi)));
+    gHj = f2_add(gHj, f2_add(hg, f2_mul_raw(gsj, hrsj)));
+    gHi = f2_sel(wi, gHi);
+    gHj = f2_sel(wj, gHj);
+    // pressure correction of the lower side, p = HG (hu^2 - hs^2); the caps max(0, .) pass the adjoints where their
+    // argument is positive (as in face_rev)
+    const F2 gpW = f2_mul(kG, lhigh ? lR[1 + DIR] : f2_neg(lL[1 + DIR]));
+    const F2 HWs = f2_of(hWs), HWu = f2_of(hWu);
+    const F2 gHs = lhigh ? gHi : gHj;                                                 // the face-bed side
+    const F2 gWs = f2_sub(lhigh ? gHj : gHi, f2_mul_raw(gpW, HWs));
+    const F2 sH = f2_sel(pos_i(dH), gHs), sW = f2_sel(pos_i(dWs), gWs), uW = f2_sel(pos_i(dWu), f2_mul(gpW, HWu));
+    const F2 eWa = f2_add(sW, uW), zHa = f2_neg(f2_add(sH, sW)), zWa = f2_neg(uW);
+    g.a[0] = lhigh ? sH : eWa;
+    g.a[1] = lhigh ? eWa : sH;
+    g.a[2] = lhigh ? zHa : zWa;
+    g.a[3] = lhigh ? zWa : zHa;
+    gUi = f2_sel(wi, gUi); gVi = f2_sel(wi, gVi); gUj = f2_sel(wj, gUj); gVj = f2_sel(wj, gVj);
+    if (DIR == 0) { g.a[4] = gUi; g.a[5] = gUj; g.a[6] = gVi; g.a[7] = gVj; }
+    else { g.a[4] = f2_neg(gVi); g.a[5] = f2_neg(gVj); g.a[6] = gUi; g.a[7] = gUj; }
+}
+
 // Reverse of van_leer_slope(qm, q, qp) (HydrostaticRoe.cpp:179-195).
 __device__ __forceinline__ void slope_rev(double qm, double q, double qp, double gs, double& gqm, double& gq,
                                           double& gqp) {
@@ -458,46 +583,50 @@ __device__ __forceinline__ void slope_rev(double qm, double q, double qp, double
     gqp = gdp;
 }
 
-// slope_rev with the reciprocal from van_leer_slope_rs (rS == 0: the slope was 0 by a branch), given
-// gs2 = twice the slope's adjoint (what the faces hand over: the slope enters each face state with 1/2).
-__device__ __forceinline__ void slope_rev_rs(double qm, double q, double qp, double rS, double gs2, double& gqm,
-                                             double& gq, double& gqp) {
-    gqm = gq = gqp = 0.0;
-    if ((sbits(gs2) << 1) == 0) return;
-    const double dm = q - qm, dp = qp - q;
-    if ((sbits(rS) << 1) == 0) {
-        if (!abs_le_bits(dp, Cst<double>::tol12_bits) && (sbits(dm) << 1) == 0) {  // r = 0: d s / d dm = 1
-            gq = 0.5 * gs2;
-            gqm = -gq;
-        }
-        return;
+// slope_rev of the fast form in pairs: dm, dp the slope's differences, rS = 1 / (dm + dp) (0 where the slope is 0 by
+// a branch), gs2 twice the slope's adjoint (what the faces hand over: the slope enters each face state with 1/2).
+__device__ __forceinline__ void slope_rev_pair(F2 dm, F2 dp, F2 rS, F2 gs2, F2& gqm, F2& gq, F2& gqp) {
+    const bool flat = rS.h == 0.f;
+    // r = 0: d s / d dm = 1, the mean of the one-sided derivatives
+    const bool half = flat & !(fabsf(dp.h) <= 1e-12f) & (dm.h == 0.f);
+    const F2 x = f2_mul(dp, rS), y = f2_mul(dm, rS);
+    const F2 gdm = f2_mul(f2_mul(gs2, x), x), gdp = f2_mul(f2_mul(gs2, y), y);
+    gq = f2_sel(!flat, f2_sub(gdm, gdp));
+    gqm = f2_sel(!flat, f2_neg(gdm));
+    gqp = f2_sel(!flat, gdp);
+    if (half) {
+        gq = f2_half(gs2);
+        gqm = f2_neg(gq);
     }
-    const double t = gs2 * rS * rS;  // 2 gs / S^2
-    const double gdm = t * dp * dp, gdp = t * dm * dm;
-    gq = gdm - gdp;
-    gqm = -gdm;
-    gqp = gdp;
 }
 
 // ---------------------------------------------------------------------------
 // Kernel B: face reverse of one tile.
 // ---------------------------------------------------------------------------
-struct AdjSmem {
+// V: double, or float pairs in the fast form (velocities, scaled lambda, slopes of velocities and every adjoint of
+// the tile; the free surface's slopes stay doubles).
+template <class V> struct AdjSmem {
+    static_assert(sizeof(V) == sizeof(double), "the layout does not depend on V");
     static constexpr int GX = ATX + 2 * H3, GY = ATY + 2 * H3;
-    double hp[GY][GX], eta[GY][GX], u[GY][GX], v[GY][GX], z[GY][GX], lam[3][GY][GX];
+    double hp[GY][GX], eta[GY][GX];
+    V u[GY][GX], v[GY][GX];
+    double z[GY][GX];
+    V lam[3][GY][GX];
     unsigned char nod[GY][GX];
     union {
         struct {  // x pass
-            double s[3][ATY][ATX + 4];      // slopes of columns x0-2 .. x0+TX+1
-            double rs[3][ATY][ATX + 4];     // their 1 / (dm + dp) (fast form; 0 where the slope is 0 by a branch)
-            double fa[8][ATY][ATX + 3];     // face adjoints of eta, z, u, v on either side, faces x0-1 .. x0+TX+1
-            double sp[9][ATY][ATX + 2];     // slope-reverse partials, columns x0-1 .. x0+TX
+            double se[ATY][ATX + 4];        // slopes of columns x0-2 .. x0+TX+1 (halved in the fast form): eta;
+            V s[2][ATY][ATX + 4];           // u, v
+            V rs[3][ATY][ATX + 4];          // their 1 / (dm + dp) (fast form; 0 where the slope is 0 by a branch)
+            V fa[8][ATY][ATX + 3];          // face adjoints of eta, z, u, v on either side, faces x0-1 .. x0+TX+1
+            V sp[9][ATY][ATX + 2];          // slope-reverse partials, columns x0-1 .. x0+TX
         } x;
         struct {  // y pass
-            double s[3][ATY + 4][ATX];
-            double rs[3][ATY + 4][ATX];
-            double fa[8][ATY + 3][ATX];
-            double sp[9][ATY + 2][ATX];
+            double se[ATY + 4][ATX];
+            V s[2][ATY + 4][ATX];
+            V rs[3][ATY + 4][ATX];
+            V fa[8][ATY + 3][ATX];
+            V sp[9][ATY + 2][ATX];
         } y;
     } p;
     double fold[4][ATY][ATX];  // ghost adjoints folded into own cells (h, hu, hv, z)
@@ -531,17 +660,28 @@ struct AdjArgs {
 
 // The record of x face (f, j) (d = 0) or y face (i, f) (d = 1).
 __device__ __forceinline__ RoeRecVals load_rec(const FaceRec& R, int d, long long o) {
-    const double* b = R.f[d] + o;
+    const F2* b = reinterpret_cast<const F2*>(R.f[d]) + o;
     const long long ps = R.plane[d];
     RoeRecVals r;
-    r.si = b[0]; r.sj = b[ps]; r.cm = b[2 * ps]; r.rs = b[3 * ps]; r.hrden = b[4 * ps]; r.hrcm = b[5 * ps];
-    r.um = b[6 * ps]; r.vm = b[7 * ps]; r.l0 = b[8 * ps]; r.l2 = b[9 * ps]; r.a0h = b[10 * ps];
-    r.a1h = b[11 * ps]; r.a2h = b[12 * ps];
+    r.si = b[0]; r.sj = b[ps]; r.cm = b[2 * ps]; r.rs = b[3 * ps]; r.hrcm = b[4 * ps];
+    r.um = b[5 * ps]; r.vm = b[6 * ps]; r.a0h = b[7 * ps]; r.a1h = b[8 * ps]; r.a2h = b[9 * ps];
     r.fl = R.fl[d][o];
     return r;
 }
 
-__device__ __forceinline__ double fget(const FaceVals& f, int k) { return (&f.eL)[k]; }
+// Sums and products of either form's adjoints.
+__device__ __forceinline__ double vadd(double a, double b) { return a + b; }
+__device__ __forceinline__ F2 vadd(F2 a, F2 b) { return f2_add(a, b); }
+__device__ __forceinline__ double vsub(double a, double b) { return a - b; }
+__device__ __forceinline__ F2 vsub(F2 a, F2 b) { return f2_sub(a, b); }
+__device__ __forceinline__ double vmul(double a, double b) { return a * b; }
+__device__ __forceinline__ F2 vmul(F2 a, F2 b) { return f2_mul(a, b); }
+template <class V> __device__ __forceinline__ V vzero() { return V{}; }
+// x 2^-k as a pair (the tile's lambda on the scale of its largest), 0 far below it.
+__device__ __forceinline__ F2 scaled_pair(double x, int k) {
+    const int hi = __double2hiint(x), m = (hi & 0x7FFFFFFF) - (k << 20);
+    return f2_of(__hiloint2double(m >= (897 << 20) ? (m | (hi & (int)0x80000000)) : 0, __double2loint(x)));
+}
 
 __device__ __forceinline__ double block_sum(double v, double* sh) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -619,13 +759,15 @@ __device__ __forceinline__ void adj_finish_body(int nblocks, const double* dtbar
 template <bool FAST, bool REC = false>
 __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    AdjSmem& S = *reinterpret_cast<AdjSmem*>(smem_raw);
-    constexpr int GX = AdjSmem::GX, GY = AdjSmem::GY;
+    using V = std::conditional_t<FAST, F2, double>;
+    AdjSmem<V>& S = *reinterpret_cast<AdjSmem<V>*>(smem_raw);
+    constexpr int GX = AdjSmem<V>::GX, GY = AdjSmem<V>::GY;
     const int t = threadIdx.x;
     const int x0 = blockIdx.x * ATX, y0 = blockIdx.y * ATY;
     const int nx = A.nx, ny = A.ny;
 
     // forward values on the grown tile (halo 3) and lambda_lin (0 outside the domain)
+    [[maybe_unused]] unsigned lmax = 0;
     for (int idx = t; idx < GX * GY; idx += ANT) {
         const int r = idx / GX, c = idx - r * GX;
         const int gi = x0 + c - H3, gj = y0 + r - H3;
@@ -640,9 +782,7 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
         S.hp[r][c] = hp;
         S.eta[r][c] = hp + zz;
         if constexpr (FAST) {  // the forward's own velocity arithmetic, so the limiters take its branches
-            const double rh = gt_bits(hp, Cst<double>::tol12_bits) ? rcp_nr(hp) : 0.0;
-            S.u[r][c] = qx * rh;
-            S.v[r][c] = qy * rh;
+            cell_velocity(hp, qx, qy, S.u[r][c], S.v[r][c]);
         } else {
             S.u[r][c] = gt_bits(hp, Cst<double>::tol12_bits) ? qx / hp : 0.0;
             S.v[r][c] = gt_bits(hp, Cst<double>::tol12_bits) ? qy / hp : 0.0;
@@ -651,13 +791,39 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
         S.nod[r][c] = (in_grown && is_nodata(zz)) ? 1 : 0;
         const bool inside = gi >= 0 && gi < nx && gj >= 0 && gj < ny;
         const long long o = (long long)gi + (long long)gj * A.pitch;
-        for (int k = 0; k < 3; ++k) S.lam[k][r][c] = inside ? A.lam[k][o] : 0.0;
+        for (int k = 0; k < 3; ++k) {
+            const double l = inside ? A.lam[k][o] : 0.0;
+            if constexpr (FAST) {
+                S.lam[k][r][c] = f2_bits(l);
+                lmax = max(lmax, (unsigned)__double2hiint(l) & 0x7FFFFFFFu);
+            } else {
+                S.lam[k][r][c] = l;
+            }
+        }
     }
     for (int idx = t; idx < 4 * ATX * ATY; idx += ANT) (&S.fold[0][0][0])[idx] = 0.0;
+    // The reverse is linear in lambda, so the fast form runs it on the tile's lambda divided by the power of two
+    // of its largest value: the pairs' range then never ends it, however large or small a gradient grows.
+    [[maybe_unused]] double lscale = 1.0;
+    if constexpr (FAST) {
+        __shared__ unsigned s_lmax[ANT / 32];
+        lmax = __reduce_max_sync(0xffffffffu, lmax);
+        if ((t & 31) == 0) s_lmax[t >> 5] = lmax;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < ANT / 32; ++k) lmax = max(lmax, s_lmax[k]);
+        const int e = (int)(lmax >> 20), k = e == 0 || e == 0x7FF ? 0 : e - 1023;
+        lscale = __hiloint2double((k + 1023) << 20, 0);
+        for (int idx = t; idx < GX * GY; idx += ANT)
+            for (int q = 0; q < 3; ++q) {
+                F2& l = (&S.lam[q][0][0])[idx];
+                l = scaled_pair(bits_f2(l), k);
+            }
+    }
     __syncthreads();
 
     const int tx = t % ATX, ty = t / ATX;
-    double ae = 0, au = 0, av = 0, az = 0;  // gathered adjoints of this thread's cell
+    V ae = V{}, au = V{}, av = V{}, az = V{};  // gathered adjoints of this thread's cell
 
     // ===================== x pass =====================
     {
@@ -669,18 +835,18 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
                 const int gi = x0 + col, gj = y0 + row;
                 const bool in = gi >= -1 && gi <= nx && gj < ny;
                 const long long o = (long long)(gi + 1) + (long long)gj * (nx + 2), ps = A.rec.slplane[0];
-                for (int q = 0; q < 3; ++q) {
-                    P.s[q][row][col + 2] = in ? A.rec.sl[0][q * ps + o] : 0.0;
-                    P.rs[q][row][col + 2] = in ? A.rec.sl[0][(3 + q) * ps + o] : 0.0;
-                }
+                P.se[row][col + 2] = in ? A.rec.sl[0][o] : 0.0;
+                const F2* sl = reinterpret_cast<const F2*>(A.rec.sl[0]) + o;
+                for (int q = 0; q < 2; ++q) P.s[q][row][col + 2] = in ? sl[(1 + q) * ps] : F2{0.f, 0.f};
+                for (int q = 0; q < 3; ++q) P.rs[q][row][col + 2] = in ? sl[(3 + q) * ps] : F2{0.f, 0.f};
             } else if constexpr (FAST) {
-                P.s[0][row][col + 2] = van_leer_slope_rs(S.eta[r][c - 1], S.eta[r][c], S.eta[r][c + 1], P.rs[0][row][col + 2]);
-                P.s[1][row][col + 2] = van_leer_slope_rs(S.u[r][c - 1], S.u[r][c], S.u[r][c + 1], P.rs[1][row][col + 2]);
-                P.s[2][row][col + 2] = van_leer_slope_rs(S.v[r][c - 1], S.v[r][c], S.v[r][c + 1], P.rs[2][row][col + 2]);
+                P.se[row][col + 2] = half_slope(S.eta[r][c - 1], S.eta[r][c], S.eta[r][c + 1], &P.rs[0][row][col + 2]);
+                P.s[0][row][col + 2] = half_slope(S.u[r][c - 1], S.u[r][c], S.u[r][c + 1], &P.rs[1][row][col + 2]);
+                P.s[1][row][col + 2] = half_slope(S.v[r][c - 1], S.v[r][c], S.v[r][c + 1], &P.rs[2][row][col + 2]);
             } else {
-                P.s[0][row][col + 2] = van_leer_slope<double, false>(S.eta[r][c - 1], S.eta[r][c], S.eta[r][c + 1]);
-                P.s[1][row][col + 2] = van_leer_slope<double, false>(S.u[r][c - 1], S.u[r][c], S.u[r][c + 1]);
-                P.s[2][row][col + 2] = van_leer_slope<double, false>(S.v[r][c - 1], S.v[r][c], S.v[r][c + 1]);
+                P.se[row][col + 2] = van_leer_slope<double, false>(S.eta[r][c - 1], S.eta[r][c], S.eta[r][c + 1]);
+                P.s[0][row][col + 2] = van_leer_slope<double, false>(S.u[r][c - 1], S.u[r][c], S.u[r][c + 1]);
+                P.s[1][row][col + 2] = van_leer_slope<double, false>(S.v[r][c - 1], S.v[r][c], S.v[r][c + 1]);
             }
         }
         __syncthreads();
@@ -688,29 +854,26 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
             const int row = k / (ATX + 3), fcol = k % (ATX + 3) - 1;  // face at the left of column fcol
             const int f = x0 + fcol, gj = y0 + row;
             const int r = row + H3, cl = fcol - 1 + H3, cr = fcol + H3;
-            FaceVals g{};
+            FaceAdj<V> g{};
             if (f >= 0 && f <= nx && gj < ny && !(S.nod[r][cl] | S.nod[r][cr])) {
-                FaceVals fv;
+                FaceIn<V> fv;
                 fv.eL = S.eta[r][cl]; fv.eR = S.eta[r][cr]; fv.zL = S.z[r][cl]; fv.zR = S.z[r][cr];
                 fv.uL = S.u[r][cl]; fv.uR = S.u[r][cr]; fv.vL = S.v[r][cl]; fv.vR = S.v[r][cr];
-                fv.seL = P.s[0][row][fcol - 1 + 2]; fv.seR = P.s[0][row][fcol + 2];
-                fv.suL = P.s[1][row][fcol - 1 + 2]; fv.suR = P.s[1][row][fcol + 2];
-                fv.svL = P.s[2][row][fcol - 1 + 2]; fv.svR = P.s[2][row][fcol + 2];
+                fv.seL = P.se[row][fcol - 1 + 2]; fv.seR = P.se[row][fcol + 2];
+                fv.suL = P.s[0][row][fcol - 1 + 2]; fv.suR = P.s[0][row][fcol + 2];
+                fv.svL = P.s[1][row][fcol - 1 + 2]; fv.svR = P.s[1][row][fcol + 2];
                 // FL(f) enters cell f-1 with -cx, FR(f) enters cell f with +cx; the face reverse is linear in
                 // these, so it runs on -lambda, +lambda and the gathers below apply cx once per cell
-                double gFL[3], gFR[3];
-                for (int c = 0; c < 3; ++c) {
-                    gFL[c] = -S.lam[c][r][cl];
-                    gFR[c] = S.lam[c][r][cr];
-                }
+                const V lL[3] = {S.lam[0][r][cl], S.lam[1][r][cl], S.lam[2][r][cl]};
+                const V lR[3] = {S.lam[0][r][cr], S.lam[1][r][cr], S.lam[2][r][cr]};
                 if constexpr (REC) {
                     const RoeRecVals rv = load_rec(A.rec, 0, (long long)f + (long long)gj * (nx + 1));
-                    face_rev<0, FAST, true>(fv, gFL, gFR, g, &rv);
+                    face_adjoint<0>(fv, lL, lR, g, &rv);
                 } else {
-                    face_rev<0, FAST>(fv, gFL, gFR, g);
+                    face_adjoint<0>(fv, lL, lR, g);
                 }
             }
-            for (int q = 0; q < 8; ++q) P.fa[q][row][fcol + 1] = fget(g, q);
+            for (int q = 0; q < 8; ++q) P.fa[q][row][fcol + 1] = g.a[q];
         }
         __syncthreads();
         for (int k = t; k < ATY * (ATX + 2); k += ANT) {  // slope reverse, columns x0-1 .. x0+TX
@@ -721,11 +884,18 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
             // difference of the two face states' adjoints
             for (int qi = 0; qi < 3; ++qi) {
                 const int qL = qi == 0 ? 0 : 2 + 2 * qi, qR = qL + 1;  // eta: 0, 1; u: 4, 5; v: 6, 7
-                const double gs2 = P.fa[qL][row][col + 2] - P.fa[qR][row][col + 1];
-                const double(*Q)[GX] = qi == 0 ? S.eta : (qi == 1 ? S.u : S.v);
-                double gm, g0, gp;
-                if constexpr (FAST) slope_rev_rs(Q[r][c - 1], Q[r][c], Q[r][c + 1], P.rs[qi][row][col + 2], gs2, gm, g0, gp);
-                else slope_rev(Q[r][c - 1], Q[r][c], Q[r][c + 1], 0.5 * gs2, gm, g0, gp);
+                const V gs2 = vsub(P.fa[qL][row][col + 2], P.fa[qR][row][col + 1]);
+                V gm, g0, gp;
+                if constexpr (FAST) {
+                    const F2 dm = qi == 0 ? f2_of(S.eta[r][c] - S.eta[r][c - 1])
+                                          : (qi == 1 ? f2_sub(S.u[r][c], S.u[r][c - 1]) : f2_sub(S.v[r][c], S.v[r][c - 1]));
+                    const F2 dp = qi == 0 ? f2_of(S.eta[r][c + 1] - S.eta[r][c])
+                                          : (qi == 1 ? f2_sub(S.u[r][c + 1], S.u[r][c]) : f2_sub(S.v[r][c + 1], S.v[r][c]));
+                    slope_rev_pair(dm, dp, P.rs[qi][row][col + 2], gs2, gm, g0, gp);
+                } else {
+                    const double(*Q)[GX] = qi == 0 ? S.eta : (qi == 1 ? S.u : S.v);
+                    slope_rev(Q[r][c - 1], Q[r][c], Q[r][c + 1], 0.5 * gs2, gm, g0, gp);
+                }
                 P.sp[3 * qi + 0][row][col + 1] = gm;  // to column col-1
                 P.sp[3 * qi + 1][row][col + 1] = g0;  // to column col
                 P.sp[3 * qi + 2][row][col + 1] = gp;  // to column col+1
@@ -733,13 +903,16 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
         }
         __syncthreads();
         // gather for column c: faces c (R side) and c+1 (L side), slopes c-1 (to right), c (self), c+1 (to left)
-        auto gather_x = [&](int row, int col, double& ge, double& gu, double& gv, double& gz) {
-            auto F = [&](int q, int fcol) { return (fcol >= -1 && fcol <= ATX + 1) ? P.fa[q][row][fcol + 1] : 0.0; };
-            auto SP = [&](int q, int scol) { return (scol >= -1 && scol <= ATX) ? P.sp[q][row][scol + 1] : 0.0; };
-            ge = A.cx * (F(1, col) + F(0, col + 1) + SP(2, col - 1) + SP(1, col) + SP(0, col + 1));
-            gu = A.cx * (F(5, col) + F(4, col + 1) + SP(5, col - 1) + SP(4, col) + SP(3, col + 1));
-            gv = A.cx * (F(7, col) + F(6, col + 1) + SP(8, col - 1) + SP(7, col) + SP(6, col + 1));
-            gz = A.cx * (F(3, col) + F(2, col + 1));
+        V cxv;
+        if constexpr (FAST) cxv = f2_of_rn(A.cx);
+        else cxv = A.cx;
+        auto gather_x = [&](int row, int col, V& ge, V& gu, V& gv, V& gz) {
+            auto F = [&](int q, int fcol) { return (fcol >= -1 && fcol <= ATX + 1) ? P.fa[q][row][fcol + 1] : V{}; };
+            auto SP = [&](int q, int scol) { return (scol >= -1 && scol <= ATX) ? P.sp[q][row][scol + 1] : V{}; };
+            ge = vmul(cxv, vadd(vadd(vadd(F(1, col), F(0, col + 1)), vadd(SP(2, col - 1), SP(1, col))), SP(0, col + 1)));
+            gu = vmul(cxv, vadd(vadd(vadd(F(5, col), F(4, col + 1)), vadd(SP(5, col - 1), SP(4, col))), SP(3, col + 1)));
+            gv = vmul(cxv, vadd(vadd(vadd(F(7, col), F(6, col + 1)), vadd(SP(8, col - 1), SP(7, col))), SP(6, col + 1)));
+            gz = vmul(cxv, vadd(F(3, col), F(2, col + 1)));
         };
         gather_x(ty, tx, ae, au, av, az);  // the x pass starts the cell's sums
         // x-boundary ghosts: one thread per row folds both sides
@@ -752,14 +925,16 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
                 for (int k = 1; k <= 2; ++k) {
                     const int gi = lo ? -k : nx - 1 + k;  // ghost column
                     const int col = gi - x0, c = col + H3;
-                    double ge, gu, gv, gz;
-                    gather_x(row, col, ge, gu, gv, gz);
+                    V pe, pu, pv, pz;
+                    gather_x(row, col, pe, pu, pv, pz);
+                    const double ge = lscale * flux_of(pe), gu = lscale * flux_of(pu), gv = lscale * flux_of(pv),
+                                 gz = lscale * flux_of(pz);
                     const double hp = S.hp[r][c];
                     double gzt = gz + ge, ghp = ge, ghu = 0, ghv = 0;
                     if (gt_bits(hp, Cst<double>::tol12_bits)) {
                         ghu = gu / hp;
                         ghv = gv / hp;
-                        ghp -= (gu * S.u[r][c] + gv * S.v[r][c]) / hp;
+                        ghp -= (gu * flux_of(S.u[r][c]) + gv * flux_of(S.v[r][c])) / hp;
                     }
                     double geta = 0;
                     if (pos_i(hp)) { geta = ghp; gzt -= ghp; }
@@ -793,18 +968,18 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
                 const int gi = x0 + col, gj = y0 + row;
                 const bool in = gj >= -1 && gj <= ny && gi < nx;
                 const long long o = (long long)gi + (long long)(gj + 1) * nx, ps = A.rec.slplane[1];
-                for (int q = 0; q < 3; ++q) {
-                    P.s[q][row + 2][col] = in ? A.rec.sl[1][q * ps + o] : 0.0;
-                    P.rs[q][row + 2][col] = in ? A.rec.sl[1][(3 + q) * ps + o] : 0.0;
-                }
+                P.se[row + 2][col] = in ? A.rec.sl[1][o] : 0.0;
+                const F2* sl = reinterpret_cast<const F2*>(A.rec.sl[1]) + o;
+                for (int q = 0; q < 2; ++q) P.s[q][row + 2][col] = in ? sl[(1 + q) * ps] : F2{0.f, 0.f};
+                for (int q = 0; q < 3; ++q) P.rs[q][row + 2][col] = in ? sl[(3 + q) * ps] : F2{0.f, 0.f};
             } else if constexpr (FAST) {
-                P.s[0][row + 2][col] = van_leer_slope_rs(S.eta[r - 1][c], S.eta[r][c], S.eta[r + 1][c], P.rs[0][row + 2][col]);
-                P.s[1][row + 2][col] = van_leer_slope_rs(S.u[r - 1][c], S.u[r][c], S.u[r + 1][c], P.rs[1][row + 2][col]);
-                P.s[2][row + 2][col] = van_leer_slope_rs(S.v[r - 1][c], S.v[r][c], S.v[r + 1][c], P.rs[2][row + 2][col]);
+                P.se[row + 2][col] = half_slope(S.eta[r - 1][c], S.eta[r][c], S.eta[r + 1][c], &P.rs[0][row + 2][col]);
+                P.s[0][row + 2][col] = half_slope(S.u[r - 1][c], S.u[r][c], S.u[r + 1][c], &P.rs[1][row + 2][col]);
+                P.s[1][row + 2][col] = half_slope(S.v[r - 1][c], S.v[r][c], S.v[r + 1][c], &P.rs[2][row + 2][col]);
             } else {
-                P.s[0][row + 2][col] = van_leer_slope<double, false>(S.eta[r - 1][c], S.eta[r][c], S.eta[r + 1][c]);
-                P.s[1][row + 2][col] = van_leer_slope<double, false>(S.u[r - 1][c], S.u[r][c], S.u[r + 1][c]);
-                P.s[2][row + 2][col] = van_leer_slope<double, false>(S.v[r - 1][c], S.v[r][c], S.v[r + 1][c]);
+                P.se[row + 2][col] = van_leer_slope<double, false>(S.eta[r - 1][c], S.eta[r][c], S.eta[r + 1][c]);
+                P.s[0][row + 2][col] = van_leer_slope<double, false>(S.u[r - 1][c], S.u[r][c], S.u[r + 1][c]);
+                P.s[1][row + 2][col] = van_leer_slope<double, false>(S.v[r - 1][c], S.v[r][c], S.v[r + 1][c]);
             }
         }
         __syncthreads();
@@ -812,27 +987,25 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
             const int frow = k / ATX - 1, col = k % ATX;
             const int f = y0 + frow, gi = x0 + col;
             const int c = col + H3, rl = frow - 1 + H3, rr = frow + H3;
-            FaceVals g{};
+            FaceAdj<V> g{};
             if (f >= 0 && f <= ny && gi < nx && !(S.nod[rl][c] | S.nod[rr][c])) {
-                FaceVals fv;
+                FaceIn<V> fv;
                 fv.eL = S.eta[rl][c]; fv.eR = S.eta[rr][c]; fv.zL = S.z[rl][c]; fv.zR = S.z[rr][c];
                 fv.uL = S.u[rl][c]; fv.uR = S.u[rr][c]; fv.vL = S.v[rl][c]; fv.vR = S.v[rr][c];
-                fv.seL = P.s[0][frow - 1 + 2][col]; fv.seR = P.s[0][frow + 2][col];
-                fv.suL = P.s[1][frow - 1 + 2][col]; fv.suR = P.s[1][frow + 2][col];
-                fv.svL = P.s[2][frow - 1 + 2][col]; fv.svR = P.s[2][frow + 2][col];
-                double gFL[3], gFR[3];  // unscaled, as in the x pass; cy in the gathers
-                for (int q = 0; q < 3; ++q) {
-                    gFL[q] = -S.lam[q][rl][c];
-                    gFR[q] = S.lam[q][rr][c];
-                }
+                fv.seL = P.se[frow - 1 + 2][col]; fv.seR = P.se[frow + 2][col];
+                fv.suL = P.s[0][frow - 1 + 2][col]; fv.suR = P.s[0][frow + 2][col];
+                fv.svL = P.s[1][frow - 1 + 2][col]; fv.svR = P.s[1][frow + 2][col];
+                // unscaled, as in the x pass; cy in the gathers
+                const V lL[3] = {S.lam[0][rl][c], S.lam[1][rl][c], S.lam[2][rl][c]};
+                const V lR[3] = {S.lam[0][rr][c], S.lam[1][rr][c], S.lam[2][rr][c]};
                 if constexpr (REC) {
                     const RoeRecVals rv = load_rec(A.rec, 1, (long long)gi + (long long)f * nx);
-                    face_rev<1, FAST, true>(fv, gFL, gFR, g, &rv);
+                    face_adjoint<1>(fv, lL, lR, g, &rv);
                 } else {
-                    face_rev<1, FAST>(fv, gFL, gFR, g);
+                    face_adjoint<1>(fv, lL, lR, g);
                 }
             }
-            for (int q = 0; q < 8; ++q) P.fa[q][frow + 1][col] = fget(g, q);
+            for (int q = 0; q < 8; ++q) P.fa[q][frow + 1][col] = g.a[q];
         }
         __syncthreads();
         for (int k = t; k < (ATY + 2) * ATX; k += ANT) {  // slope reverse, rows y0-1 .. y0+TY
@@ -840,29 +1013,39 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
             const int r = row + H3, c = col + H3;
             for (int qi = 0; qi < 3; ++qi) {  // as in the x pass: faces row (R side) and row+1 (L side)
                 const int qL = qi == 0 ? 0 : 2 + 2 * qi, qR = qL + 1;
-                const double gs2 = P.fa[qL][row + 2][col] - P.fa[qR][row + 1][col];
-                const double(*Q)[GX] = qi == 0 ? S.eta : (qi == 1 ? S.u : S.v);
-                double gm, g0, gp;
-                if constexpr (FAST) slope_rev_rs(Q[r - 1][c], Q[r][c], Q[r + 1][c], P.rs[qi][row + 2][col], gs2, gm, g0, gp);
-                else slope_rev(Q[r - 1][c], Q[r][c], Q[r + 1][c], 0.5 * gs2, gm, g0, gp);
+                const V gs2 = vsub(P.fa[qL][row + 2][col], P.fa[qR][row + 1][col]);
+                V gm, g0, gp;
+                if constexpr (FAST) {
+                    const F2 dm = qi == 0 ? f2_of(S.eta[r][c] - S.eta[r - 1][c])
+                                          : (qi == 1 ? f2_sub(S.u[r][c], S.u[r - 1][c]) : f2_sub(S.v[r][c], S.v[r - 1][c]));
+                    const F2 dp = qi == 0 ? f2_of(S.eta[r + 1][c] - S.eta[r][c])
+                                          : (qi == 1 ? f2_sub(S.u[r + 1][c], S.u[r][c]) : f2_sub(S.v[r + 1][c], S.v[r][c]));
+                    slope_rev_pair(dm, dp, P.rs[qi][row + 2][col], gs2, gm, g0, gp);
+                } else {
+                    const double(*Q)[GX] = qi == 0 ? S.eta : (qi == 1 ? S.u : S.v);
+                    slope_rev(Q[r - 1][c], Q[r][c], Q[r + 1][c], 0.5 * gs2, gm, g0, gp);
+                }
                 P.sp[3 * qi + 0][row + 1][col] = gm;
                 P.sp[3 * qi + 1][row + 1][col] = g0;
                 P.sp[3 * qi + 2][row + 1][col] = gp;
             }
         }
         __syncthreads();
-        auto gather_y = [&](int row, int col, double& ge, double& gu, double& gv, double& gz) {
-            auto F = [&](int q, int frow) { return (frow >= -1 && frow <= ATY + 1) ? P.fa[q][frow + 1][col] : 0.0; };
-            auto SP = [&](int q, int srow) { return (srow >= -1 && srow <= ATY) ? P.sp[q][srow + 1][col] : 0.0; };
-            ge = A.cy * (F(1, row) + F(0, row + 1) + SP(2, row - 1) + SP(1, row) + SP(0, row + 1));
-            gu = A.cy * (F(5, row) + F(4, row + 1) + SP(5, row - 1) + SP(4, row) + SP(3, row + 1));
-            gv = A.cy * (F(7, row) + F(6, row + 1) + SP(8, row - 1) + SP(7, row) + SP(6, row + 1));
-            gz = A.cy * (F(3, row) + F(2, row + 1));
+        V cyv;
+        if constexpr (FAST) cyv = f2_of_rn(A.cy);
+        else cyv = A.cy;
+        auto gather_y = [&](int row, int col, V& ge, V& gu, V& gv, V& gz) {
+            auto F = [&](int q, int frow) { return (frow >= -1 && frow <= ATY + 1) ? P.fa[q][frow + 1][col] : V{}; };
+            auto SP = [&](int q, int srow) { return (srow >= -1 && srow <= ATY) ? P.sp[q][srow + 1][col] : V{}; };
+            ge = vmul(cyv, vadd(vadd(vadd(F(1, row), F(0, row + 1)), vadd(SP(2, row - 1), SP(1, row))), SP(0, row + 1)));
+            gu = vmul(cyv, vadd(vadd(vadd(F(5, row), F(4, row + 1)), vadd(SP(5, row - 1), SP(4, row))), SP(3, row + 1)));
+            gv = vmul(cyv, vadd(vadd(vadd(F(7, row), F(6, row + 1)), vadd(SP(8, row - 1), SP(7, row))), SP(6, row + 1)));
+            gz = vmul(cyv, vadd(F(3, row), F(2, row + 1)));
         };
         {
-            double ge, gu, gv, gz;
+            V ge, gu, gv, gz;
             gather_y(ty, tx, ge, gu, gv, gz);
-            ae += ge; au += gu; av += gv; az += gz;
+            ae = vadd(ae, ge); au = vadd(au, gu); av = vadd(av, gv); az = vadd(az, gz);
         }
         if (t < ATX && x0 + t < nx) {
             const int col = t, c = col + H3;
@@ -873,14 +1056,16 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
                 for (int k = 1; k <= 2; ++k) {
                     const int gj = lo ? -k : ny - 1 + k;
                     const int row = gj - y0, r = row + H3;
-                    double ge, gu, gv, gz;
-                    gather_y(row, col, ge, gu, gv, gz);
+                    V pe, pu, pv, pz;
+                    gather_y(row, col, pe, pu, pv, pz);
+                    const double ge = lscale * flux_of(pe), gu = lscale * flux_of(pu), gv = lscale * flux_of(pv),
+                                 gz = lscale * flux_of(pz);
                     const double hp = S.hp[r][c];
                     double gzt = gz + ge, ghp = ge, ghu = 0, ghv = 0;
                     if (gt_bits(hp, Cst<double>::tol12_bits)) {
                         ghu = gu / hp;
                         ghv = gv / hp;
-                        ghp -= (gu * S.u[r][c] + gv * S.v[r][c]) / hp;
+                        ghp -= (gu * flux_of(S.u[r][c]) + gv * flux_of(S.v[r][c])) / hp;
                     }
                     double geta = 0;
                     if (pos_i(hp)) { geta = ghp; gzt -= ghp; }
@@ -912,24 +1097,40 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
     if (own) {
         const int r = ty + H3, c = tx + H3;
         const double hp = S.hp[r][c];
-        double gz = az + ae, ghp = ae, ghu = 0, ghv = 0;
-        if (gt_bits(hp, Cst<double>::tol12_bits)) {
-            const double rh = FAST ? rcp_nr(hp) : 1.0 / hp;
-            ghu = au * rh;
-            ghv = av * rh;
-            ghp -= (au * S.u[r][c] + av * S.v[r][c]) * rh;
+        double gz, gh = 0.0, ghu = 0.0, ghv = 0.0;
+        // h' = max(0, (h + z) - z): dh'/dh = 1, dh'/dz = 0 where h' > 0
+        if constexpr (FAST) {
+            const bool wet = gt_bits(hp, Cst<double>::tol12_bits);
+            F2 h2 = f2_of(hp);
+            h2.h = wet ? h2.h : 1.f;
+            const F2 rh = f2_rcp(h2);
+            const F2 pu = f2_sel(wet, f2_mul(au, rh)), pv = f2_sel(wet, f2_mul(av, rh));
+            const F2 ph = f2_sub(ae, f2_add(f2_mul_raw(pu, S.u[r][c]), f2_mul_raw(pv, S.v[r][c])));
+            gz = lscale * f64_of(f2_add(az, ae));
+            gh = pos_i(hp) ? lscale * f64_of(ph) : 0.0;
+            ghu = lscale * f64_of(pu);
+            ghv = lscale * f64_of(pv);
+        } else {
+            gz = az + ae;
+            double ghp = ae;
+            if (gt_bits(hp, Cst<double>::tol12_bits)) {
+                const double rh = 1.0 / hp;
+                ghu = au * rh;
+                ghv = av * rh;
+                ghp -= (au * S.u[r][c] + av * S.v[r][c]) * rh;
+            }
+            if (pos_i(hp)) gh = ghp;
         }
-        double gh = 0;
-        if (pos_i(hp)) gh = ghp;  // h' = max(0, (h + z) - z): dh'/dh = 1, dh'/dz = 0
         const long long o = (long long)gi + (long long)gj * A.pitch;
         // lambda^n = lambda_lin (the stored state passes through the update) + the flux part + ghost folds
-        A.out[0][o] = S.lam[0][r][c] + gh + S.fold[0][ty][tx];
-        A.out[1][o] = S.lam[1][r][c] + ghu + S.fold[1][ty][tx];
-        A.out[2][o] = S.lam[2][r][c] + ghv + S.fold[2][ty][tx];
+        const double l0 = A.lam[0][o], l1 = A.lam[1][o], l2 = A.lam[2][o];
+        A.out[0][o] = l0 + gh + S.fold[0][ty][tx];
+        A.out[1][o] = l1 + ghu + S.fold[1][ty][tx];
+        A.out[2][o] = l2 + ghv + S.fold[2][ty][tx];
         A.zbar[o] += gz + S.fold[3][ty][tx];
         if (A.un1[0])
-            dtb = (S.lam[0][r][c] * (A.un1[0][o] - A.src.h[o]) + S.lam[1][r][c] * (A.un1[1][o] - A.src.hu[o]) +
-                   S.lam[2][r][c] * (A.un1[2][o] - A.src.hv[o])) * A.idt;
+            dtb = (l0 * (A.un1[0][o] - A.src.h[o]) + l1 * (A.un1[1][o] - A.src.hu[o]) +
+                   l2 * (A.un1[2][o] - A.src.hv[o])) * A.idt;
     }
     // The block's CFL arg max.  The fast form screens it in float first (as the forward's fold does): only
     // the cells within 2^-12 of the block's largest float estimate, or with a non-finite one, take the FP64
@@ -1478,7 +1679,7 @@ int adjoint_reverse_binomial(const hx_level_f64* L, int nsteps, double cfl, int 
     double* lamb[2] = {V.state(A.lam, 0), V.state(A.lam, 1)};
     if (e == cudaSuccess) e = cudaMemsetAsync(lamb[0], 0, 3 * pb, st);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_adj_faces<FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AdjSmem));
+        e = cudaFuncSetAttribute(k_adj_faces<FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AdjSmem<double>));
     if (e != cudaSuccess) return set_error(HX_ERR_CUDA, cudaGetErrorString(e));
     const IBox vb{0, 0, L->nx - 1, L->ny - 1};
     const dim3 grid = tile_grid(vb, ATX, ATY);
@@ -1546,7 +1747,7 @@ int adjoint_reverse_binomial(const hx_level_f64* L, int nsteps, double cfl, int 
         }
         AdjArgs B = faces_args(L, A, base, Uj, un1, lam_for_faces, lam0, grad_z, dt);
         fused_finish(B, (int)j);
-        k_adj_faces<FAST><<<grid, ANT, sizeof(AdjSmem), st>>>(B);
+        k_adj_faces<FAST><<<grid, ANT, sizeof(AdjSmem<double>), st>>>(B);
         ++launches;
         if (r == cudaSuccess) r = cudaGetLastError();
         if (r == cudaSuccess && j > 0) r = cudaMemcpyAsync(nxt, Uj, 3 * pb, cudaMemcpyDeviceToDevice, st);
@@ -1621,11 +1822,11 @@ int adjoint_reverse(const hx_level_f64* L, int nsteps, double cfl, int ngauges, 
     double* lamb[2] = {V.state(A.lam, 0), V.state(A.lam, 1)};
     if (e == cudaSuccess) e = cudaMemsetAsync(lamb[0], 0, 3 * pb, st);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_adj_faces<FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AdjSmem));
+        e = cudaFuncSetAttribute(k_adj_faces<FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AdjSmem<double>));
     if constexpr (FAST) {
         if (e == cudaSuccess && use_rec)
             e = cudaFuncSetAttribute(k_adj_faces<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sizeof(AdjSmem));
+                                     (int)sizeof(AdjSmem<double>));
     }
     SideStream side;
     if (e == cudaSuccess && A.seg) e = side.init();
@@ -1728,12 +1929,12 @@ int adjoint_reverse(const hx_level_f64* L, int nsteps, double cfl, int ngauges, 
             if constexpr (FAST) {
                 if (use_rec) {
                     B.rec = rec_at(A, base, (sg & 1) * L_seg + (n - n0), L->nx, L->ny);
-                    k_adj_faces<true, true><<<grid, ANT, sizeof(AdjSmem), st>>>(B);
+                    k_adj_faces<true, true><<<grid, ANT, sizeof(AdjSmem<double>), st>>>(B);
                 } else {
-                    k_adj_faces<FAST><<<grid, ANT, sizeof(AdjSmem), st>>>(B);
+                    k_adj_faces<FAST><<<grid, ANT, sizeof(AdjSmem<double>), st>>>(B);
                 }
             } else {
-                k_adj_faces<FAST><<<grid, ANT, sizeof(AdjSmem), st>>>(B);
+                k_adj_faces<FAST><<<grid, ANT, sizeof(AdjSmem<double>), st>>>(B);
             }
             ++launches;
             if (e == cudaSuccess) e = cudaGetLastError();
@@ -1775,7 +1976,7 @@ int adjoint_step(const hx_level_f64* L, double dt, const double* const* lam, dou
                               L->nx * sizeof(double), L->ny, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_adj_faces<FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AdjSmem));
+        e = cudaFuncSetAttribute(k_adj_faces<FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AdjSmem<double>));
     if (e != cudaSuccess) return set_error(HX_ERR_CUDA, cudaGetErrorString(e));
     e = linear_step<FAST>(L, un, A.plane, lin, dth, st);
     if (e != cudaSuccess) return set_error(HX_ERR_LAUNCH, cudaGetErrorString(e));
@@ -1787,7 +1988,7 @@ int adjoint_step(const hx_level_f64* L, double dt, const double* const* lam, dou
     k_adj_post<<<grid, ANT, 0, st>>>(P);
     AdjArgs B = faces_args(L, A, base, un, nullptr, ll, ll, zbar, dt);  // outputs replaced below
     for (int k = 0; k < 3; ++k) B.out[k] = outs[k];
-    k_adj_faces<FAST><<<grid, ANT, sizeof(AdjSmem), st>>>(B);
+    k_adj_faces<FAST><<<grid, ANT, sizeof(AdjSmem<double>), st>>>(B);
     e = cudaGetLastError();
     if (e == cudaSuccess) {  // dtbar = sum of the per-block partials
         std::vector<double> parts((size_t)A.nblocks);

@@ -511,27 +511,25 @@ __host__ __device__ __forceinline__ void roe_hydrostatic_exact(R hi, R hui, R hv
     else { F1 = -f2; F2 = f1; }
 }
 
-// Intermediates of one fast-form face flux that its reverse needs: square
-// roots, the shared reciprocal, Roe averages, the entropy-fixed speeds and the
-// half wave strengths, with the branch flags.  Recorded by the adjoint's
-// segment recompute so the reverse sweep does not evaluate them again.
+// Intermediates of one fast-form FP64 face flux that its reverse needs, in float pairs: square roots, the shared
+// reciprocals, Roe averages and the half wave strengths, with the branch flags.  Recorded by the adjoint's segment
+// recompute so the reverse sweep does not evaluate them again; a face with RR_OTHER (an entropy fix, or a state past
+// the pairs' range) holds nothing else, and its reverse evaluates it in FP64.
 struct RoeRecVals {
-    double si, sj, cm, rs, hrden, hrcm, um, vm, l0, l2, a0h, a1h, a2h;  // 1/sden, 1/(2 den), 1/(2 cm)
-    unsigned fl;  // RR_WI | RR_WJ | RR_HM | RR_FIX0 | RR_FIX2
+    F2 si, sj, cm, rs, hrcm, um, vm, a0h, a1h, a2h;  // rs = 1 / sden, hrcm = 1 / (2 cm)
+    unsigned fl;
 };
-constexpr int NREC = 13;  // doubles of a RoeRecVals
-constexpr unsigned RR_WI = 1u, RR_WJ = 2u, RR_HM = 4u, RR_FIX0 = 8u, RR_FIX2 = 16u;
+constexpr int NREC = 10;  // pairs of a RoeRecVals
+constexpr unsigned RR_WI = 1u, RR_WJ = 2u, RR_HM = 4u, RR_OTHER = 8u;
 
 // Fast form: inputs are the face depths and face velocities (the reference
 // rebuilds the velocity as (h u)/h, which equals u to an ulp).  In FP64 one
 // reciprocal 1/(sden den) gives both 1/sden (the Roe averages) and 1/den (two
 // wave strengths), and 1/cm (the contact wave) comes from the correction step
-// of cm's own square root; the wave speeds sqrt(g h) reuse sqrt(h).  With REC
-// the intermediates go to *rv (values only stored: the arithmetic is the same
-// instruction for instruction).
-template <class R, int DIR, bool REC = false>
+// of cm's own square root; the wave speeds sqrt(g h) reuse sqrt(h).
+template <class R, int DIR>
 __host__ __device__ __forceinline__ void roe_hydrostatic_fast(R hi, R ui, R vi, R hj, R uj, R vj, R& F0, R& F1,
-                                                             R& F2, RoeRecVals* rv = nullptr) {
+                                                             R& F2) {
     using C = Cst<R>;
     // depths arrive non-negative (capped with max(0, .)), so bit comparisons apply
     const bool wi = ge_bits(hi, C::toldry_bits), wj = ge_bits(hj, C::toldry_bits);
@@ -616,13 +614,6 @@ __host__ __device__ __forceinline__ void roe_hydrostatic_fast(R hi, R ui, R vi, 
     F0 = f0;
     if (DIR == 0) { F1 = f1; F2 = f2; }
     else { F1 = -f2; F2 = f1; }
-    if constexpr (REC) {
-        rv->si = si; rv->sj = sj; rv->cm = cm; rv->rs = rs; rv->hrden = hrden; rv->hrcm = hrcm;
-        rv->um = um; rv->vm = vm; rv->l0 = l0; rv->l2 = l2;
-        rv->a0h = a0h; rv->a1h = a1h; rv->a2h = a2h;
-        rv->fl = (wi ? RR_WI : 0u) | (wj ? RR_WJ : 0u) | (hmb ? RR_HM : 0u) | (fix0 ? RR_FIX0 : 0u) |
-                 (fix2 ? RR_FIX2 : 0u);
-    }
 }
 
 // ----------------------------------------------------------------------------

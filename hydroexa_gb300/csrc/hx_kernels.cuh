@@ -66,10 +66,9 @@ using TileSmem = HydroSmem<R, TXv, TYv, std::conditional_t<kPairs<R, FAST>, F2, 
 
 // One hydrostatic face (src/solvers/HydrostaticRoe.cpp:218-396).  L and R are
 // the cells on either side; sX are the cells' slopes along the face normal.
-template <class R, bool FAST, int DIR, bool REC = false>
+template <class R, bool FAST, int DIR>
 __device__ __forceinline__ void hydro_face(bool wall, R zL, R zR, R eL, R eR, R seL, R seR, R uL, R uR, R suL, R suR,
-                                           R vL, R vR, R svL, R svR, R& Fm, R& Fl, R& Fr, R& Ft,
-                                           RoeRecVals* rv = nullptr) {
+                                           R vL, R vR, R svL, R svR, R& Fm, R& Fl, R& Fr, R& Ft) {
     // wall: either side is NODATA (HydrostaticRoe.cpp:237-245)
     if (wall) {
         Fm = Fl = Fr = Ft = R(0);
@@ -116,7 +115,7 @@ __device__ __forceinline__ void hydro_face(bool wall, R zL, R zR, R eL, R eR, R 
         const R hvR = (hRs > R(0)) ? hRs * vRf : R(0);
         roe_hydrostatic_exact<DIR>(hLs, huL, hvL, hRs, huR, hvR, f0, f1, f2);
     } else {
-        roe_hydrostatic_fast<R, DIR, REC>(hLs, uLf, vLf, hRs, uRf, vRf, f0, f1, f2, rv);
+        roe_hydrostatic_fast<R, DIR>(hLs, uLf, vLf, hRs, uRf, vRf, f0, f1, f2);
     }
     // hydrostatic pressure correction on the normal momentum
     Fm = f0;
@@ -190,11 +189,50 @@ __device__ __forceinline__ double half_slope(double qm, double q, double qp, F2*
 
 // The flux of roe_hydrostatic_fast for states beyond the pair form's range (depths from 2^32 m, speeds from
 // 2^24 m/s, NaN and infinities), in FP64 throughout.  Not inlined: no ordinary face comes here.
-template <int DIR, bool REC>
+template <int DIR>
 __device__ __noinline__ void roe_hydrostatic_far(double hi, double ui, double vi, double hj, double uj, double vj,
-                                                 double* F, RoeRecVals* rv) {
-    roe_hydrostatic_fast<double, DIR, REC>(hi, ui, vi, hj, uj, vj, F[0], F[1], F[2], rv);
+                                                 double* F) {
+    roe_hydrostatic_fast<double, DIR>(hi, ui, vi, hj, uj, vj, F[0], F[1], F[2]);
 }
+// The Roe averages and wave terms of a face in pairs, from its depths Hi, Hj, their difference dh and the normal and
+// tangential velocities (0 on a dry side): see roe_hydrostatic_pair.
+struct RoePair {
+    F2 si, sj, ghm, cm, rc, rs, um, vm;  // rc = 1 / cm, rs = 1 / (si + sj + tol12)
+    F2 m, mv;                            // si sj du / 2, si sj dv / 2
+    F2 A, cB;                            // dh / 2, c B
+    float tc;                            // tol12 / (2 c)
+    bool hmb, rule0, rule2;              // hm above its floor; the entropy fixes ruled out
+};
+__device__ __forceinline__ RoePair roe_pair_state(F2 Hi, F2 Hj, F2 dh, F2 uni, F2 uti, F2 unj, F2 utj) {
+    float r;
+    const F2 si = f2_sqrt(Hi, r), sj = f2_sqrt(Hj, r);
+    const F2 hs = f2_add(Hi, Hj);
+    const bool hmb = hs.h > 2e-6f;
+    // c^2 = g hm: (g / 2)(hi + hj), floored at g toldry
+    F2 ghm = f2_mul(F2{4.905f, (float)(4.905 - (double)4.905f)}, hs);
+    if (!hmb) ghm = F2{9.81e-6f, (float)(9.81e-6 - (double)9.81e-6f)};
+    const F2 cm = f2_sqrt(ghm, r);
+    const F2 rc = f2_norm(r, __fmul_rn(r, __fmaf_rn(-cm.l, r, __fmaf_rn(-cm.h, r, 1.f))));  // 1 / cm
+    const float tc = __fmul_rn(0.5e-12f, rc.h);                                            // tol12 / (2 c)
+    const F2 rs = f2_rcp(f2_add(f2_add(si, sj), F2{1e-12f, 0.f}));
+    const F2 um = f2_mul(f2_add(f2_mul_raw(uni, si), f2_mul_raw(unj, sj)), rs);
+    const F2 vm = f2_mul(f2_add(f2_mul_raw(uti, si), f2_mul_raw(utj, sj)), rs);
+    const float ts = __fmul_rn(__fmul_rn(1e-12f, rs.h), dh.h);  // dh tol12 / (si + sj)
+    const F2 ss = f2_half(f2_mul(si, sj));
+    F2 m = f2_mul(ss, f2_sub(unj, uni)), mv = f2_mul(ss, f2_sub(utj, uti));  // halved
+    m.l = __fmaf_rn(0.5f * um.h, ts, m.l);  // the averages' guard: -(um - u) dh / 2
+    mv.l = __fmaf_rn(0.5f * vm.h, ts, mv.l);
+    F2 A = f2_half(dh), cB = m;
+    A.l = __fmaf_rn(-tc, A.h, A.l);
+    cB.l = __fmaf_rn(-tc, cB.h, cB.l);
+    // the entropy fixes, ruled out in float where a sign is certain (roe_hydrostatic_fast)
+    const float ci = __fmul_rn(3.13209195f, si.h), cj = __fmul_rn(3.13209195f, sj.h);
+    const float mi = 0x1p-16f * (fabsf(uni.h) + ci), mj = 0x1p-16f * (fabsf(unj.h) + cj);
+    const bool rule0 = (uni.h - ci >= mi) | (unj.h - cj <= -mj);
+    const bool rule2 = (uni.h + ci >= mi) | (unj.h + cj <= -mj);
+    return {si, sj, ghm, cm, rc, rs, um, vm, m, mv, A, cB, tc, hmb, rule0, rule2};
+}
+
 // roe_hydrostatic_fast with velocities and every dissipation term in float pairs: the mass flux Fm, the
 // normal momentum flux Fn and the transverse one Ft (all along +x, +y).  What stays in FP64: the
 // jump dh = hj - hi, exact where the depths are close, so that the dissipation scales with it; the hydrostatic
@@ -226,8 +264,6 @@ __device__ __forceinline__ void roe_hydrostatic_pair(double hi, F2 ui, F2 vi, do
     const F2 uni = f2_sel(wi, DIR == 0 ? ui : vi), uti = f2_sel(wi, DIR == 0 ? vi : f2_neg(ui));
     const F2 unj = f2_sel(wj, DIR == 0 ? uj : vj), utj = f2_sel(wj, DIR == 0 ? vj : f2_neg(uj));
     const F2 Hi = f2_of(hi), Hj = f2_of(hj), dh = f2_of(__dadd_rn(hj, -hi));
-    float r;
-    const F2 si = f2_sqrt(Hi, r), sj = f2_sqrt(Hj, r);
     {
         const unsigned top = (1023u + 32u) << 20;  // depths are non-negative here; NaN and inf are above
         const bool in = ((unsigned)__double2hiint(hi) < top) & ((unsigned)__double2hiint(hj) < top) &
@@ -235,36 +271,21 @@ __device__ __forceinline__ void roe_hydrostatic_pair(double hi, F2 ui, F2 vi, do
                         (fabsf(utj.h) < 0x1p24f);
         if (!in) {
             double F[3];
-            roe_hydrostatic_far<DIR, REC>(hi, f64_of(ui), f64_of(vi), hj, f64_of(uj), f64_of(vj), F, rv);
+            roe_hydrostatic_far<DIR>(hi, f64_of(ui), f64_of(vi), hj, f64_of(uj), f64_of(vj), F);
+            if constexpr (REC) *rv = RoeRecVals{{}, {}, {}, {}, {}, {}, {}, {}, {}, {}, RR_OTHER};
             Fm = f2_of(F[0]);
             Fn = F[1 + DIR];
             Ft = f2_of(F[2 - DIR]);
             return;
         }
     }
-    const F2 hs = f2_add(Hi, Hj);
-    const bool hmb = hs.h > 2e-6f;
-    // c^2 = g hm: (g / 2)(hi + hj), floored at g toldry
-    F2 ghm = f2_mul(F2{4.905f, (float)(4.905 - (double)4.905f)}, hs);
-    if (!hmb) ghm = F2{9.81e-6f, (float)(9.81e-6 - (double)9.81e-6f)};
-    const F2 cm = f2_sqrt(ghm, r);
-    const F2 rc = f2_norm(r, __fmul_rn(r, __fmaf_rn(-cm.l, r, __fmaf_rn(-cm.h, r, 1.f))));  // 1 / cm
-    const float tc = __fmul_rn(0.5e-12f, rc.h);                                            // tol12 / (2 c)
-    const F2 rs = f2_rcp(f2_add(f2_add(si, sj), F2{1e-12f, 0.f}));
-    const F2 um = f2_mul(f2_add(f2_mul_raw(uni, si), f2_mul_raw(unj, sj)), rs);
-    const F2 vm = f2_mul(f2_add(f2_mul_raw(uti, si), f2_mul_raw(utj, sj)), rs);
-    const float ts = __fmul_rn(__fmul_rn(1e-12f, rs.h), dh.h);  // dh tol12 / (si + sj)
-    const F2 ss = f2_half(f2_mul(si, sj));
-    F2 m = f2_mul(ss, f2_sub(unj, uni)), mv = f2_mul(ss, f2_sub(utj, uti));  // halved
-    m.l = __fmaf_rn(0.5f * um.h, ts, m.l);  // the averages' guard: -(um - u) dh / 2
-    mv.l = __fmaf_rn(0.5f * vm.h, ts, mv.l);
-    F2 A = f2_half(dh), cB = m;
-    A.l = __fmaf_rn(-tc, A.h, A.l);
-    cB.l = __fmaf_rn(-tc, cB.h, cB.l);
+    const RoePair q = roe_pair_state(Hi, Hj, dh, uni, uti, unj, utj);
+    const F2 &si = q.si, &sj = q.sj, &ghm = q.ghm, &cm = q.cm, &rc = q.rc, &um = q.um, &vm = q.vm, &m = q.m, &mv = q.mv;
+    const F2 &A = q.A, &cB = q.cB;
+    const float tc = q.tc;
     // the signs of um - cm and um + cm, certain in float where they differ and irrelevant where they do not
     const bool super = fabsf(um.h) > cm.h;
     F2 P, cQ, w, wl;
-    F2 l0, l2;
     bool fix0 = false, fix2 = false;
     {
         const F2 B = f2_mul(cB, rc), cA = f2_mul(cm, A);
@@ -275,53 +296,38 @@ __device__ __forceinline__ void roe_hydrostatic_pair(double hi, F2 ui, F2 vi, do
         cQ.l = super ? __int_as_float(__float_as_int(cB.l) ^ s) : cA.l;
         w = f2_add(f2_mul_raw(um, P), cQ);
         wl = f2_add(f2_mul_raw(f2_add(f2_mul_raw(um, um), ghm), P), f2_mul_raw(F2{um.h + um.h, um.l + um.l}, cQ));
-        F2 a0 = f2_half(f2_sub(A, B)), a2 = f2_half(f2_add(A, B));
-        // the entropy fixes, ruled out in float where a sign is certain (roe_hydrostatic_fast)
-        const float ci = __fmul_rn(3.13209195f, si.h), cj = __fmul_rn(3.13209195f, sj.h);
-        const float mi = 0x1p-16f * (fabsf(uni.h) + ci), mj = 0x1p-16f * (fabsf(unj.h) + cj);
-        const bool rule0 = (uni.h - ci >= mi) | (unj.h - cj <= -mj);
-        const bool rule2 = (uni.h + ci >= mi) | (unj.h + cj <= -mj);
-        if (REC || !(rule0 && rule2)) {
-            l0 = f2_sub(um, cm);
-            l2 = f2_add(um, cm);
-        }
-        if (!(rule0 && rule2)) {
+        if (!(q.rule0 & q.rule2)) {
+            F2 l0 = f2_sub(um, cm), l2 = f2_add(um, cm);
             constexpr F2 kSqrtG{3.1320919526731650f, (float)(3.1320919526731650 - (double)3.1320919526731650f)};
             const F2 Ci = f2_mul(kSqrtG, si), Cj = f2_mul(kSqrtG, sj);
             F2 ei = f2_sub(uni, Ci), ej = f2_sub(unj, Cj);
-            fix0 = !rule0 && ei.h < 0.f && ej.h > 0.f;
+            fix0 = !q.rule0 && ei.h < 0.f && ej.h > 0.f;
             if (fix0) {
                 const F2 d = f2_sub(ej, ei);
                 l0 = f2_div(f2_mul(ei, f2_sub(ej, l0)), d, f_rcp(d.h));
             }
             ei = f2_add(uni, Ci);
             ej = f2_add(unj, Cj);
-            fix2 = !rule2 && ei.h < 0.f && ej.h > 0.f;
+            fix2 = !q.rule2 && ei.h < 0.f && ej.h > 0.f;
             if (fix2) {
                 const F2 d = f2_sub(ej, ei);
                 l2 = f2_div(f2_mul(ej, f2_sub(l2, ei)), d, f_rcp(d.h));
             }
             if (fix0 || fix2) {  // the wave strengths of the fixed speeds: (l2 - u) dh - m, (u - l0) dh + m
-                const F2 q = f2_half(rc), m2{m.h + m.h, m.l + m.l};
-                const F2 hd = f2_half(F2{q.h, __fmaf_rn(-tc, q.h, q.l)});  // 1 / (4 c + 2 tol12)
-                a0 = f2_mul(f2_sub(f2_mul_raw(f2_sub(l2, um), dh), m2), hd);
-                a2 = f2_mul(f2_add(f2_mul_raw(f2_sub(um, l0), dh), m2), hd);
+                const F2 k = f2_half(rc), m2{m.h + m.h, m.l + m.l};
+                const F2 hd = f2_half(F2{k.h, __fmaf_rn(-tc, k.h, k.l)});  // 1 / (4 c + 2 tol12)
+                const F2 a0 = f2_mul(f2_sub(f2_mul_raw(f2_sub(l2, um), dh), m2), hd);
+                const F2 a2 = f2_mul(f2_add(f2_mul_raw(f2_sub(um, l0), dh), m2), hd);
                 const F2 w0 = f2_mul(f2_abs(l0), a0), w2 = f2_mul(f2_abs(l2), a2);
                 w = f2_add(w0, w2);
                 wl = f2_add(f2_mul_raw(w0, l0), f2_mul_raw(w2, l2));
             }
         }
-        if constexpr (REC) {
-            const float h = __fmul_rn(0.25f, rc.h);  // 1 / (4 cm + 2 tol12)
-            rv->si = f64_of(si); rv->sj = f64_of(sj); rv->cm = f64_of(cm); rv->rs = f64_of(rs);
-            rv->hrden = f64_of(f2_norm(h, __fmaf_rn(0.25f, rc.l, -__fmul_rn(h, tc))));
-            rv->hrcm = 0.5 * f64_of(rc);
-            rv->um = f64_of(um); rv->vm = f64_of(vm); rv->l0 = f64_of(l0); rv->l2 = f64_of(l2);
-            rv->a0h = f64_of(a0); rv->a2h = f64_of(a2);
-            rv->a1h = f64_of(f2_mul(mv, rc));
-            rv->fl = (wi ? RR_WI : 0u) | (wj ? RR_WJ : 0u) | (hmb ? RR_HM : 0u) | (fix0 ? RR_FIX0 : 0u) |
-                     (fix2 ? RR_FIX2 : 0u);
-        }
+        if constexpr (REC)
+            *rv = RoeRecVals{si, sj, cm, q.rs, f2_half(rc), um, vm, f2_half(f2_sub(A, B)), f2_mul(mv, rc),
+                             f2_half(f2_add(A, B)),
+                             (wi ? RR_WI : 0u) | (wj ? RR_WJ : 0u) | (q.hmb ? RR_HM : 0u) |
+                                 (q.rule0 & q.rule2 ? 0u : RR_OTHER)};
     }
     const F2 qi = f2_mul(Hi, uni), qj = f2_mul(Hj, unj);
     const F2 d0 = f2_sub(f2_half(f2_add(qi, qj)), w);
@@ -546,8 +552,13 @@ __device__ __forceinline__ void hydro_face_of(bool wall, R zL, R zR, R eL, R eR,
     if constexpr (kIeee<R, FAST>)
         hydro_face_ieee<DIR>(wall, zL, zR, eL, eR, seL, seR, uL, uR, suL, suR, vL, vR, svL, svR, Fm, Fl, Fr, Ft);
     else
-        hydro_face<R, FAST, DIR, REC>(wall, zL, zR, eL, eR, seL, seR, uL, uR, suL, suR, vL, vR, svL, svR, Fm, Fl, Fr,
-                                      Ft, rv);
+        {
+        if constexpr (kPairs<R, FAST>)
+            hydro_face<R, FAST, DIR, REC>(wall, zL, zR, eL, eR, seL, seR, uL, uR, suL, suR, vL, vR, svL, svR, Fm, Fl,
+                                          Fr, Ft, rv);
+        else
+            hydro_face<R, FAST, DIR>(wall, zL, zR, eL, eR, seL, seR, uL, uR, suL, suR, vL, vR, svL, svR, Fm, Fl, Fr, Ft);
+    }
 }
 
 // Fluxes and their differences as the update and the face arrays take them.
@@ -708,7 +719,7 @@ struct NoRec {
 // j in 0..ny, at i + j nx.  Each face is written once, by the tile of the cell
 // on its high side (the domain's last face by the last tile); wall faces are
 // not written (the reverse skips them).  Slope records: per direction the
-// three van Leer slopes (eta, u, v) and their reciprocals 1 / (dm + dp), six
+// three halved van Leer slopes (eta; u and v in pairs) and the reciprocals 1 / (dm + dp) in pairs, six
 // planes, of the cells the faces use: x slopes of cells i in -1..nx at
 // (i + 1) + j (nx + 2), y slopes of cells j in -1..ny at i + (j + 1) nx; each
 // written by the tile that owns the cell (ghost cells by the edge tiles).
@@ -720,28 +731,27 @@ struct FaceRec {
     double* sl[2];
     long long slplane[2];
     int nx, ny;
-    __device__ __forceinline__ void put_sx(int col, int TXv, int gi, int gj, int k, double s, double rS) const {
+    template <class V> __device__ __forceinline__ void put_sx(int col, int TXv, int gi, int gj, int k, V s, F2 rS) const {
         if (gj < 0 || gj >= ny) return;
         const bool own = (col >= 0 && col < TXv) ? (gi <= nx) : (col < 0 ? gi == -1 : gi == nx);
         if (!own) return;
         const long long o = (long long)(gi + 1) + (long long)gj * (nx + 2);
-        sl[0][k * slplane[0] + o] = s;
-        sl[0][(3 + k) * slplane[0] + o] = rS;
+        reinterpret_cast<V*>(sl[0])[k * slplane[0] + o] = s;
+        reinterpret_cast<F2*>(sl[0])[(3 + k) * slplane[0] + o] = rS;
     }
-    __device__ __forceinline__ void put_sy(int row, int TYv, int gi, int gj, int k, double s, double rS) const {
+    template <class V> __device__ __forceinline__ void put_sy(int row, int TYv, int gi, int gj, int k, V s, F2 rS) const {
         if (gi < 0 || gi >= nx) return;
         const bool own = (row >= 0 && row < TYv) ? (gj <= ny) : (row < 0 ? gj == -1 : gj == ny);
         if (!own) return;
         const long long o = (long long)gi + (long long)(gj + 1) * nx;
-        sl[1][k * slplane[1] + o] = s;
-        sl[1][(3 + k) * slplane[1] + o] = rS;
+        reinterpret_cast<V*>(sl[1])[k * slplane[1] + o] = s;
+        reinterpret_cast<F2*>(sl[1])[(3 + k) * slplane[1] + o] = rS;
     }
     __device__ __forceinline__ void put(int d, long long o, const RoeRecVals& r) const {
-        double* b = f[d] + o;
+        F2* b = reinterpret_cast<F2*>(f[d]) + o;
         const long long ps = plane[d];
-        b[0] = r.si; b[ps] = r.sj; b[2 * ps] = r.cm; b[3 * ps] = r.rs; b[4 * ps] = r.hrden; b[5 * ps] = r.hrcm;
-        b[6 * ps] = r.um; b[7 * ps] = r.vm; b[8 * ps] = r.l0; b[9 * ps] = r.l2; b[10 * ps] = r.a0h;
-        b[11 * ps] = r.a1h; b[12 * ps] = r.a2h;
+        b[0] = r.si; b[ps] = r.sj; b[2 * ps] = r.cm; b[3 * ps] = r.rs; b[4 * ps] = r.hrcm;
+        b[5 * ps] = r.um; b[6 * ps] = r.vm; b[7 * ps] = r.a0h; b[8 * ps] = r.a1h; b[9 * ps] = r.a2h;
         fl[d][o] = (unsigned char)r.fl;
     }
     __device__ __forceinline__ void put_x(int gi, int gj, const RoeRecVals& r, bool extra) const {
@@ -1058,9 +1068,9 @@ __device__ __forceinline__ void hydro_tile_body(TileSmem<R, FAST, TXv, TYv>& S, 
             const F2 s2 = half_slope(S.v[r][c - 1], S.v[r][c], S.v[r][c + 1], &rs2);
             S.sxe[row][col + 1] = s0; S.sxu[row][col + 1] = s1; S.sxv[row][col + 1] = s2;
             const int gi = x0 + col, gj = y0 + row;
-            rec.put_sx(col, TXv, gi, gj, 0, 2.0 * s0, f64_of(rs0));
-            rec.put_sx(col, TXv, gi, gj, 1, 2.0 * f64_of(s1), f64_of(rs1));
-            rec.put_sx(col, TXv, gi, gj, 2, 2.0 * f64_of(s2), f64_of(rs2));
+            rec.put_sx(col, TXv, gi, gj, 0, s0, rs0);
+            rec.put_sx(col, TXv, gi, gj, 1, s1, rs1);
+            rec.put_sx(col, TXv, gi, gj, 2, s2, rs2);
         } else if constexpr (kPairs<R, FAST>) {
             S.sxe[row][col + 1] = half_slope(S.eta[r][c - 1], S.eta[r][c], S.eta[r][c + 1]);
             S.sxu[row][col + 1] = half_slope(S.u[r][c - 1], S.u[r][c], S.u[r][c + 1]);
@@ -1084,9 +1094,9 @@ __device__ __forceinline__ void hydro_tile_body(TileSmem<R, FAST, TXv, TYv>& S, 
             const F2 s2 = half_slope(S.v[r - 1][c], S.v[r][c], S.v[r + 1][c], &rs2);
             S.sye[row + 1][col] = s0; S.syu[row + 1][col] = s1; S.syv[row + 1][col] = s2;
             const int gi = x0 + col, gj = y0 + row;
-            rec.put_sy(row, TYv, gi, gj, 0, 2.0 * s0, f64_of(rs0));
-            rec.put_sy(row, TYv, gi, gj, 1, 2.0 * f64_of(s1), f64_of(rs1));
-            rec.put_sy(row, TYv, gi, gj, 2, 2.0 * f64_of(s2), f64_of(rs2));
+            rec.put_sy(row, TYv, gi, gj, 0, s0, rs0);
+            rec.put_sy(row, TYv, gi, gj, 1, s1, rs1);
+            rec.put_sy(row, TYv, gi, gj, 2, s2, rs2);
         } else if constexpr (kPairs<R, FAST>) {
             S.sye[row + 1][col] = half_slope(S.eta[r - 1][c], S.eta[r][c], S.eta[r + 1][c]);
             S.syu[row + 1][col] = half_slope(S.u[r - 1][c], S.u[r][c], S.u[r + 1][c]);

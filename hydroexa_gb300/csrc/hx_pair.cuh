@@ -24,6 +24,12 @@ struct F2 {
     float h, l;
 };
 
+// A double kept in a pair's place, and back.
+__device__ __forceinline__ F2 f2_bits(double x) {
+    return {__int_as_float(__double2hiint(x)), __int_as_float(__double2loint(x))};
+}
+__device__ __forceinline__ double bits_f2(F2 a) { return __hiloint2double(__float_as_int(a.h), __float_as_int(a.l)); }
+
 __device__ __forceinline__ float f_rcp(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

@@ -61,6 +61,11 @@ namespace {
 
 constexpr double G = 9.81, HG = 0.5 * 9.81, TD = 1e-6, T12 = 1e-12;
 constexpr int ATX = 32, ATY = 16, ANT = 512;
+// Threads of the reverse kernel: every phase of a tile (560 and 608 faces, 576 and 640 slopes, 544 and 576 slope
+// reverses) is one pass of 20 warps where 16 warps took two, the second nearly empty.  (The exact form is bound by
+// FP64 issue and spills at 96 registers: 16 warps.)
+template <bool FAST> constexpr int kAdjThreads = FAST ? 640 : 512;
+static_assert((ATY + 4) * ATX <= kAdjThreads<true> && ATY * (ATX + 4) <= kAdjThreads<true>, "one pass per phase");
 constexpr int H3 = 3;  // forward halo of the reverse tile
 
 // sign with sgn(+-0) = 0, decided on the integer pipe
@@ -703,15 +708,15 @@ __device__ __forceinline__ void adj_finish_body(int nblocks, const double* dtbar
                                                      const double* hv, double* lam_h, double* lam_hu, double* lam_hv,
                                                      int with_dt, int ngauges, const long long* gauges,
                                                      const double* href, double seed) {
-    __shared__ double sh[ANT / 32];
-    __shared__ double s_rate[ANT / 32];
-    __shared__ long long s_idx[ANT / 32];
-    __shared__ unsigned s_fl[ANT / 32];
+    __shared__ double sh[32];
+    __shared__ double s_rate[32];
+    __shared__ long long s_idx[32];
+    __shared__ unsigned s_fl[32];
     double d = 0, rate = 0;
     long long idx = 0x7fffffffffffffffll;
     unsigned fl = 0;
     if (with_dt) {
-        for (int k = threadIdx.x; k < nblocks; k += ANT) {
+        for (int k = threadIdx.x; k < nblocks; k += (int)blockDim.x) {
             d += __ldcg(dtbar_p + k);
             const double pr = __ldcg(prate + k);
             const long long pi = __ldcg(pidx + k);
@@ -733,7 +738,7 @@ __device__ __forceinline__ void adj_finish_body(int nblocks, const double* dtbar
     }
     __syncthreads();
     if (threadIdx.x == 0 && with_dt) {
-        for (int k = 1; k < ANT / 32; ++k) {
+        for (int k = 1; k < (int)(blockDim.x >> 5); ++k) {
             if (s_rate[k] > rate || (s_rate[k] == rate && s_idx[k] < idx)) { rate = s_rate[k]; idx = s_idx[k]; }
             fl |= s_fl[k];
         }
@@ -749,7 +754,7 @@ __device__ __forceinline__ void adj_finish_body(int nblocks, const double* dtbar
         }
     }
     __syncthreads();
-    for (int k = threadIdx.x; k < ngauges; k += ANT) {  // atomic: a cell may be listed twice
+    for (int k = threadIdx.x; k < ngauges; k += (int)blockDim.x) {  // atomic: a cell may be listed twice
         const long long gcell = gauges[k];
         atomicAdd(&lam_h[gcell], seed * 2.0 * (h[gcell] - href[k]));
     }
@@ -757,7 +762,8 @@ __device__ __forceinline__ void adj_finish_body(int nblocks, const double* dtbar
 
 
 template <bool FAST, bool REC = false>
-__global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
+__global__ void __launch_bounds__(kAdjThreads<FAST>) k_adj_faces(AdjArgs A) {
+    constexpr int AFT = kAdjThreads<FAST>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using V = std::conditional_t<FAST, F2, double>;
     AdjSmem<V>& S = *reinterpret_cast<AdjSmem<V>*>(smem_raw);
@@ -768,7 +774,7 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
 
     // forward values on the grown tile (halo 3) and lambda_lin (0 outside the domain)
     [[maybe_unused]] unsigned lmax = 0;
-    for (int idx = t; idx < GX * GY; idx += ANT) {
+    for (int idx = t; idx < GX * GY; idx += AFT) {
         const int r = idx / GX, c = idx - r * GX;
         const int gi = x0 + c - H3, gj = y0 + r - H3;
         double e = 0, zz = 0, qx = 0, qy = 0, nn = 0;
@@ -801,20 +807,20 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
             }
         }
     }
-    for (int idx = t; idx < 4 * ATX * ATY; idx += ANT) (&S.fold[0][0][0])[idx] = 0.0;
+    for (int idx = t; idx < 4 * ATX * ATY; idx += AFT) (&S.fold[0][0][0])[idx] = 0.0;
     // The reverse is linear in lambda, so the fast form runs it on the tile's lambda divided by the power of two
     // of its largest value: the pairs' range then never ends it, however large or small a gradient grows.
     [[maybe_unused]] double lscale = 1.0;
     if constexpr (FAST) {
-        __shared__ unsigned s_lmax[ANT / 32];
+        __shared__ unsigned s_lmax[AFT / 32];
         lmax = __reduce_max_sync(0xffffffffu, lmax);
         if ((t & 31) == 0) s_lmax[t >> 5] = lmax;
         __syncthreads();
 #pragma unroll
-        for (int k = 0; k < ANT / 32; ++k) lmax = max(lmax, s_lmax[k]);
+        for (int k = 0; k < AFT / 32; ++k) lmax = max(lmax, s_lmax[k]);
         const int e = (int)(lmax >> 20), k = e == 0 || e == 0x7FF ? 0 : e - 1023;
         lscale = __hiloint2double((k + 1023) << 20, 0);
-        for (int idx = t; idx < GX * GY; idx += ANT)
+        for (int idx = t; idx < GX * GY; idx += AFT)
             for (int q = 0; q < 3; ++q) {
                 F2& l = (&S.lam[q][0][0])[idx];
                 l = scaled_pair(bits_f2(l), k);
@@ -828,7 +834,7 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
     // ===================== x pass =====================
     {
         auto& P = S.p.x;
-        for (int k = t; k < ATY * (ATX + 4); k += ANT) {  // slopes, columns x0-2 .. x0+TX+1
+        for (int k = t; k < ATY * (ATX + 4); k += AFT) {  // slopes, columns x0-2 .. x0+TX+1
             const int row = k / (ATX + 4), col = k % (ATX + 4) - 2;
             const int r = row + H3, c = col + H3;
             if constexpr (REC) {  // recorded for cells -1..nx; others feed no face of the domain
@@ -850,7 +856,7 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
             }
         }
         __syncthreads();
-        for (int k = t; k < ATY * (ATX + 3); k += ANT) {  // faces x0-1 .. x0+TX+1
+        for (int k = t; k < ATY * (ATX + 3); k += AFT) {  // faces x0-1 .. x0+TX+1
             const int row = k / (ATX + 3), fcol = k % (ATX + 3) - 1;  // face at the left of column fcol
             const int f = x0 + fcol, gj = y0 + row;
             const int r = row + H3, cl = fcol - 1 + H3, cr = fcol + H3;
@@ -876,7 +882,7 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
             for (int q = 0; q < 8; ++q) P.fa[q][row][fcol + 1] = g.a[q];
         }
         __syncthreads();
-        for (int k = t; k < ATY * (ATX + 2); k += ANT) {  // slope reverse, columns x0-1 .. x0+TX
+        for (int k = t; k < ATY * (ATX + 2); k += AFT) {  // slope reverse, columns x0-1 .. x0+TX
             const int row = k / (ATX + 2), col = k % (ATX + 2) - 1;
             const int r = row + H3, c = col + H3;
             // slope of this column: read as the R slope by face col (index col+1), where the face state is
@@ -914,7 +920,7 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
             gv = vmul(cxv, vadd(vadd(vadd(F(7, col), F(6, col + 1)), vadd(SP(8, col - 1), SP(7, col))), SP(6, col + 1)));
             gz = vmul(cxv, vadd(F(3, col), F(2, col + 1)));
         };
-        gather_x(ty, tx, ae, au, av, az);  // the x pass starts the cell's sums
+        if (t < ATX * ATY) gather_x(ty, tx, ae, au, av, az);  // the x pass starts the cell's sums
         // x-boundary ghosts: one thread per row folds both sides
         if (t < ATY && y0 + t < ny) {
             const int row = t, gj = y0 + row, r = row + H3;
@@ -961,7 +967,7 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
     // ===================== y pass =====================
     {
         auto& P = S.p.y;
-        for (int k = t; k < (ATY + 4) * ATX; k += ANT) {  // slopes, rows y0-2 .. y0+TY+1
+        for (int k = t; k < (ATY + 4) * ATX; k += AFT) {  // slopes, rows y0-2 .. y0+TY+1
             const int row = k / ATX - 2, col = k % ATX;
             const int r = row + H3, c = col + H3;
             if constexpr (REC) {
@@ -983,7 +989,7 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
             }
         }
         __syncthreads();
-        for (int k = t; k < (ATY + 3) * ATX; k += ANT) {  // faces y0-1 .. y0+TY+1
+        for (int k = t; k < (ATY + 3) * ATX; k += AFT) {  // faces y0-1 .. y0+TY+1
             const int frow = k / ATX - 1, col = k % ATX;
             const int f = y0 + frow, gi = x0 + col;
             const int c = col + H3, rl = frow - 1 + H3, rr = frow + H3;
@@ -1008,7 +1014,7 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
             for (int q = 0; q < 8; ++q) P.fa[q][frow + 1][col] = g.a[q];
         }
         __syncthreads();
-        for (int k = t; k < (ATY + 2) * ATX; k += ANT) {  // slope reverse, rows y0-1 .. y0+TY
+        for (int k = t; k < (ATY + 2) * ATX; k += AFT) {  // slope reverse, rows y0-1 .. y0+TY
             const int row = k / ATX - 1, col = k % ATX;
             const int r = row + H3, c = col + H3;
             for (int qi = 0; qi < 3; ++qi) {  // as in the x pass: faces row (R side) and row+1 (L side)
@@ -1042,7 +1048,7 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
             gv = vmul(cyv, vadd(vadd(vadd(F(7, row), F(6, row + 1)), vadd(SP(8, row - 1), SP(7, row))), SP(6, row + 1)));
             gz = vmul(cyv, vadd(F(3, row), F(2, row + 1)));
         };
-        {
+        if (t < ATX * ATY) {
             V ge, gu, gv, gz;
             gather_y(ty, tx, ge, gu, gv, gz);
             ae = vadd(ae, ge); au = vadd(au, gu); av = vadd(av, gv); az = vadd(az, gz);
@@ -1090,7 +1096,7 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
 
     // ===================== own cell: rebuild reverse, outputs, CFL rate, dt partial =====================
     const int gi = x0 + tx, gj = y0 + ty;
-    const bool own = gi < nx && gj < ny;
+    const bool own = t < ATX * ATY && gi < nx && gj < ny;
     double rate = 0.0, dtb = 0.0;
     long long ridx = 0x7fffffffffffffffll;
     unsigned rfl = 0;
@@ -1135,10 +1141,10 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
     // The block's CFL arg max.  The fast form screens it in float first (as the forward's fold does): only
     // the cells within 2^-12 of the block's largest float estimate, or with a non-finite one, take the FP64
     // rate; the cell holding the true maximum is always among them, ties included.
-    __shared__ double s_sum[ANT / 32], s_rate[ANT / 32];
-    __shared__ long long s_idx[ANT / 32];
-    __shared__ unsigned s_fl[ANT / 32];
-    __shared__ float s_r32[ANT / 32];
+    __shared__ double s_sum[AFT / 32], s_rate[AFT / 32];
+    __shared__ long long s_idx[AFT / 32];
+    __shared__ unsigned s_fl[AFT / 32];
+    __shared__ float s_r32[AFT / 32];
     {
         const int r = ty + H3, c = tx + H3;
         const long long o = (long long)gi + (long long)gj * A.pitch;
@@ -1166,7 +1172,7 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
             __syncthreads();
             float br = 0.f;
 #pragma unroll
-            for (int k = 0; k < ANT / 32; ++k) br = fmaxf(br, s_r32[k]);
+            for (int k = 0; k < AFT / 32; ++k) br = fmaxf(br, s_r32[k]);
             wet = bad || (wet && r32 >= br * (1.f - 0x1p-12f));
         }
         if (wet) {
@@ -1189,7 +1195,7 @@ __global__ void __launch_bounds__(ANT) k_adj_faces(AdjArgs A) {
     __syncthreads();
     if (t == 0) {
         double sum = s_sum[0];
-        for (int k = 1; k < ANT / 32; ++k) {
+        for (int k = 1; k < AFT / 32; ++k) {
             sum += s_sum[k];
             if (s_rate[k] > rate || (s_rate[k] == rate && s_idx[k] < ridx)) { rate = s_rate[k]; ridx = s_idx[k]; }
             rfl |= s_fl[k];
@@ -1747,7 +1753,7 @@ int adjoint_reverse_binomial(const hx_level_f64* L, int nsteps, double cfl, int 
         }
         AdjArgs B = faces_args(L, A, base, Uj, un1, lam_for_faces, lam0, grad_z, dt);
         fused_finish(B, (int)j);
-        k_adj_faces<FAST><<<grid, ANT, sizeof(AdjSmem<double>), st>>>(B);
+        k_adj_faces<FAST><<<grid, kAdjThreads<FAST>, sizeof(AdjSmem<double>), st>>>(B);
         ++launches;
         if (r == cudaSuccess) r = cudaGetLastError();
         if (r == cudaSuccess && j > 0) r = cudaMemcpyAsync(nxt, Uj, 3 * pb, cudaMemcpyDeviceToDevice, st);
@@ -1929,12 +1935,12 @@ int adjoint_reverse(const hx_level_f64* L, int nsteps, double cfl, int ngauges, 
             if constexpr (FAST) {
                 if (use_rec) {
                     B.rec = rec_at(A, base, (sg & 1) * L_seg + (n - n0), L->nx, L->ny);
-                    k_adj_faces<true, true><<<grid, ANT, sizeof(AdjSmem<double>), st>>>(B);
+                    k_adj_faces<true, true><<<grid, kAdjThreads<true>, sizeof(AdjSmem<double>), st>>>(B);
                 } else {
-                    k_adj_faces<FAST><<<grid, ANT, sizeof(AdjSmem<double>), st>>>(B);
+                    k_adj_faces<FAST><<<grid, kAdjThreads<FAST>, sizeof(AdjSmem<double>), st>>>(B);
                 }
             } else {
-                k_adj_faces<FAST><<<grid, ANT, sizeof(AdjSmem<double>), st>>>(B);
+                k_adj_faces<FAST><<<grid, kAdjThreads<FAST>, sizeof(AdjSmem<double>), st>>>(B);
             }
             ++launches;
             if (e == cudaSuccess) e = cudaGetLastError();
@@ -1988,7 +1994,7 @@ int adjoint_step(const hx_level_f64* L, double dt, const double* const* lam, dou
     k_adj_post<<<grid, ANT, 0, st>>>(P);
     AdjArgs B = faces_args(L, A, base, un, nullptr, ll, ll, zbar, dt);  // outputs replaced below
     for (int k = 0; k < 3; ++k) B.out[k] = outs[k];
-    k_adj_faces<FAST><<<grid, ANT, sizeof(AdjSmem<double>), st>>>(B);
+    k_adj_faces<FAST><<<grid, kAdjThreads<FAST>, sizeof(AdjSmem<double>), st>>>(B);
     e = cudaGetLastError();
     if (e == cudaSuccess) {  // dtbar = sum of the per-block partials
         std::vector<double> parts((size_t)A.nblocks);

@@ -93,6 +93,15 @@ __device__ __forceinline__ F2 f2_sqrt(F2 a, float& r) {
     return f2_norm(s, __fmul_rn(d, __fmul_rn(0.5f, r)));
 }
 
+// h^(-1/3), 0 < h in the float range: the float seed rcbrtf (within ~2^-22) and one third-order step,
+// r + r e (1/3 + 2 e / 9) with e = 1 - h r^3 in pairs
+__device__ __forceinline__ F2 f2_rcbrt(F2 h) {
+    const float r = rcbrtf(h.h);
+    const F2 r1{r, 0.f}, r3 = f2_mul(f2_mul(r1, r1), r1);
+    const F2 e = f2_add(F2{1.f, 0.f}, f2_neg(f2_mul_raw(h, r3)));
+    return f2_norm(r, __fmul_rn(__fmul_rn(r, e.h), __fmaf_rn(0.22222222f, e.h, 0.33333334f)));
+}
+
 // The leading ~48 bits of a double, made on the integer pipe (a double to
 // float conversion issues on the FP64 pipe): h the leading 24 significand bits
 // (truncated), l the other 29 rounded to a float.  Below 2^-71 l is 0, below

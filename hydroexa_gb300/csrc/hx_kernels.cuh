@@ -1154,15 +1154,29 @@ __device__ __forceinline__ void hydro_tile_body(TileSmem<R, FAST, TXv, TYv>& S, 
             S.syv[row + 1][col] = van_leer_slope<R, FAST>(S.v[r - 1][c], S.v[r][c], S.v[r + 1][c]);
         }
     };
-    for (int k = t; k < CELLS; k += NTv) {
-        xslopes(k / TXv, k % TXv);
-        yslopes(k / TXv, k % TXv);
-    }
-    for (int k = t; k < 2 * TYv + 2 * TXv; k += NTv) {
-        if (k < 2 * TYv) xslopes(k % TYv, (k < TYv) ? -1 : TXv);  // columns -1 and TX
-        else {
-            const int m = k - 2 * TYv;
-            yslopes((m < TXv) ? -1 : TYv, m % TXv);                // rows -1 and TY
+    // WIDE (a block of more than two threads per cell): every thread one cell's slopes of one direction, then one
+    // face, the y items starting at a whole warp; else every thread both directions of its cell, then the edges.
+    constexpr bool WIDE = NTv >= 2 * CELLS;
+    if constexpr (WIDE) {
+        constexpr int XS = TYv * (TXv + 2), XP = (XS + 31) / 32 * 32, YS = (TYv + 2) * TXv;
+        for (int k = t; k < XP + YS; k += NTv) {
+            if (k < XP) {
+                if (k < XS) xslopes(k / (TXv + 2), k % (TXv + 2) - 1);
+            } else {
+                yslopes((k - XP) / TXv - 1, (k - XP) % TXv);
+            }
+        }
+    } else {
+        for (int k = t; k < CELLS; k += NTv) {
+            xslopes(k / TXv, k % TXv);
+            yslopes(k / TXv, k % TXv);
+        }
+        for (int k = t; k < 2 * TYv + 2 * TXv; k += NTv) {
+            if (k < 2 * TYv) xslopes(k % TYv, (k < TYv) ? -1 : TXv);  // columns -1 and TX
+            else {
+                const int m = k - 2 * TYv;
+                yslopes((m < TXv) ? -1 : TYv, m % TXv);                // rows -1 and TY
+            }
         }
     }
     sy.bar();
@@ -1206,29 +1220,42 @@ __device__ __forceinline__ void hydro_tile_body(TileSmem<R, FAST, TXv, TYv>& S, 
             fo.store_y(x0 + fi, y0 + fj, vb, F * flux_of(Fm), F * flux_of(Ft), F * Fl, F * Fr, fj == TYv);
         }
     };
-    for (int k = t; k < CELLS; k += NTv) {
-        const int tx = k % TXv, ty = k / TXv;
-        const int gi = x0 + tx, gj = y0 + ty;
-        // a face is needed if it bounds a valid cell
-        if (gi <= vb.hi0 + 1 && gj <= vb.hi1) xface(tx, ty);
-        if (gi <= vb.hi0 && gj <= vb.hi1 + 1) yface(tx, ty);
-    }
-    // the right column and the top row: where the tile leaves enough threads without a cell, those take them
-    // (two faces at most, as every other thread), so that no thread computes a third face while the rest wait
-    constexpr int SPARE = NTv - CELLS;
-    if constexpr (SPARE >= TXv && SPARE >= TYv) {
-        const int e = t - CELLS;
-        if (e >= 0) {
-            if (e < TYv && x0 + TXv <= vb.hi0 + 1 && y0 + e <= vb.hi1) xface(TXv, e);
-            if (e < TXv && x0 + e <= vb.hi0 && y0 + TYv <= vb.hi1 + 1) yface(e, TYv);
+    if constexpr (WIDE) {
+        constexpr int XF = TYv * (TXv + 1), XP = (XF + 31) / 32 * 32, YF = (TYv + 1) * TXv;
+        for (int k = t; k < XP + YF; k += NTv) {
+            if (k < XP) {
+                const int fi = k % (TXv + 1), fj = k / (TXv + 1);
+                if (k < XF && x0 + fi <= vb.hi0 + 1 && y0 + fj <= vb.hi1) xface(fi, fj);
+            } else {
+                const int fi = (k - XP) % TXv, fj = (k - XP) / TXv;
+                if (x0 + fi <= vb.hi0 && y0 + fj <= vb.hi1 + 1) yface(fi, fj);
+            }
         }
     } else {
-        for (int k = t; k < TYv + TXv; k += NTv) {
-            if (k < TYv) {
-                if (x0 + TXv <= vb.hi0 + 1 && y0 + k <= vb.hi1) xface(TXv, k);
-            } else {
-                const int m = k - TYv;
-                if (x0 + m <= vb.hi0 && y0 + TYv <= vb.hi1 + 1) yface(m, TYv);
+        for (int k = t; k < CELLS; k += NTv) {
+            const int tx = k % TXv, ty = k / TXv;
+            const int gi = x0 + tx, gj = y0 + ty;
+            // a face is needed if it bounds a valid cell
+            if (gi <= vb.hi0 + 1 && gj <= vb.hi1) xface(tx, ty);
+            if (gi <= vb.hi0 && gj <= vb.hi1 + 1) yface(tx, ty);
+        }
+        // the right column and the top row: where the tile leaves enough threads without a cell, those take them
+        // (two faces at most, as every other thread), so that no thread computes a third face while the rest wait
+        constexpr int SPARE = NTv - CELLS;
+        if constexpr (SPARE >= TXv && SPARE >= TYv) {
+            const int e = t - CELLS;
+            if (e >= 0) {
+                if (e < TYv && x0 + TXv <= vb.hi0 + 1 && y0 + e <= vb.hi1) xface(TXv, e);
+                if (e < TXv && x0 + e <= vb.hi0 && y0 + TYv <= vb.hi1 + 1) yface(e, TYv);
+            }
+        } else {
+            for (int k = t; k < TYv + TXv; k += NTv) {
+                if (k < TYv) {
+                    if (x0 + TXv <= vb.hi0 + 1 && y0 + k <= vb.hi1) xface(TXv, k);
+                } else {
+                    const int m = k - TYv;
+                    if (x0 + m <= vb.hi0 && y0 + TYv <= vb.hi1 + 1) yface(m, TYv);
+                }
             }
         }
     }
@@ -1306,6 +1333,16 @@ constexpr int min_ctas(int threads) { return threads >= 1024 ? 1 : (threads >= 5
 struct SmallTile {
     static constexpr int X = TX, Y = TY;
 };
+// Tiles of the smallest FP64 levels and boxes, 32 x Y cells with a thread for each slope of a phase (WIDE in
+// hydro_tile_body): a level of fewer cells than the GPU has lanes is bound by the phases' latency and by the FP64
+// pipe of the few SMs it occupies, so its tiles shrink (Y = 8, 4, 2) as long as every SM still gets at most one
+// and every phase is one pass.  us per step, 32 x 8 tiles of 256 threads against these (exact / fast form): 64 x 48
+// 38.6 -> 16.3 / 18.2 -> 11.8, 128^2 38.8 -> 20.2 / 18.3 -> 14.0, 192^2 38.6 -> 28.2 / 18.2 -> 16.1; from more than
+// one tile per SM on the 256-thread tiles win, three to an SM (256^2: 50.9 against 51.9 exact, 23.0 against 28.2
+// fast).
+template <int Y> struct WideTile {
+    static constexpr int N = (Y * (TX + 2) + 31) / 32 * 32 + (Y + 2) * TX;  // slopes, more than faces
+};
 template <class R> inline bool big_tile(const IBox& vb) {
     return BigTile<R>::Y != TY &&
            (long long)(vb.hi0 - vb.lo0 + 1) * (long long)(vb.hi1 - vb.lo1 + 1) >= kBigTileCells;
@@ -1313,8 +1350,8 @@ template <class R> inline bool big_tile(const IBox& vb) {
 
 // EPI: the advance epilogue (eta and this tile's diagnostics partial, slot =
 // the block's linear index).
-template <class R, bool FAST, class Src, int TXH = TX, int TYH = TY, bool EPI = false>
-__global__ void __launch_bounds__(TXH * TYH, min_ctas(TXH * TYH))
+template <class R, bool FAST, class Src, int TXH = TX, int TYH = TY, bool EPI = false, int NTH = TXH * TYH>
+__global__ void __launch_bounds__(NTH, NTH == TXH * TYH ? min_ctas(NTH) : 1)
     k_hydro_tile(Src src, Cells3<R> uo, Plane<R> nplane, Cells3W<R> out, FaceOut<R> fo, IBox vb, StepCtl<R> ctl,
                  EpiOut<R> epi) {
     static_assert(!EPI || sizeof(TileSmem<R, FAST, TXH, TYH>) >= 4 * TXH * TYH * sizeof(double),
@@ -1325,7 +1362,7 @@ __global__ void __launch_bounds__(TXH * TYH, min_ctas(TXH * TYH))
     if (!resolve_dt(ctl, dt)) return;
     step_bookkeeping(ctl, dt);
     DiagAcc acc;
-    hydro_tile_body<R, FAST, TXH, TYH, TXH * TYH, Src, false, NoDiv, NoRec, Cells3<R>, Plane<R>, NoHooks, BlockSync,
+    hydro_tile_body<R, FAST, TXH, TYH, NTH, Src, false, NoDiv, NoRec, Cells3<R>, Plane<R>, NoHooks, BlockSync,
                     EPI>(S, src, uo, nplane, out, fo, vb, vb.lo0 + (int)blockIdx.x * TXH,
                          vb.lo1 + (int)blockIdx.y * TYH, dt, ctl.dx, ctl.dy, ctl.dt_out, ctl.status, nullptr,
                          NoDiv{}, NoRec{}, NoHooks{}, nullptr, BlockSync{}, true, &epi, &acc);
@@ -2530,11 +2567,32 @@ cudaError_t launch_hydro_k(const Src& src, const Cells3<R>& uo, const Plane<R>& 
         nblocks = (long long)g.x * g.y;
         return cudaGetLastError();
     }
+    const dim3 g = tile_grid(vb, TX, TY);
+    if constexpr (std::is_same_v<R, double> && !EPI) {
+        const long long tiles = (long long)g.x * g.y;
+        auto wide = [&](auto y) -> cudaError_t {
+            constexpr int Y = decltype(y)::value, N = WideTile<Y>::N;
+            const size_t sm = sizeof(HydroSmem<R, TX, Y>);
+            auto k = k_hydro_tile<R, FAST, Src, TX, Y, false, N>;
+            cudaError_t e = ensure_smem(k, sm);
+            if (e != cudaSuccess) return e;
+            const dim3 gw = tile_grid(vb, TX, Y);
+            k<<<gw, N, sm, st>>>(src, uo, np, out, fo, vb, ctl, epi);
+            nblocks = (long long)gw.x * gw.y;
+            return cudaGetLastError();
+        };
+        int dev = 0, sms = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        if (4 * tiles <= sms) return wide(std::integral_constant<int, 2>{});
+        if (2 * tiles <= sms) return wide(std::integral_constant<int, 4>{});
+        if (tiles <= sms) return wide(std::integral_constant<int, 8>{});
+    }
     const size_t sm = sizeof(HydroSmem<R>);
     auto k = k_hydro_tile<R, FAST, Src, TX, TY, EPI>;
     cudaError_t e = ensure_smem(k, sm);
     if (e != cudaSuccess) return e;
-    const dim3 g = tile_grid(vb, TX, TY);
     k<<<g, NT, sm, st>>>(src, uo, np, out, fo, vb, ctl, epi);
     nblocks = (long long)g.x * g.y;
     return cudaGetLastError();

@@ -171,18 +171,19 @@ __device__ __forceinline__ F2 half_slope(F2 qm, F2 q, F2 qp, F2* rs = nullptr) {
     }
     return s;
 }
-// The free surface's slope stays in FP64: the pressure that balances the bed follows from it.
+// The free surface's: its differences in FP64 (the surface hangs over a deep or high bed), rounded pairs from there,
+// within 2^-48.4 of the slope: the pressure that balances the bed follows from it.
 __device__ __forceinline__ double half_slope(double qm, double q, double qp, F2* rs = nullptr) {
-    const double dm = __dadd_rn(q, -qm), dp = __dadd_rn(qp, -q);
-    const double p = __dmul_rn(dm, dp);
-    const bool slope = !abs_le_bits(dp, Cst<double>::tol12_bits) & pos_i(p);
+    const F2 dm = f2_of_rn(__dadd_rn(q, -qm)), dp = f2_of_rn(__dadd_rn(qp, -q));
+    const bool slope = !((fabsf(dp.h) <= 1e-12f) | (__fmul_rn(dm.h, dp.h) <= 0.f));
     double s = 0.0;
     if (rs) *rs = F2{0.f, 0.f};
     const unsigned lanes = __activemask();
     if (__any_sync(lanes, slope)) {
-        const double S = __dadd_rn(dm, dp), t = van_leer_half_div(p, S);
-        s = slope ? t : 0.0;
-        if (rs) *rs = f2_sel(slope, f2_of(rcp_nr(S)));
+        const F2 S = f2_add(dm, dp);
+        const float y0 = f_rcp(S.h), y = __fmaf_rn(y0, __fmaf_rn(-S.h, y0, 1.f), y0);
+        s = f64_of(f2_sel(slope, f2_mul(dm, f2_div_rn(dp, S, y))));
+        if (rs) *rs = f2_sel(slope, f2_rcp(S));
     }
     return s;
 }

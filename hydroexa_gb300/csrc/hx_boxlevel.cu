@@ -1,9 +1,9 @@
 // C-ABI of the multi-box level: a same-level BoxArray advanced without
 // FillPatch.  The host checks that the boxes tile the domain, builds the map
 // from g x g blocks of the domain to boxes (g: the greatest common divisor of
-// the box corners) and the table of the tiles of all boxes -- 32 x 8, or on
-// levels of 2048^2 cells and more 32 x 32 for the persistent kernel, as the
-// single-box level takes them; each step is one launch over that table, with
+// the box corners) and the table of the tiles of all boxes -- 32 x 8, or from
+// kPersistCells on 32 x 32 for the persistent kernel, as the single-box level
+// takes them; each step is one launch over that table, with
 // one dt chain for the level.
 #include <cstring>
 #include <numeric>
@@ -46,7 +46,13 @@ int make_plan(int nb, const hx_levelbox_f64* boxes, int nx, int ny, Plan& P) {
         g = std::gcd(g, std::gcd(std::gcd(b.lo[0], b.lo[1]), std::gcd(b.hi[0] + 1, b.hi[1] + 1)));
     }
     P.g = g;
-    P.big = (long long)nx * (long long)ny >= kBigTileCells;
+    // the persistent kernel where a single-box level takes it, unless (below the size from which it always won) small
+    // boxes leave more than a fifth of its 32 x 32 tiles empty
+    long long full = 0;
+    for (int k = 0; k < nb; ++k)
+        full += (long long)((boxes[k].hi[0] - boxes[k].lo[0] + 32) / 32) * ((boxes[k].hi[1] - boxes[k].lo[1] + 32) / 32);
+    const long long cells = (long long)nx * (long long)ny;
+    P.big = cells >= kBigTileCells || (cells >= kPersistCells && full * 32 * 32 <= cells + cells / 4);
     const int tx = P.big ? 32 : TX, ty = P.big ? 32 : TY;
     P.mnx = nx / g;
     P.mny = ny / g;

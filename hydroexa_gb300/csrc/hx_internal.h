@@ -28,9 +28,14 @@ struct IBox {
     int lo0, lo1, hi0, hi1;
 };
 
-// Boxes (and levels) from 2048 x 2048 cells take the big FP64 tile (32 x 32, one block of 1024 threads per
-// SM): the persistent kernels on whole levels, the 32 x 32 tile kernel on boxes.
+// Boxes whose ghosts the caller fills, and the adjoint's forward steps, take the big FP64 tile kernel (32 x 32, one
+// block of 1024 threads per SM) from 2048 x 2048 cells.
 constexpr long long kBigTileCells = 1ll << 22;
+// Cells from which a level (or a band of its rows, or a multi-box level) takes a persistent kernel: six 32 x 32 tiles
+// for each of 152 SMs, below which the last round of tiles leaves too many SMs idle.  us per step, 32 x 8 tiles
+// against the persistent kernel (exact / fast form): 896^2 422 against 441 / 144 against 139, 1000^2 557 against
+// 517 / 183 against 162, 2047 x 1531 1688 against 1538 / 538 against 482.
+constexpr long long kPersistCells = 6ll * 152 * 32 * 32;
 
 // Array4-like strided view: element (i, j, c) at p[(i-lo0) + (j-lo1)*js + c*ns].
 template <class T> struct V4 {

@@ -1328,9 +1328,10 @@ template <> struct BigTile<float> {
     static constexpr int X = 32, Y = 8;
 };
 // Resident CTAs per SM the tile kernels are compiled for: 1024-thread tiles
-// one, 512-thread tiles two, 256-thread tiles three (85 registers; four, at
-// 64, spill in the exact form and moved the fast form's small levels by 1%).
-constexpr int min_ctas(int threads) { return threads >= 1024 ? 1 : (threads >= 512 ? 2 : 3); }
+// one, 512-thread tiles two, 256-thread tiles four (64 registers, against three
+// at 80: 613 x 389 rough cells 2.71 -> 2.50 ms for 41 fast steps, 512^2 exact
+// 156 -> 144 us a step although it spills).
+constexpr int min_ctas(int threads) { return threads >= 1024 ? 1 : (threads >= 512 ? 2 : 4); }
 struct SmallTile {
     static constexpr int X = TX, Y = TY;
 };
@@ -1344,10 +1345,8 @@ struct SmallTile {
 template <int Y> struct WideTile {
     static constexpr int N = (Y * (TX + 2) + 31) / 32 * 32 + (Y + 2) * TX;  // slopes, more than faces
 };
-template <class R> inline bool big_tile(const IBox& vb) {
-    return BigTile<R>::Y != TY &&
-           (long long)(vb.hi0 - vb.lo0 + 1) * (long long)(vb.hi1 - vb.lo1 + 1) >= kBigTileCells;
-}
+inline long long box_cells(const IBox& vb) { return (long long)(vb.hi0 - vb.lo0 + 1) * (long long)(vb.hi1 - vb.lo1 + 1); }
+template <class R> inline bool big_tile(const IBox& vb) { return BigTile<R>::Y != TY && box_cells(vb) >= kBigTileCells; }
 
 // EPI: the advance epilogue (eta and this tile's diagnostics partial, slot =
 // the block's linear index).
@@ -1669,7 +1668,7 @@ __global__ void __launch_bounds__(kPN, 1)
 }
 
 // ---------------------------------------------------------------------------
-// The persistent step of a multi-box level of 2048^2 cells and more: the tile
+// The persistent step of a multi-box level (from kPersistCells on): the tile
 // loop of k_hydro_persist over a table of the 32 x 32 tiles of every box.  A
 // tile's grown region is staged by cp.async from the boxes that own its cells
 // (the map of the domain), its ghosts outside the level are resolved from the
@@ -2537,9 +2536,10 @@ cudaError_t launch_hydro_k(const Src& src, const Cells3<R>& uo, const Plane<R>& 
     if constexpr (std::is_same_v<Src, LevelSrc<double>>) {
         // a whole level (or a band of its rows) on the big tile: the persistent kernel, when the stored state
         // and roughness are the level's own planes and no face arrays are asked for
-        if (big_tile<R>(vb) && !fo.on && !fo.mean && uo.p[0] == src.h && uo.p[1] == src.hu && uo.p[2] == src.hv &&
-            uo.js == src.pitch && uo.lo0 == 0 && uo.lo1 == 0 && np.p == src.n && np.js == src.pitch &&
-            np.lo0 == 0 && np.lo1 == 0) {
+        // (with an epilogue from the size on that its block sums were laid out for)
+        if (box_cells(vb) >= (EPI ? kBigTileCells : kPersistCells) && !fo.on && !fo.mean && uo.p[0] == src.h &&
+            uo.p[1] == src.hu && uo.p[2] == src.hv && uo.js == src.pitch && uo.lo0 == 0 && uo.lo1 == 0 &&
+            np.p == src.n && np.js == src.pitch && np.lo0 == 0 && np.lo1 == 0) {
             const dim3 tg = tile_grid(vb, kPX, kPY);
             const int ntiles = (int)(tg.x * tg.y);
             int dev = 0, sms = 0;
@@ -2683,7 +2683,7 @@ template <class R, bool FAST>
 cudaError_t launch_hydro_split(const LevelSrc<R>& src, const Cells3<R>& uo, const Plane<R>& np, const DivOut<R>& div,
                                const IBox& vb, R dx, R dy, cudaStream_t st) {
     if constexpr (std::is_same_v<R, double>) {
-        if (big_tile<R>(vb) && uo.p[0] == src.h && uo.p[1] == src.hu && uo.p[2] == src.hv) {
+        if (box_cells(vb) >= kPersistCells && uo.p[0] == src.h && uo.p[1] == src.hu && uo.p[2] == src.hv) {
             const dim3 tg = tile_grid(vb, kPX, kPY);
             const int ntiles = (int)(tg.x * tg.y);
             int dev = 0, sms = 0;

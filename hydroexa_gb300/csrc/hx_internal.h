@@ -36,6 +36,9 @@ constexpr long long kBigTileCells = 1ll << 22;
 // against the persistent kernel (exact / fast form): 896^2 422 against 441 / 144 against 139, 1000^2 557 against
 // 517 / 183 against 162, 2047 x 1531 1688 against 1538 / 538 against 482.
 constexpr long long kPersistCells = 6ll * 152 * 32 * 32;
+// Cells from which an FP32 level takes the marching kernel, in the fast and the exact form: below, its strips
+// leave the GPU idle in part, and a strip's rows come one after another.  us per step, 32 x 8 tiles against it: fast 768^2 27.7 / 27.6, 1000^2 39.9 / 35.9, exact 1700 x 1500 204 / 214, 2500 x 2000 390 / 366.
+constexpr long long kMarchCells = 900000, kMarchCellsExact = 3ll << 20;
 
 // Array4-like strided view: element (i, j, c) at p[(i-lo0) + (j-lo1)*js + c*ns].
 template <class T> struct V4 {

@@ -1374,6 +1374,142 @@ __global__ void __launch_bounds__(NTH, NTH == TXH * TYH ? min_ctas(NTH) : 1)
 }
 
 // ---------------------------------------------------------------------------
+// The FP32 level step without shared memory.  Bound by instruction issue, not
+// by memory: in the tile kernel a quarter of a cell's instructions move values
+// between the phases through shared memory and compute their addresses.  Here
+// a warp takes a strip of 28 columns (a lane per column, two halo lanes on
+// either side) and marches up its rows: the rows above and below stay in
+// registers, the columns beside come by shuffles, and nothing waits at a
+// barrier.  A row's y slopes and the y face below it are computed once and
+// kept for the next row.  The strips are independent of one another, so the
+// rows per strip are chosen to fill the GPU (launch_march).  The operations of
+// a face, a slope and a cell are the tile kernel's, so the state is too.
+// us per step, 32 x 8 tiles -> this (fast / exact form): 1000^2 39.9 -> 35.9 /
+// (tiles), 3001 x 2500 249 -> 184 / 579 -> 504, 8192 x 4096 1069 -> 727 /
+// 2523 -> 2034.
+// ---------------------------------------------------------------------------
+constexpr int kMarchN = 128;                                 // threads of a block
+constexpr int kMarchCols = 28, kMarchStrips = kMarchN / 32;  // columns of a strip, strips of a block
+// Blocks per SM the kernel is compiled for: the fast form six (80 registers; 3001 x 2500 188 us a step against 195 at
+// eight, where it spills, and 193 at five), the exact form, which waits for its divisions and roots, eight (505
+// against 553).
+constexpr int march_ctas(bool fast) { return fast ? 6 : 8; }
+template <class R, bool FAST>
+__global__ void __launch_bounds__(kMarchN, march_ctas(FAST))
+    k_hydro_march(LevelSrc<R> src, Cells3<R> uo, Plane<R> nplane, Cells3W<R> out, IBox vb, StepCtl<R> ctl, int rows) {
+    R dt;
+    if (!resolve_dt(ctl, dt)) return;
+    step_bookkeeping(ctl, dt);
+    struct Cell {
+        R z, eta, u, v;
+    };
+    struct Raw {
+        R e, z, qx, qy;  // e: the stored depth (fast form, cells of the level), else the free surface
+        bool stored;
+    };
+    struct Loaded {  // the roughness as the update reads it
+        R n;
+        __device__ __forceinline__ R ld(int, int) const { return n; }
+    };
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int x0 = vb.lo0 + ((int)blockIdx.x * kMarchStrips + (int)(threadIdx.x >> 5)) * kMarchCols;
+    const int y0 = vb.lo1 + (int)blockIdx.y * rows;
+    const int y1 = y0 + rows - 1 < vb.hi1 ? y0 + rows - 1 : vb.hi1;
+    const int gi = x0 - 2 + lane;
+    R kc[4];
+    tile_constants<R, FAST>(kc, dt, ctl.dx, ctl.dy);
+    R rate = R(0), mv = R(0);
+    unsigned flags = 0, pflags = 0;
+    if (x0 <= vb.hi0 && y0 <= y1) {  // the same for every lane of the warp
+        const bool act = lane >= 2 && lane < 2 + kMarchCols && gi <= vb.hi0;
+        const bool inner = src.interior(x0 - 2, 0, x0 + 29, 0);
+        auto load = [&](int j) {  // row j; ghosts by the level's rules, as the tile kernel resolves them
+            Raw w{R(0), R(0), R(0), R(0), false};
+            if (inner && j >= 0 && j < src.ny) {
+                src.fetch_in(gi, j, w.e, w.z, w.qx, w.qy);
+                if constexpr (FAST) w.stored = true;
+                else w.e += w.z;
+            } else {
+                if constexpr (FAST) w.stored = src.interior(gi, j, gi, j);
+                R nn;
+                if (w.stored) src.fetch_in(gi, j, w.e, w.z, w.qx, w.qy);
+                else if (src.inside(gi, j)) src.fetch(gi, j, w.e, w.z, w.qx, w.qy, nn);
+            }
+            return w;
+        };
+        auto cell = [&](const Raw& w) {
+            Cell c;
+            R hp;
+            if constexpr (FAST) {
+                hp = w.stored ? max0_i(w.e) : max0_i(w.e - w.z);
+                cell_velocity(hp, w.qx, w.qy, c.u, c.v);
+            } else {
+                hp = max0(w.e - w.z);
+                c.u = (hp > Cst<R>::tol12) ? w.qx / hp : R(0);
+                c.v = (hp > Cst<R>::tol12) ? w.qy / hp : R(0);
+            }
+            c.z = w.z;
+            c.eta = hp + w.z;
+            return c;
+        };
+        Cell A = cell(load(y0 - 2)), B = cell(load(y0 - 1));  // rows j and j + 1
+        R sAe = R(0), sAu = R(0), sAv = R(0);                 // y slopes of row j
+        R bm = R(0), br = R(0), bt = R(0);                    // the y face below row j, as row j sees it
+        Raw next = load(y0);
+        for (int j = y0 - 2; j <= y1; ++j) {
+            const Cell C = cell(next);  // row j + 2
+            if (j < y1) next = load(j + 3);
+            const R se = van_leer_slope<R, FAST>(A.eta, B.eta, C.eta), su = van_leer_slope<R, FAST>(A.u, B.u, C.u),
+                    sv = van_leer_slope<R, FAST>(A.v, B.v, C.v);
+            if (j >= y0 - 1) {
+                const bool update = act && j >= y0;
+                R o0 = R(0), o1 = R(0), o2 = R(0);
+                Loaded rough{R(0)};
+                if (update) {
+                    o0 = uo.ld(0, gi, j);
+                    o1 = uo.ld(1, gi, j);
+                    o2 = uo.ld(2, gi, j);
+                    rough.n = nplane.ld(gi, j);
+                }
+                const bool nodA = is_nodata(A.z);
+                R tm, tl, tr, tt;  // the y face above row j
+                hydro_face<R, FAST, 1>(nodA | is_nodata(B.z), A.z, B.z, A.eta, B.eta, sAe, se, A.u, B.u, sAu, su, A.v,
+                                       B.v, sAv, sv, tm, tl, tr, tt);
+                if (j >= y0) {
+                    const R eL = __shfl_up_sync(ALL, A.eta, 1), uL = __shfl_up_sync(ALL, A.u, 1),
+                            vL = __shfl_up_sync(ALL, A.v, 1), zL = __shfl_up_sync(ALL, A.z, 1);
+                    const R xe = van_leer_slope<R, FAST>(eL, A.eta, __shfl_down_sync(ALL, A.eta, 1));
+                    const R xu = van_leer_slope<R, FAST>(uL, A.u, __shfl_down_sync(ALL, A.u, 1));
+                    const R xv = van_leer_slope<R, FAST>(vL, A.v, __shfl_down_sync(ALL, A.v, 1));
+                    const R xeL = __shfl_up_sync(ALL, xe, 1), xuL = __shfl_up_sync(ALL, xu, 1),
+                            xvL = __shfl_up_sync(ALL, xv, 1);
+                    R fm, fl, fr, ft;  // the x face at the left of the cell
+                    hydro_face<R, FAST, 0>(is_nodata(zL) | nodA, zL, A.z, eL, A.eta, xeL, xe, uL, A.u, xuL, xu, vL, A.v,
+                                           xvL, xv, fm, fl, fr, ft);
+                    const R dx0 = __shfl_down_sync(ALL, fm, 1) - fm, dx1 = __shfl_down_sync(ALL, fl, 1) - fr,
+                            dx2 = __shfl_down_sync(ALL, ft, 1) - ft;
+                    if (update)
+                        step_cell<R, FAST, false, Loaded>(o0, o1, o2, dx0, dx1, dx2, tm - bm, tt - bt, tl - br, kc[0],
+                                                          kc[1], dt, rough, out, gi, j, nodA, ctl.dx, ctl.dy, kc[2],
+                                                          kc[3], ctl.dt_out != nullptr, rate, mv, flags, pflags);
+                }
+                bm = tm;
+                br = tr;
+                bt = tt;
+            }
+            A = B;
+            B = C;
+            sAe = se;
+            sAu = su;
+            sAv = sv;
+        }
+    }
+    if (ctl.dt_out) block_fold_dt<R, kMarchN>(rate, mv, flags, ctl.dt_out);
+    if ((flags & DTF_NAN) && ctl.status) atomicOr(ctl.status, (unsigned)HX_STATUS_NAN);
+}
+
+// ---------------------------------------------------------------------------
 // The persistent FP64 level step on 32 x 32 tiles.  One block of 1024 threads
 // per SM walks its tiles (k = blockIdx.x, blockIdx.x + gridDim.x, ...; row-major
 // over the box, so the blocks in flight share halo rows in L2).  The grown tile
@@ -2528,6 +2664,34 @@ template <class K> inline cudaError_t ensure_smem(K kernel, size_t bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// Rows per strip.  Fast form: a level of at most 20 rows a strip in one round of resident blocks takes that round
+// (8 rows at least: a strip loads four more rows than it updates); larger ones 16 rows, which leaves the blocks enough
+// rounds to even out wet and dry strips, and from 16 rounds on 32.  us per step at 12 / 16 / 32 rows: 3001 x 2500
+// 187 / 184 / 188, 8192 x 4096 762 / 744 / 727; one round against 16 rows: 1000^2 35.9 / 40.0, 1400^2 60.4 / 65.8.
+// Exact form: 12 rows (3001 x 2500 504, against 511 at 16 and 558 at 32).
+template <bool FAST>
+cudaError_t launch_march(const LevelSrc<float>& src, const Cells3<float>& uo, const Plane<float>& np,
+                         const Cells3W<float>& out, const IBox& vb, const StepCtl<float>& ctl, cudaStream_t st) {
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    const long long nx = vb.hi0 - vb.lo0 + 1, ny = vb.hi1 - vb.lo1 + 1;
+    const long long cols = (nx + kMarchCols * kMarchStrips - 1) / (kMarchCols * kMarchStrips);
+    const long long slots = (long long)sms * march_ctas(FAST);
+    long long rows = 12;
+    if (FAST) {
+        const long long bands = slots / cols > 0 ? slots / cols : 1;  // of one round
+        rows = (ny + bands - 1) / bands;
+        if (rows > 20) rows = cols * ((ny + 15) / 16) >= 16 * slots ? 32 : 16;
+        if (rows < 8) rows = 8;
+    }
+    while ((ny + rows - 1) / rows > 65535) rows *= 2;  // the grid's limit
+    const dim3 g((unsigned)cols, (unsigned)((ny + rows - 1) / rows));
+    k_hydro_march<float, FAST><<<g, kMarchN, 0, st>>>(src, uo, np, out, vb, ctl, (int)rows);
+    return cudaGetLastError();
+}
+
 // The step's kernel; nblocks receives its block count (the epilogue's partials).
 template <class R, bool FAST, class Src, bool EPI>
 cudaError_t launch_hydro_k(const Src& src, const Cells3<R>& uo, const Plane<R>& np, const Cells3W<R>& out,
@@ -2556,6 +2720,13 @@ cudaError_t launch_hydro_k(const Src& src, const Cells3<R>& uo, const Plane<R>& 
             nblocks = grid;
             return cudaGetLastError();
         }
+    }
+    if constexpr (std::is_same_v<Src, LevelSrc<float>> && !EPI) {
+        // unless strips in whole blocks would leave a fifth of the lanes without a column
+        const long long nx = vb.hi0 - vb.lo0 + 1, w = kMarchCols * kMarchStrips;
+        if (box_cells(vb) >= (FAST ? kMarchCells : kMarchCellsExact) && 4 * ((nx + w - 1) / w * w) <= 5 * nx && !fo.on &&
+            !fo.mean)
+            return launch_march<FAST>(src, uo, np, out, vb, ctl, st);
     }
     if (big_tile<R>(vb)) {
         constexpr int BX = BigTile<R>::X, BY = BigTile<R>::Y;

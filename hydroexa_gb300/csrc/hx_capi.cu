@@ -470,7 +470,8 @@ constexpr int kHostBands = 10;  // at most: a short first and last band, up to e
 constexpr int kHeadRows = 2;  // rows of the next band the flux differences of a band read (the MUSCL reach)
 // Share of the rows whose first step is split (flux differences as the rows land, the update once dt is
 // known), before a call has measured this host: on GB300 the upload of the level (40 B per cell at
-// ~210 GB/s) takes about as long as the flux work of 45% of the rows (~3.1 us per row of 8192 cells).
+// ~210 GB/s) takes about as long as the exact form's flux work on 45% of the rows (~3.4 us per row of 8192
+// cells); the fast form's (~1 us per row) fits under it whole, and its calls move towards the upper limit.
 constexpr double kSplitFrac = 0.45;
 // The split share for the next call from this call's upload time and the fused bands' time per row: the
 // split flux work should last as long as the upload (dt is known when the last rows have landed), less a

@@ -214,6 +214,10 @@ __host__ __device__ __forceinline__ bool in_f32_range(double x) {
 // correction steps issue on the FP64 pipe (GB300 issues FP64 at 1/64 of its
 // FP32 rate).  The seeds carry a relative error delta below 2^-21.5.
 //
+// The level steps form their roots and quotients in float pairs (hx_pair.cuh) or, in the exact form, on the integer
+// pipe (hx_ieee.cuh); these remain for states past the pairs' range, faces the reverse takes in FP64, the CFL rate and
+// the classic flux.
+//
 // The flux arithmetic takes ONE Newton step, whose error is of order delta^2
 // (below 2^-42 relative, typically ~2^-46): two FMAs for 1/x, three FP64
 // instructions for sqrt(x).  A face flux built from them differs from the
@@ -388,22 +392,6 @@ __device__ __forceinline__ double van_leer_div2(double p, double S) {
     return fma(r2, t, s0);
 }
 
-// Half of it, p / S, by the same steps.
-__device__ __forceinline__ double van_leer_half_div(double p, double S) {
-    const unsigned hp = (unsigned)__double2hiint(p), lp = (unsigned)__double2loint(p);
-    const unsigned hS = (unsigned)__double2hiint(S), lS = (unsigned)__double2loint(S);
-    const int ep = (int)((hp >> 20) & 0x7FFu), eS = (int)((hS >> 20) & 0x7FFu);
-    const float mp = __int_as_float((int)(0x3F800000u | ((hp & 0xFFFFFu) << 3) | (lp >> 29)));
-    const float mS = __int_as_float((int)(0x3F800000u | ((hS & 0xFFFFFu) << 3) | (lS >> 29)));
-    const float rf = f_rcp(mS), hf = mp * rf;
-    const unsigned sg = hS & 0x80000000u;
-    const double r = f64_of_f32_scaled(rf, 1023 - eS, sg);
-    const int ks = ep - eS;
-    const bool ok = (ep != 0) & ((int)((unsigned)__float_as_int(hf) >> 23) + 896 + ks >= 1);
-    const double s0 = ok ? f64_of_f32_scaled(hf, ks, sg) : 0.0;
-    return __fma_rn(r, __fma_rn(-s0, S, p), s0);
-}
-
 // ----------------------------------------------------------------------------
 // MUSCL van Leer slope (src/solvers/HydrostaticRoe.cpp:173-195), floating abs.
 // ----------------------------------------------------------------------------
@@ -428,24 +416,6 @@ template <class R, bool FAST> __host__ __device__ __forceinline__ R van_leer_slo
 #endif
         else return pos_i(p) ? (p + p) * rcp_nr(dm + dp) : R(0);
     }
-}
-
-// The fast van Leer slope (van_leer_slope<double, true>, same operations) that
-// also hands back the reciprocal 1 / (dm + dp) its reverse needs (0 where the
-// slope is 0 by a branch).
-__host__ __device__ __forceinline__ double van_leer_slope_rs(double qm, double q, double qp, double& rS) {
-    const double dm = q - qm, dp = qp - q;
-    rS = 0.0;
-    if (abs_le_bits(dp, Cst<double>::tol12_bits)) return 0.0;
-    const double p = dm * dp;
-    if (!pos_i(p)) return 0.0;
-    const double S = dm + dp;
-    rS = rcp_nr(S);
-#ifdef __CUDA_ARCH__
-    return van_leer_div2(p, S);
-#else
-    return (p + p) * rS;
-#endif
 }
 
 // ----------------------------------------------------------------------------

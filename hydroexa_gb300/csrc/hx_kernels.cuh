@@ -251,8 +251,9 @@ __device__ __forceinline__ RoePair roe_pair_state(F2 Hi, F2 Hj, F2 dh, F2 uni, F
 // denominators si + sj and 2 c enter to first order: um = u (1 - tol12 / (si + sj)), 1 / (2 c + tol12) =
 // (1 - tol12 / (2 c)) / (2 c), the second order being below 1e-18.
 //
-// Measured on the 8192^2 FP64 level: 24.6 -> 8.8 ms a step, the FP64 instructions of a cell's update 190 -> 50;
-// error of four steps against 64-bit arithmetic 8.9e-16 -> 5.8e-16 (2-norm).  The entropy-fixed faces in pairs too
+// Measured on the 8192^2 FP64 level: 24.6 -> 8.8 ms a step (8.4 with the free-surface slopes and the friction in pairs
+// too), the FP64 instructions of a cell's update 190 -> 50; error of four steps against 64-bit arithmetic 8.9e-16 ->
+// 5.8e-16 (2-norm).  The entropy-fixed faces in pairs too
 // (in FP64 out of line at first: 9.2 ms).  A first version that kept the wave
 // strengths l2 dh - d(hu), l0 dh - d(hu) in pairs lost 2^-48 (|u| / c)^2 of thin fast flow and was 5% slower.
 template <int DIR, bool REC = false>
@@ -1315,12 +1316,12 @@ __device__ __forceinline__ void hydro_tile_body(TileSmem<R, FAST, TXv, TYv>& S, 
     }
 }
 
-// Tile shapes of the level kernels, one cell per thread.  FP64 is bound by
-// FP64 issue: a 32 x 32 tile loads 1.27 cells, computes 6.4 slopes and 2.06
-// faces per cell (32 x 8: 1.69, 6.9, 2.16) and runs ~9% faster on large boxes
-// (one CTA of 1024 threads per SM).  On boxes of a few waves the four 32 x 8
-// CTAs per SM overlap each other's barriers and win, and FP32 (bound by issue
-// of every kind) always prefers them.
+// Tile shapes of the level kernels, one cell per thread.  A 32 x 32 tile loads
+// 1.27 cells, computes 6.4 slopes and 2.06 faces per cell (32 x 8: 1.69, 6.9,
+// 2.16), which pays in FP64 on large boxes (one CTA of 1024 threads per SM).
+// On boxes of a few waves the four 32 x 8 CTAs per SM overlap each other's
+// barriers and win, and FP32 levels too small to march (k_hydro_march) take
+// them.
 template <class R> struct BigTile {
     static constexpr int X = 32, Y = 32;
 };
@@ -1340,7 +1341,7 @@ struct SmallTile {
 // pipe of the few SMs it occupies, so its tiles shrink (Y = 8, 4, 2) as long as every SM still gets at most one
 // and every phase is one pass.  us per step, 32 x 8 tiles of 256 threads against these (exact / fast form): 64 x 48
 // 38.6 -> 16.3 / 18.2 -> 11.8, 128^2 38.8 -> 20.2 / 18.3 -> 14.0, 192^2 38.6 -> 28.2 / 18.2 -> 16.1; from more than
-// one tile per SM on the 256-thread tiles win, three to an SM (256^2: 50.9 against 51.9 exact, 23.0 against 28.2
+// one tile per SM on the 256-thread tiles win (256^2, three of them to an SM then: 50.9 against 51.9 exact, 23.0 against 28.2
 // fast).
 template <int Y> struct WideTile {
     static constexpr int N = (Y * (TX + 2) + 31) / 32 * 32 + (Y + 2) * TX;  // slopes, more than faces

@@ -688,11 +688,14 @@ def adjoint_summary(adj):
 
 def dominant_kernel(args, arith, cells):
     """The kernel that advances the level in the timed loop: the persistent
-    32 x 32 kernel for FP64 hydrostatic levels of 2048^2 cells and more, else
-    the tile kernel of the method and precision."""
+    32 x 32 kernel for FP64 hydrostatic levels of 933,888 cells and more, the
+    marching kernel for FP32 ones from 900,000 (fast) or 3 * 2^20 (exact)
+    cells, else the tile kernel of the method and precision."""
     form = "true" if arith else "false"
-    if (args.method, args.precision) == ("hydrostatic", "f64") and cells >= 1 << 22:
+    if (args.method, args.precision) == ("hydrostatic", "f64") and cells >= 6 * 152 * 1024:
         return "k_hydro_persist<%s>" % form
+    if (args.method, args.precision) == ("hydrostatic", "f32") and cells >= (900000 if arith else 3 << 20):
+        return "k_hydro_march<float,%s>" % form
     return "%s<%s,%s,LevelSrc>" % ("k_hydro_tile" if args.method == "hydrostatic" else "k_classic_tile",
                                    "double" if args.precision == "f64" else "float", form)
 
@@ -716,7 +719,7 @@ def profiled_traffic(profile, cells, args):
     hydrostatic persistent kernel; other variants report null."""
     per_cell = profile.get("traffic_bytes_per_cell")
     if per_cell is None or (args.method, args.precision, args.arith) != ("hydrostatic", "f64", "fast") or \
-            cells < 1 << 22:  # the capture is of the 32 x 32 tile that levels of 2048^2 cells and more take
+            cells < 1 << 22:  # the capture is of a 2048^2 level
         return None
     return per_cell * cells
 

@@ -110,8 +110,9 @@ class BaseSolver:
         R = ctypes.c_double if U.dtype == torch.float64 else ctypes.c_float
         sfx = "f64" if U.dtype == torch.float64 else "f32"
         th = (phys_params.h_grad_thresh[lev], phys_params.umag_grad_thresh[lev], phys_params.z_grad_thresh[lev])
+        U, terrain = U.contiguous(), terrain.contiguous()  # array4 keeps an address: the copies of views live to the end
         rc = getattr(capi.lib(), f"hx_tag_level_{sfx}")(
-            self.method, ctypes.byref(array4(U.contiguous())), ctypes.byref(array4(terrain.contiguous())),
+            self.method, ctypes.byref(array4(U)), ctypes.byref(array4(terrain)),
             ctypes.byref(array4(tg)), box((0, 0), (geom.nx - 1, geom.ny - 1)), R(geom.dx), R(geom.dy),
             R(time), *(R(x) for x in th), set_value, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
         capi.check(rc, "hx_tag_level")

@@ -106,7 +106,9 @@ class BaseSolver:
         stencil reads follows the level's boundary rules (the reference reads
         whatever its MultiFab ghosts hold): each ghost holds its edge cell,
         a wall's up to a momentum sign that the tags do not depend on."""
-        tg = tags if tags.dtype == torch.int8 and tags.is_contiguous() else tags.to(torch.int8).contiguous()
+        if tuple(tags.shape[-2:]) != (geom.ny, geom.nx) or tags.numel() != geom.ny * geom.nx:
+            raise RuntimeError(f"tag_cells: tags of shape {tuple(tags.shape)} on a level of {geom.ny} x {geom.nx} cells")
+        tg = tags.to(device=U.device, dtype=torch.int8).contiguous()  # the tensor itself where it already is one
         R = ctypes.c_double if U.dtype == torch.float64 else ctypes.c_float
         sfx = "f64" if U.dtype == torch.float64 else "f32"
         th = (phys_params.h_grad_thresh[lev], phys_params.umag_grad_thresh[lev], phys_params.z_grad_thresh[lev])

@@ -1,5 +1,5 @@
 """tag_cells on tensors that are not the plain case: the copies it makes of strided views must live until the kernel
-has been launched."""
+has been launched, and the kernel writes tags of the level's shape on the state's device, whatever tags the caller holds."""
 import ctypes
 import types
 import weakref
@@ -25,16 +25,20 @@ def cropped(a, dtype=torch.float64):
 @pytest.fixture
 def call(monkeypatch):
     """tag_cells on host tensors with the library call replaced by one that looks at what it is handed."""
-    seen = types.SimpleNamespace(tensors=[], arrays=None)
+    seen = types.SimpleNamespace(tensors=[], devices=set(), arrays=None)
     real = solver.array4
 
     def array4(t, *a):
         seen.tensors.append(weakref.ref(t))
+        seen.devices.add(t.device.type)
         return real(t, *a)
 
     def tag(method, U, T, tags, *rest):
         assert all(r() is not None for r in seen.tensors), "a tensor was freed before the launch"
+        assert len(seen.devices) == 1, "tensors of different devices"
         seen.arrays = [x._obj for x in (U, T, tags)]
+        a = seen.arrays[2]
+        assert (a.lo[0], a.lo[1], a.hi[0], a.hi[1]) == (0, 0, NX - 1, NY - 1), "tags of another shape"
         ctypes.memset(seen.arrays[2].p, 1, NX * NY)
         return 0
 
@@ -54,6 +58,38 @@ def test_copies_of_views_live_until_the_launch(call, dtype):
     tags = torch.zeros((NY, NX), dtype=torch.int8)
     call(tags, cropped(U, dtype), cropped(T, dtype))
     assert (tags == 1).all()
+
+
+def test_tags_of_another_device_are_copied(call):
+    """Meta tensors stand for the other device: they have no data to copy, so an attempt to copy them raises."""
+    U, T = (torch.rand((k, NY, NX), dtype=torch.float64) for k in (3, 2))
+    with pytest.raises(NotImplementedError):
+        call(torch.zeros((NY, NX), dtype=torch.int8, device="meta"), U, T)
+
+
+@pytest.mark.parametrize("shape", [(NY, NX), (1, NY, NX), (NY + 1, NX), (NY, NX + 3), (2, NY, NX), (NY, 1), (NX * NY,)])
+@pytest.mark.parametrize("dtype", [torch.int8, torch.int32])
+def test_tags_have_the_level_shape(call, shape, dtype):
+    U, T = (torch.rand((k, NY, NX), dtype=torch.float64) for k in (3, 2))
+    tags = torch.zeros(shape, dtype=dtype)
+    if shape[-2:] == (NY, NX) and tags.numel() == NY * NX:
+        call(tags, U, T)
+        assert (tags == 1).all()
+    else:
+        with pytest.raises(RuntimeError):
+            call(tags, U, T)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.int8, torch.int32])
+def test_host_tags_are_written_back(cuda, hxlib, dtype):
+    g = torch.Generator(device="cuda").manual_seed(4)
+    U, T = (torch.rand((k, NY, NX), dtype=torch.float64, device=cuda, generator=g) for k in (3, 2))
+    a, b = torch.zeros((NY, NX), dtype=torch.int8, device=cuda), torch.zeros((NY, NX), dtype=dtype)
+    a[3, 4] = b[3, 4] = 5  # what was tagged stays tagged
+    for tags in (a, b):
+        solver.HydrostaticRoe().tag_cells(tags, U, T, Geometry(NX, NY, 0.1, 0.13), 0, 0.0, TH)
+    assert torch.equal(a.cpu(), b.to(torch.int8)) and 0 < int((a == 2).sum()) < NX * NY
 
 
 @pytest.mark.gpu

@@ -285,8 +285,10 @@ __device__ __forceinline__ void roe_hydrostatic_pair(double hi, F2 ui, F2 vi, do
     const F2 &si = q.si, &sj = q.sj, &ghm = q.ghm, &cm = q.cm, &rc = q.rc, &um = q.um, &vm = q.vm, &m = q.m, &mv = q.mv;
     const F2 &A = q.A, &cB = q.cB;
     const float tc = q.tc;
-    // the signs of um - cm and um + cm, certain in float where they differ and irrelevant where they do not
-    const bool super = fabsf(um.h) > cm.h;
+    // the signs of um - cm and um + cm, by the whole pair: taken from the high parts alone, a wave that all but stands
+    // (|um| within 2^-24 of c: a bore at rest) kept |l| a of the wrong sign, up to 3e-8 of the flux (now 2^-46)
+    const F2 au = f2_abs(um);
+    const bool super = (au.h > cm.h) | ((au.h == cm.h) & (au.l > cm.l));
     F2 P, cQ, w, wl;
     bool fix0 = false, fix2 = false;
     {

@@ -569,7 +569,17 @@ __device__ __forceinline__ void hydro_face_of(bool wall, R zL, R zR, R eL, R eR,
 template <class R> __device__ __forceinline__ R flux_of(R f) { return f; }
 __device__ __forceinline__ double flux_of(F2 f) { return f64_of(f); }
 template <class R> __device__ __forceinline__ R flux_diff(R a, R b) { return a - b; }
-__device__ __forceinline__ double flux_diff(F2 a, F2 b) { return f64_of(f2_sub(a, b)); }
+// Of two fluxes in pairs, rounded once, as an FP64 difference is (f2_sub loses 2^-49 of the fluxes, and one face would
+// take from a cell what it does not give the next): the roundings of the low parts' sums go into the last places of
+// the double.  Nearly equal fluxes, where those could reach its leading places, subtract in FP64, exactly.
+static __device__ __noinline__ double flux_diff_close(F2 a, F2 b) { return f64_of(a) - f64_of(b); }
+__device__ __forceinline__ double flux_diff(F2 a, F2 b) {
+    const F2 s = f2_two_sum(a.h, -b.h), t = f2_two_sum(a.l, -b.l), v = f2_two_sum(s.l, t.h);
+    const F2 n = f2_norm(s.h, v.h);
+    double d = f64_of<true>(n, __fadd_rn(v.l, t.l));
+    if (fabsf(n.h) < __fmul_rn(0x1p-20f, fabsf(a.h))) d = flux_diff_close(a, b);
+    return d;
+}
 
 // dt of a step of the device time loop.  A collapse (min CFL bound < 1e-12,
 // HydrostaticRoe.cpp:77-80) is carried forward as a flag in the next

@@ -153,13 +153,14 @@ __device__ __forceinline__ F2 f2_div_rn(F2 a, F2 d, float y) {
 
 // h + l as a double, rounded to nearest, on the integer pipe: l in units of the high part's last place is
 // added to the bits of h (an FP64 addition costs a warp 64 issue cycles, this ~35).  0 where h is 0 or
-// subnormal, h alone below 2^-75, NaN where h is not finite.
-__device__ __forceinline__ double f64_of(F2 a) {
+// subnormal, h alone below 2^-75, NaN where h is not finite.  THIRD: with a third part e, below 2^-28 of h.
+template <bool THIRD = false> __device__ __forceinline__ double f64_of(F2 a, float e = 0.f) {
     const int b = __float_as_int(a.h);
     const unsigned m = (unsigned)b & 0x7FFFFFFFu, sg = (unsigned)b & 0x80000000u;
     // l 2^(52 - e) for a high part of exponent e (biased E = e + 127): 306 - E is that factor's biased exponent
     const float sc = __uint_as_float((306u << 23) - (m & 0x7F800000u));
     int li = __float2int_rn(__fmul_rn(__int_as_float(__float_as_int(a.l) ^ (int)sg), sc));
+    if constexpr (THIRD) li += __float2int_rn(__fmul_rn(__int_as_float(__float_as_int(e) ^ (int)sg), sc));
     if (li < 0 && (m & 0x7FFFFFu) == 0) li += li;  // below a power of two the last place is half as large
     li = m >= (52u << 23) ? li : 0;
     const unsigned long long v =

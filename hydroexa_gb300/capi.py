@@ -36,6 +36,11 @@ HX_FAST_OP_SLOPE = 2
 HX_FAST_OP_RCP_FAITHFUL = 3
 HX_FAST_OP_SQRT_FAITHFUL = 4
 HX_FAST_OP_RCBRT = 5
+HX_FAST_OP_PAIR = 6
+HX_FAST_OP_VELOCITY = 7
+HX_FAST_OP_SURFACE_SLOPE = 8
+HX_FAST_OP_VELOCITY_SLOPE = 9
+HX_FAST_OP_FRICTION = 10
 
 
 class HxError(RuntimeError):

@@ -123,7 +123,7 @@ __device__ __forceinline__ F2 f2_of(double x) {
     }
     return r;
 }
-// The same rounded: h the nearest float, so that l is at most half a place of h and the pair within 2^-50.7 of x
+// The same rounded: h the nearest float, so that l is at most half a place of h and the pair within 2^-50.6 of x
 // (root mean square; f2_of 2^-49.6), for a few more integer instructions.
 __device__ __forceinline__ F2 f2_of_rn(double x) {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
@@ -143,7 +143,8 @@ __device__ __forceinline__ F2 f2_of_rn(double x) {
     }
     return r;
 }
-// a / d for rounded pairs, y within 2^-24 of 1 / d.h: every rounding falls on the low parts, ~2^-50 of the quotient.
+// a / d for rounded pairs, y within 2^-24 of 1 / d.h: every rounding falls on the low parts (of two doubles' quotient,
+// conversions included, 2^-48.6 root mean square and 2^-45.5 at most over 10^6 random pairs).
 __device__ __forceinline__ F2 f2_div_rn(F2 a, F2 d, float y) {
     const float q = __fmul_rn(a.h, y);
     const F2 r = f2_two_sum(__fmaf_rn(-q, d.h, a.h), __fmaf_rn(-q, d.l, a.l));

@@ -716,15 +716,24 @@ int hx_debug_sqrt_f64(long n, const double* x, double* y, hx_stream_t stream);
  * face flux's), HX_FAST_OP_SLOPE (the van Leer slope of the triplets
  * x[3i], x[3i+1], x[3i+2]: x holds 3n values), HX_FAST_OP_RCP_FAITHFUL and
  * HX_FAST_OP_SQRT_FAITHFUL (the CFL rate's, within an ulp), HX_FAST_OP_RCBRT
- * (h^(-1/3) of the Manning factor, for depths within the float range).  y holds
- * n values. */
+ * (h^(-1/3), for depths within the float range).  The level step's own, in
+ * float pairs: HX_FAST_OP_PAIR (a double as a rounded pair and back),
+ * HX_FAST_OP_VELOCITY (q / h of x[2i] = h, x[2i+1] = q), HX_FAST_OP_SURFACE_SLOPE
+ * and HX_FAST_OP_VELOCITY_SLOPE (the van Leer slope of triplets of free surfaces
+ * and of velocities), HX_FAST_OP_FRICTION (the Manning factor of
+ * x[5i..5i+4] = h, hu, hv, n, dt; 1 for none).  y holds n values. */
 enum {
     HX_FAST_OP_RCP = 0,
     HX_FAST_OP_SQRT = 1,
     HX_FAST_OP_SLOPE = 2,
     HX_FAST_OP_RCP_FAITHFUL = 3,
     HX_FAST_OP_SQRT_FAITHFUL = 4,
-    HX_FAST_OP_RCBRT = 5
+    HX_FAST_OP_RCBRT = 5,
+    HX_FAST_OP_PAIR = 6,
+    HX_FAST_OP_VELOCITY = 7,
+    HX_FAST_OP_SURFACE_SLOPE = 8,
+    HX_FAST_OP_VELOCITY_SLOPE = 9,
+    HX_FAST_OP_FRICTION = 10
 };
 int hx_debug_fast_op_f64(int op, long n, const double* x, double* y, hx_stream_t stream);
 /* Test setting of the persistent level kernel's TMA staging: the next launches wait for this many bytes

@@ -415,10 +415,10 @@ template <int DIR>
 __device__ __noinline__ void face_rev_far(const FaceIn<F2>& f, const F2* lL, const F2* lR, FaceAdj<F2>& g) {
     FaceVals v;
     v.eL = f.eL; v.eR = f.eR; v.zL = f.zL; v.zR = f.zR;
-    v.uL = f64_of(f.uL); v.uR = f64_of(f.uR); v.vL = f64_of(f.vL); v.vR = f64_of(f.vR);
+    v.uL = f64_any(f.uL); v.uR = f64_any(f.uR); v.vL = f64_any(f.vL); v.vR = f64_any(f.vR);
     v.seL = 2.0 * f.seL; v.seR = 2.0 * f.seR;
-    v.suL = 2.0 * f64_of(f.suL); v.suR = 2.0 * f64_of(f.suR);
-    v.svL = 2.0 * f64_of(f.svL); v.svR = 2.0 * f64_of(f.svR);
+    v.suL = 2.0 * f64_any(f.suL); v.suR = 2.0 * f64_any(f.suR);
+    v.svL = 2.0 * f64_any(f.svL); v.svR = 2.0 * f64_any(f.svR);
     double gFL[3], gFR[3];
     for (int k = 0; k < 3; ++k) { gFL[k] = -f64_of(lL[k]); gFR[k] = f64_of(lR[k]); }
     FaceVals r{};
@@ -591,11 +591,12 @@ __device__ __forceinline__ void slope_rev(double qm, double q, double qp, double
 }
 
 // slope_rev of the fast form in pairs: dm, dp the slope's differences, rS = 1 / (dm + dp) (0 where the slope is 0 by
-// a branch), gs2 twice the slope's adjoint (what the faces hand over: the slope enters each face state with 1/2).
-__device__ __forceinline__ void slope_rev_pair(F2 dm, F2 dp, F2 rS, F2 gs2, F2& gqm, F2& gq, F2& gqp) {
+// a branch), gs2 twice the slope's adjoint (what the faces hand over: the slope enters each face state with 1/2),
+// tiny: |dp| not above tol12.
+__device__ __forceinline__ void slope_rev_pair(F2 dm, F2 dp, bool tiny, F2 rS, F2 gs2, F2& gqm, F2& gq, F2& gqp) {
     const bool flat = rS.h == 0.f;
     // r = 0: d s / d dm = 1, the mean of the one-sided derivatives
-    const bool half = flat & !(fabsf(dp.h) <= 1e-12f) & (dm.h == 0.f);
+    const bool half = flat & !tiny & (dm.h == 0.f);
     const F2 x = f2_mul(dp, rS), y = f2_mul(dm, rS);
     const F2 gdm = f2_mul(f2_mul(gs2, x), x), gdp = f2_mul(f2_mul(gs2, y), y);
     gq = f2_sel(!flat, f2_sub(gdm, gdp));
@@ -604,6 +605,36 @@ __device__ __forceinline__ void slope_rev_pair(F2 dm, F2 dp, F2 rS, F2 gs2, F2& 
     if (half) {
         gq = f2_half(gs2);
         gqm = f2_neg(gq);
+    }
+}
+// Whether half_slope took FP64 for these differences (or would have, had they one sign).
+__device__ __forceinline__ bool slope_rev_far(F2 dm, F2 dp) { return !(fabsf(dm.h + dp.h) < 0x1p120f); }
+// The reverse of those slopes, in FP64: bit qi of which says that the eta (0), u (1) or v (2) slope of a cell is one.
+// eta, u, v: the cell in its array, with neighbours st apart; fl, fr: the adjoints of the L and R face state that its
+// slope enters (planes fs apart); sp: the cell's partials (planes ss apart).
+static __device__ __noinline__ void slope_rev_fix(unsigned which, const double* eta, const F2* u, const F2* v, int st,
+                                                  const F2* fl, const F2* fr, int fs, F2* sp, int ss) {
+    for (int qi = 0; qi < 3; ++qi) {
+        if (!(which >> qi & 1u)) continue;
+        const F2* w = qi == 1 ? u : v;
+        const double dm = qi == 0 ? eta[0] - eta[-st] : f64_any(w[0]) - f64_any(w[-st]);
+        const double dp = qi == 0 ? eta[st] - eta[0] : f64_any(w[st]) - f64_any(w[0]);
+        const int qL = qi == 0 ? 0 : 2 + 2 * qi;
+        const F2 gs2 = f2_sub(fl[qL * fs], fr[(qL + 1) * fs]);
+        double x = 0.0, y = 0.0;
+        if (!abs_le_bits(dp, Cst<double>::tol12_bits)) {
+            if (dm == 0.0) {
+                x = 0.5;
+            } else if ((sbits(dm) ^ sbits(dp)) >= 0) {
+                const double rS = 1.0 / (dm + dp);
+                x = (dp * rS) * (dp * rS);
+                y = (dm * rS) * (dm * rS);
+            }
+        }
+        const F2 a = f2_neg(f2_mul(gs2, f2_of(x))), b = f2_mul(gs2, f2_of(y));
+        sp[3 * qi * ss] = a;
+        sp[(3 * qi + 1) * ss] = f2_neg(f2_add(a, b));
+        sp[(3 * qi + 2) * ss] = b;
     }
 }
 
@@ -688,6 +719,12 @@ template <class V> __device__ __forceinline__ V vzero() { return V{}; }
 __device__ __forceinline__ F2 scaled_pair(double x, int k) {
     const int hi = __double2hiint(x), m = (hi & 0x7FFFFFFF) - (k << 20);
     return f2_of(__hiloint2double(m >= (897 << 20) ? (m | (hi & (int)0x80000000)) : 0, __double2loint(x)));
+}
+
+// The adjoints of (h, hu, hv) of a cell whose velocities are boxed (cell_velocity_far).
+static __device__ __noinline__ double3 cell_rev_far(double hp, F2 u, F2 v, F2 ae, F2 au, F2 av) {
+    const double gu = f64_of(au) / hp, gv = f64_of(av) / hp;
+    return {f64_of(ae) - (gu * f64_any(u) + gv * f64_any(v)), gu, gv};
 }
 
 __device__ __forceinline__ double block_sum(double v, double* sh) {
@@ -890,16 +927,20 @@ __global__ void __launch_bounds__(kAdjThreads<FAST>) k_adj_faces(AdjArgs A) {
             // slope of this column: read as the R slope by face col (index col+1), where the face state is
             // q - s/2, and as the L slope by face col+1, where it is q + s/2; twice its adjoint is the
             // difference of the two face states' adjoints
+            [[maybe_unused]] unsigned far = 0;
             for (int qi = 0; qi < 3; ++qi) {
                 const int qL = qi == 0 ? 0 : 2 + 2 * qi, qR = qL + 1;  // eta: 0, 1; u: 4, 5; v: 6, 7
                 const V gs2 = vsub(P.fa[qL][row][col + 2], P.fa[qR][row][col + 1]);
                 V gm, g0, gp;
                 if constexpr (FAST) {
+                    const double ep = S.eta[r][c + 1] - S.eta[r][c];
                     const F2 dm = qi == 0 ? f2_of(S.eta[r][c] - S.eta[r][c - 1])
                                           : (qi == 1 ? f2_sub(S.u[r][c], S.u[r][c - 1]) : f2_sub(S.v[r][c], S.v[r][c - 1]));
-                    const F2 dp = qi == 0 ? f2_of(S.eta[r][c + 1] - S.eta[r][c])
+                    const F2 dp = qi == 0 ? f2_of(ep)
                                           : (qi == 1 ? f2_sub(S.u[r][c + 1], S.u[r][c]) : f2_sub(S.v[r][c + 1], S.v[r][c]));
-                    slope_rev_pair(dm, dp, P.rs[qi][row][col + 2], gs2, gm, g0, gp);
+                    slope_rev_pair(dm, dp, qi == 0 ? abs_le_bits(ep, Cst<double>::tol12_bits) : fabsf(dp.h) <= 1e-12f,
+                                   P.rs[qi][row][col + 2], gs2, gm, g0, gp);
+                    far |= slope_rev_far(dm, dp) ? 1u << qi : 0u;
                 } else {
                     const double(*Q)[GX] = qi == 0 ? S.eta : (qi == 1 ? S.u : S.v);
                     slope_rev(Q[r][c - 1], Q[r][c], Q[r][c + 1], 0.5 * gs2, gm, g0, gp);
@@ -907,6 +948,11 @@ __global__ void __launch_bounds__(kAdjThreads<FAST>) k_adj_faces(AdjArgs A) {
                 P.sp[3 * qi + 0][row][col + 1] = gm;  // to column col-1
                 P.sp[3 * qi + 1][row][col + 1] = g0;  // to column col
                 P.sp[3 * qi + 2][row][col + 1] = gp;  // to column col+1
+            }
+            if constexpr (FAST) {
+                if (far)
+                    slope_rev_fix(far, &S.eta[r][c], &S.u[r][c], &S.v[r][c], 1, &P.fa[0][row][col + 2],
+                                  &P.fa[0][row][col + 1], ATY * (ATX + 3), &P.sp[0][row][col + 1], ATY * (ATX + 2));
             }
         }
         __syncthreads();
@@ -1019,16 +1065,20 @@ __global__ void __launch_bounds__(kAdjThreads<FAST>) k_adj_faces(AdjArgs A) {
         for (int k = t; k < (ATY + 2) * ATX; k += AFT) {  // slope reverse, rows y0-1 .. y0+TY
             const int row = k / ATX - 1, col = k % ATX;
             const int r = row + H3, c = col + H3;
+            [[maybe_unused]] unsigned far = 0;
             for (int qi = 0; qi < 3; ++qi) {  // as in the x pass: faces row (R side) and row+1 (L side)
                 const int qL = qi == 0 ? 0 : 2 + 2 * qi, qR = qL + 1;
                 const V gs2 = vsub(P.fa[qL][row + 2][col], P.fa[qR][row + 1][col]);
                 V gm, g0, gp;
                 if constexpr (FAST) {
+                    const double ep = S.eta[r + 1][c] - S.eta[r][c];
                     const F2 dm = qi == 0 ? f2_of(S.eta[r][c] - S.eta[r - 1][c])
                                           : (qi == 1 ? f2_sub(S.u[r][c], S.u[r - 1][c]) : f2_sub(S.v[r][c], S.v[r - 1][c]));
-                    const F2 dp = qi == 0 ? f2_of(S.eta[r + 1][c] - S.eta[r][c])
+                    const F2 dp = qi == 0 ? f2_of(ep)
                                           : (qi == 1 ? f2_sub(S.u[r + 1][c], S.u[r][c]) : f2_sub(S.v[r + 1][c], S.v[r][c]));
-                    slope_rev_pair(dm, dp, P.rs[qi][row + 2][col], gs2, gm, g0, gp);
+                    slope_rev_pair(dm, dp, qi == 0 ? abs_le_bits(ep, Cst<double>::tol12_bits) : fabsf(dp.h) <= 1e-12f,
+                                   P.rs[qi][row + 2][col], gs2, gm, g0, gp);
+                    far |= slope_rev_far(dm, dp) ? 1u << qi : 0u;
                 } else {
                     const double(*Q)[GX] = qi == 0 ? S.eta : (qi == 1 ? S.u : S.v);
                     slope_rev(Q[r - 1][c], Q[r][c], Q[r + 1][c], 0.5 * gs2, gm, g0, gp);
@@ -1036,6 +1086,11 @@ __global__ void __launch_bounds__(kAdjThreads<FAST>) k_adj_faces(AdjArgs A) {
                 P.sp[3 * qi + 0][row + 1][col] = gm;
                 P.sp[3 * qi + 1][row + 1][col] = g0;
                 P.sp[3 * qi + 2][row + 1][col] = gp;
+            }
+            if constexpr (FAST) {
+                if (far)
+                    slope_rev_fix(far, &S.eta[r][c], &S.u[r][c], &S.v[r][c], GX, &P.fa[0][row + 2][col],
+                                  &P.fa[0][row + 1][col], (ATY + 3) * ATX, &P.sp[0][row + 1][col], (ATY + 2) * ATX);
             }
         }
         __syncthreads();
@@ -1118,6 +1173,12 @@ __global__ void __launch_bounds__(kAdjThreads<FAST>) k_adj_faces(AdjArgs A) {
             gh = pos_i(hp) ? lscale * f64_of(ph) : 0.0;
             ghu = lscale * f64_of(pu);
             ghv = lscale * f64_of(pv);
+            if (wet && !((S.u[r][c].h == S.u[r][c].h) & (S.v[r][c].h == S.v[r][c].h))) {
+                const double3 g = cell_rev_far(hp, S.u[r][c], S.v[r][c], ae, au, av);
+                gh = lscale * g.x;
+                ghu = lscale * g.y;
+                ghv = lscale * g.z;
+            }
         } else {
             gz = az + ae;
             double ghp = ae;

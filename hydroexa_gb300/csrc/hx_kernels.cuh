@@ -144,6 +144,12 @@ template <class R> __device__ __forceinline__ void cell_velocity(R h, R qx, R qy
     u = qx * rh;
     v = qy * rh;
 }
+// (Past the float range in FP64: such a velocity stays one, boxed.)
+static __device__ __noinline__ float4 cell_velocity_far(double h, double qx, double qy) {
+    const double rh = rcp_nr(h);
+    const F2 u = f2_any(qx * rh), v = f2_any(qy * rh);
+    return {u.h, u.l, v.h, v.l};
+}
 __device__ __forceinline__ void cell_velocity(double h, double qx, double qy, F2& u, F2& v) {
     const bool wet = gt_bits(h, Cst<double>::tol12_bits);
     F2 d = f2_of_rn(h);
@@ -152,12 +158,28 @@ __device__ __forceinline__ void cell_velocity(double h, double qx, double qy, F2
     // as near as a pair can be: the limiter of nearly equal velocities, and an adjoint through it, see this error
     u = f2_sel(wet, f2_div_rn(f2_of_rn(qx), d, y));
     v = f2_sel(wet, f2_div_rn(f2_of_rn(qy), d, y));
+    if (!(fabsf(u.h) + fabsf(v.h) < 0x1p120f)) {
+        const float4 r = cell_velocity_far(h, qx, qy);
+        u = {r.x, r.y};
+        v = {r.z, r.w};
+    }
 }
 
 // Half the van Leer slope, dm dp / (dm + dp) where the differences have one sign (van_leer_slope), as
 // dm (dp / (dm + dp)): the quotient lies in (0, 1), so nothing leaves the float range.  rs, if given,
-// receives 1 / (dm + dp) (0 where the slope is 0 by a branch).  The lanes of a warp stay together (a branch
-// per lane splits the warp, and what follows may then issue once for each part).
+// receives 1 / (dm + dp) (0 where the slope is 0 by a branch).  Where dm + dp passes 2^120 or is a NaN -- a bed with
+// voids of a float's or a double's lowest value, boxed velocities -- the slope is FP64's (rs: 0; the reverse forms its
+// own).  The lanes of a warp stay together (a branch per lane splits the warp, and what follows may then issue once for
+// each part).
+static __device__ __noinline__ double half_slope_far(double qm, double q, double qp) {
+    const double s = (q - qm) + (qp - q);
+    return pos_nan(s != s ? s : 0.5 * van_leer_slope<double, true>(qm, q, qp));
+}
+static __device__ __noinline__ float2 half_slope_far(F2 qm, F2 q, F2 qp) {
+    const F2 s = f2_any(half_slope_far(f64_any(qm), f64_any(q), f64_any(qp)));
+    return {s.h, s.l};
+}
+__device__ __forceinline__ bool slope_far(F2 S) { return !(fabsf(S.h) < 0x1p120f); }
 __device__ __forceinline__ F2 half_slope(F2 qm, F2 q, F2 qp, F2* rs = nullptr) {
     const F2 dm = f2_sub(q, qm), dp = f2_sub(qp, q);
     const bool slope = !((fabsf(dp.h) <= 1e-12f) | (__fmul_rn(dm.h, dp.h) <= 0.f));
@@ -168,14 +190,20 @@ __device__ __forceinline__ F2 half_slope(F2 qm, F2 q, F2 qp, F2* rs = nullptr) {
         const F2 S = f2_add(dm, dp);
         s = f2_sel(slope, f2_mul(dm, f2_div(dp, S, f_rcp(S.h))));
         if (rs) *rs = f2_sel(slope, f2_rcp(S));
+        if (slope & slope_far(S)) {
+            const float2 r = half_slope_far(qm, q, qp);
+            s = {r.x, r.y};
+            if (rs) *rs = F2{0.f, 0.f};
+        }
     }
     return s;
 }
 // The free surface's: its differences in FP64 (the surface hangs over a deep or high bed), rounded pairs from there,
-// within 2^-48.4 of the slope: the pressure that balances the bed follows from it.
+// within 2^-45 of the slope: the pressure that balances the bed follows from it.  (A dm below 2^-71 keeps 24 bits.)
 __device__ __forceinline__ double half_slope(double qm, double q, double qp, F2* rs = nullptr) {
-    const F2 dm = f2_of_rn(__dadd_rn(q, -qm)), dp = f2_of_rn(__dadd_rn(qp, -q));
-    const bool slope = !((fabsf(dp.h) <= 1e-12f) | (__fmul_rn(dm.h, dp.h) <= 0.f));
+    const double dpd = __dadd_rn(qp, -q);
+    const F2 dm = f2_of_rn(__dadd_rn(q, -qm)), dp = f2_of_rn(dpd);
+    const bool slope = !(abs_le_bits(dpd, Cst<double>::tol12_bits) | (__fmul_rn(dm.h, dp.h) <= 0.f));
     double s = 0.0;
     if (rs) *rs = F2{0.f, 0.f};
     const unsigned lanes = __activemask();
@@ -184,17 +212,14 @@ __device__ __forceinline__ double half_slope(double qm, double q, double qp, F2*
         const float y0 = f_rcp(S.h), y = __fmaf_rn(y0, __fmaf_rn(-S.h, y0, 1.f), y0);
         s = f64_of(f2_sel(slope, f2_mul(dm, f2_div_rn(dp, S, y))));
         if (rs) *rs = f2_sel(slope, f2_rcp(S));
+        if (slope & slope_far(S)) {
+            s = half_slope_far(qm, q, qp);
+            if (rs) *rs = F2{0.f, 0.f};
+        }
     }
     return s;
 }
 
-// The flux of roe_hydrostatic_fast for states beyond the pair form's range (depths from 2^32 m, speeds from
-// 2^24 m/s, NaN and infinities), in FP64 throughout.  Not inlined: no ordinary face comes here.
-template <int DIR>
-__device__ __noinline__ void roe_hydrostatic_far(double hi, double ui, double vi, double hj, double uj, double vj,
-                                                 double* F) {
-    roe_hydrostatic_fast<double, DIR>(hi, ui, vi, hj, uj, vj, F[0], F[1], F[2]);
-}
 // The Roe averages and wave terms of a face in pairs, from its depths Hi, Hj, their difference dh and the normal and
 // tangential velocities (0 on a dry side): see roe_hydrostatic_pair.
 struct RoePair {
@@ -256,8 +281,11 @@ __device__ __forceinline__ RoePair roe_pair_state(F2 Hi, F2 Hj, F2 dh, F2 uni, F
 // 5.8e-16 (2-norm).  The entropy-fixed faces in pairs too
 // (in FP64 out of line at first: 9.2 ms).  A first version that kept the wave
 // strengths l2 dh - d(hu), l0 dh - d(hu) in pairs lost 2^-48 (|u| / c)^2 of thin fast flow and was 5% slower.
+//
+// False, and no flux, for states beyond the pair form's range (depths from 2^32 m, speeds from 2^24 m/s, boxed ones, NaN
+// and infinities): the caller takes roe_hydrostatic_fast in FP64.
 template <int DIR, bool REC = false>
-__device__ __forceinline__ void roe_hydrostatic_pair(double hi, F2 ui, F2 vi, double hj, F2 uj, F2 vj, F2& Fm,
+__device__ __forceinline__ bool roe_hydrostatic_pair(double hi, F2 ui, F2 vi, double hj, F2 uj, F2 vj, F2& Fm,
                                                      double& Fn, F2& Ft, RoeRecVals* rv = nullptr) {
     using C = Cst<double>;
     const bool wi = ge_bits(hi, C::toldry_bits), wj = ge_bits(hj, C::toldry_bits);
@@ -272,13 +300,8 @@ __device__ __forceinline__ void roe_hydrostatic_pair(double hi, F2 ui, F2 vi, do
                         (fabsf(uni.h) < 0x1p24f) & (fabsf(uti.h) < 0x1p24f) & (fabsf(unj.h) < 0x1p24f) &
                         (fabsf(utj.h) < 0x1p24f);
         if (!in) {
-            double F[3];
-            roe_hydrostatic_far<DIR>(hi, f64_of(ui), f64_of(vi), hj, f64_of(uj), f64_of(vj), F);
             if constexpr (REC) *rv = RoeRecVals{{}, {}, {}, {}, {}, {}, {}, {}, {}, {}, RR_OTHER};
-            Fm = f2_of(F[0]);
-            Fn = F[1 + DIR];
-            Ft = f2_of(F[2 - DIR]);
-            return;
+            return false;
         }
     }
     const RoePair q = roe_pair_state(Hi, Hj, dh, uni, uti, unj, utj);
@@ -341,8 +364,17 @@ __device__ __forceinline__ void roe_hydrostatic_pair(double hi, F2 ui, F2 vi, do
     Fm = d0;
     Fn = __fma_rn(0.5 * C::half_g, __fma_rn(hj, hj, __dmul_rn(hi, hi)), f64_of(d1));
     Ft = DIR == 0 ? d2 : f2_neg(d2);
+    return true;
 }
 
+// The face in FP64.  Not inlined: no ordinary face comes here.
+template <int DIR>
+__device__ __noinline__ void hydro_face_far(double zL, double zR, double eL, double eR, double seL, double seR, F2 uL,
+                                            F2 uR, F2 suL, F2 suR, F2 vL, F2 vR, F2 svL, F2 svR, double* F) {
+    hydro_face<double, true, DIR>(false, zL, zR, eL, eR, 2.0 * seL, 2.0 * seR, f64_any(uL), f64_any(uR),
+                                  2.0 * f64_any(suL), 2.0 * f64_any(suR), f64_any(vL), f64_any(vR), 2.0 * f64_any(svL),
+                                  2.0 * f64_any(svR), F[0], F[1], F[2], F[3]);
+}
 // hydro_face of the FP64 fast form: velocities in pairs, half slopes (seL ... svR).
 template <class R, bool FAST, int DIR, bool REC = false>
 __device__ __forceinline__ void hydro_face(bool wall, double zL, double zR, double eL, double eR, double seL,
@@ -361,8 +393,16 @@ __device__ __forceinline__ void hydro_face(bool wall, double zL, double zR, doub
     const double hWu = max0_i(__dadd_rn(eW, -zW)), hWs = max0_i(__dadd_rn(eW, -zf));
     const double pW = __dmul_rn(__dadd_rn(hWu, -hWs), __dadd_rn(hWu, hWs));
     double fn;
-    roe_hydrostatic_pair<DIR, REC>(lhigh ? hH : hWs, f2_add(uL, suL), f2_add(vL, svL), lhigh ? hWs : hH,
-                                   f2_sub(uR, suR), f2_sub(vR, svR), Fm, fn, Ft, rv);
+    if (!roe_hydrostatic_pair<DIR, REC>(lhigh ? hH : hWs, f2_add(uL, suL), f2_add(vL, svL), lhigh ? hWs : hH,
+                                        f2_sub(uR, suR), f2_sub(vR, svR), Fm, fn, Ft, rv)) {
+        double F[4];
+        hydro_face_far<DIR>(zL, zR, eL, eR, seL, seR, uL, uR, suL, suR, vL, vR, svL, svR, F);
+        Fm = f2_any(F[0]);
+        Fl = pos_nan(F[1]);
+        Fr = pos_nan(F[2]);
+        Ft = f2_any(F[3]);
+        return;
+    }
     const double fw = __fma_rn(Cst<double>::half_g, pW, fn);
     Fl = lhigh ? fn : fw;
     Fr = lhigh ? fw : fn;
@@ -567,17 +607,18 @@ __device__ __forceinline__ void hydro_face_of(bool wall, R zL, R zR, R eL, R eR,
 
 // Fluxes and their differences as the update and the face arrays take them.
 template <class R> __device__ __forceinline__ R flux_of(R f) { return f; }
-__device__ __forceinline__ double flux_of(F2 f) { return f64_of(f); }
+__device__ __forceinline__ double flux_of(F2 f) { return f64_any(f); }
 template <class R> __device__ __forceinline__ R flux_diff(R a, R b) { return a - b; }
 // Of two fluxes in pairs, rounded once, as an FP64 difference is (f2_sub loses 2^-49 of the fluxes, and one face would
 // take from a cell what it does not give the next): the roundings of the low parts' sums go into the last places of
-// the double.  Nearly equal fluxes, where those could reach its leading places, subtract in FP64, exactly.
-static __device__ __noinline__ double flux_diff_close(F2 a, F2 b) { return f64_of(a) - f64_of(b); }
+// the double.  Nearly equal fluxes, where those could reach its leading places, subtract in FP64, exactly, and so do
+// fluxes past the float range (NaN here).
+static __device__ __noinline__ double flux_diff_close(F2 a, F2 b) { return pos_nan(f64_any(a) - f64_any(b)); }
 __device__ __forceinline__ double flux_diff(F2 a, F2 b) {
     const F2 s = f2_two_sum(a.h, -b.h), t = f2_two_sum(a.l, -b.l), v = f2_two_sum(s.l, t.h);
     const F2 n = f2_norm(s.h, v.h);
     double d = f64_of<true>(n, __fadd_rn(v.l, t.l));
-    if (fabsf(n.h) < __fmul_rn(0x1p-20f, fabsf(a.h))) d = flux_diff_close(a, b);
+    if (!(fabsf(n.h) >= __fmul_rn(0x1p-20f, fabsf(a.h)))) d = flux_diff_close(a, b);
     return d;
 }
 
@@ -2581,11 +2622,14 @@ __global__ void k_points(int method, long n, const R* __restrict__ st, const R* 
             if constexpr (kPairs<R, FAST>) {
                 F2 m, t;
                 R fn;
-                if (ydir) roe_hydrostatic_pair<1>(q[0], f2_of(ui), f2_of(vi), q[3], f2_of(uj), f2_of(vj), m, fn, t);
-                else roe_hydrostatic_pair<0>(q[0], f2_of(ui), f2_of(vi), q[3], f2_of(uj), f2_of(vj), m, fn, t);
-                f0 = f64_of(m);
-                f1 = ydir ? f64_of(t) : fn;
-                f2 = ydir ? fn : f64_of(t);
+                const F2 Ui = f2_any(ui), Vi = f2_any(vi), Uj = f2_any(uj), Vj = f2_any(vj);
+                if (ydir ? roe_hydrostatic_pair<1>(q[0], Ui, Vi, q[3], Uj, Vj, m, fn, t)
+                         : roe_hydrostatic_pair<0>(q[0], Ui, Vi, q[3], Uj, Vj, m, fn, t)) {
+                    f0 = f64_of(m);
+                    f1 = ydir ? f64_of(t) : fn;
+                    f2 = ydir ? fn : f64_of(t);
+                } else if (ydir) roe_hydrostatic_fast<R, 1>(q[0], ui, vi, q[3], uj, vj, f0, f1, f2);
+                else roe_hydrostatic_fast<R, 0>(q[0], ui, vi, q[3], uj, vj, f0, f1, f2);
             } else if (ydir) roe_hydrostatic_fast<R, 1>(q[0], ui, vi, q[3], uj, vj, f0, f1, f2);
             else roe_hydrostatic_fast<R, 0>(q[0], ui, vi, q[3], uj, vj, f0, f1, f2);
         }
@@ -2986,12 +3030,12 @@ template <bool FAST> __global__ void k_rcp_probe(long n, const double* x, double
         case 7: {
             F2 u, v;
             cell_velocity(x[2 * i], x[2 * i + 1], 0.0, u, v);
-            y[i] = f64_of(u);
+            y[i] = f64_any(u);
             break;
         }
         case 8: y[i] = 2.0 * half_slope(x[3 * i], x[3 * i + 1], x[3 * i + 2]); break;
         case 9:
-            y[i] = 2.0 * f64_of(half_slope(f2_of_rn(x[3 * i]), f2_of_rn(x[3 * i + 1]), f2_of_rn(x[3 * i + 2])));
+            y[i] = 2.0 * f64_any(half_slope(f2_any(x[3 * i]), f2_any(x[3 * i + 1]), f2_any(x[3 * i + 2])));
             break;
         default: {
             double fac;

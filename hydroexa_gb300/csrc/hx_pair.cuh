@@ -137,11 +137,28 @@ __device__ __forceinline__ F2 f2_of_rn(double x) {
     F2 r;
     r.l = m >= (952u << 20) ? __fmul_rn(lf, sc) : 0.f;
     r.h = __uint_as_float(f);
-    if (m - (897u << 20) >= (253u << 20)) {  // outside the normal float range
-        r.h = m >= (1150u << 20) ? __uint_as_float(0x7FFFFFFFu) : 0.f;
+    if (m - (897u << 20) >= (252u << 20)) {  // below 2^-126, from 2^126 on (whose reciprocal is no normal float)
+        r.h = m >= (1149u << 20) ? __uint_as_float(0x7FFFFFFFu) : 0.f;
         r.l = 0.f;
     }
     return r;
+}
+// Doubles past the float range in a pair's place (velocities, fluxes): a quiet NaN that holds the double's sign,
+// exponent and leading 43 bits of significand, so arithmetic on it gives NaN, and who meets a NaN takes FP64.  A NaN,
+// and one that arithmetic made (0x7FFFFFFF), reads as a positive NaN: comparisons of bit patterns take those for large.
+__device__ __forceinline__ double pos_nan(double x) {
+    const bool nan = ((unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull) > 0x7FF0000000000000ull;
+    return nan ? __hiloint2double(0x7FF80000, 0) : x;
+}
+__device__ __forceinline__ F2 f2_box(double x) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+    if (b > 0x7FF0000000000000ull) return {__uint_as_float(0x7FFFFFFFu), __uint_as_float(0xFFFFFFFFu)};
+    const unsigned long long p = (b + 0x100ull) >> 9;
+    return {__uint_as_float(((unsigned)__double2hiint(x) & 0x80000000u) | 0x7FC00000u | (unsigned)(p >> 32)),
+            __uint_as_float((unsigned)p)};
+}
+__device__ __forceinline__ F2 f2_any(double x) {
+    return ((unsigned)__double2hiint(x) & 0x7FFFFFFFu) < ((1023u + 126u) << 20) ? f2_of_rn(x) : f2_box(x);
 }
 // a / d for rounded pairs, y within 2^-24 of 1 / d.h: every rounding falls on the low parts (of two doubles' quotient,
 // conversions included, 2^-48.6 root mean square and 2^-45.5 at most over 10^6 random pairs).
@@ -172,6 +189,13 @@ template <bool THIRD = false> __device__ __forceinline__ double f64_of(F2 a, flo
         lo = 0u;
     }
     return __hiloint2double((int)hi, (int)lo);
+}
+// The double that f2_any put in a pair's place.
+__device__ __forceinline__ double f64_any(F2 a) {
+    if (a.h == a.h) return f64_of(a);
+    const unsigned h = __float_as_uint(a.h);
+    const unsigned long long p = ((unsigned long long)(h & 0x3FFFFFu) << 32) | __float_as_uint(a.l);
+    return __longlong_as_double((long long)(((unsigned long long)(h & 0x80000000u) << 32) | (p << 9)));
 }
 
 }  // namespace hx

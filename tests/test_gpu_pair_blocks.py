@@ -72,3 +72,38 @@ def test_friction_factor(cuda, hxlib):
     moving = m > 1e-12
     assert (y[~moving] == 1.0).all() and (~moving).any()
     assert rel(y[moving], want[moving]).max() <= 2.0 ** -42
+
+
+def test_cell_velocity(cuda, hxlib):
+    """q / h within the 2^-42 of a one-step FP64 reciprocal, depths, momenta and velocities past a float's range among
+    them."""
+    rng = np.random.default_rng(2)
+    h, u = wide_range(rng, N, 1e-11, 1e60, signed=False), wide_range(rng, N, 1e-12, 1e60)
+    h[: N // 2], u[: N // 2] = wide_range(rng, N // 2, 1e-11, 1e4, signed=False), wide_range(rng, N // 2, 1e-6, 1e3)
+    keep = np.abs(h * u) > 2.0 ** -70
+    x = np.stack([h, h * u], axis=1)[keep]
+    y = fast_op(hxlib, cuda, capi.HX_FAST_OP_VELOCITY, x.reshape(-1), len(x))
+    assert rel(y, x[:, 1].astype(LD) / x[:, 0]).max() <= 2.0 ** -42
+
+
+def test_slope_cut_off(cuda, hxlib):
+    """Surface differences up to 1e-12 give no slope, those above it do, to the last place."""
+    c = 1e-12
+    edge = [c, np.nextafter(c, 0.0), np.nextafter(c, 1.0), c * (1 + 2.0 ** -45), c * (1 - 2.0 ** -45), c * (1 - 2.0 ** -26)]
+    dp = np.array(edge + [-e for e in edge])
+    x = np.stack([-np.copysign(1.0, dp), np.zeros_like(dp), dp], axis=1)
+    y = fast_op(hxlib, cuda, capi.HX_FAST_OP_SURFACE_SLOPE, x.reshape(-1), len(x))
+    assert np.array_equal(y != 0.0, np.abs(dp) > c)
+
+
+@pytest.mark.parametrize("op", [capi.HX_FAST_OP_SURFACE_SLOPE, capi.HX_FAST_OP_VELOCITY_SLOPE])
+def test_slopes_past_the_float_range(cuda, hxlib, op):
+    """Differences beyond a float's range, or whose product is: FP64's bound, 2^-41."""
+    dm = np.array([3.4028234663852886e38, 1e100, 1e200, 1e39, 1e37, 2.0 ** 127, 2.0 ** 120, 2.0 ** 119, -1e100])
+    dp = np.array([1e-3, 0.25, 1e-11, 1e39, 1e5, 2.0 ** 127, 2.0 ** 126, 2.0 ** 119, 1e100])
+    dm, dp = (np.concatenate([a, -a, b, -b]) for a, b in ((dm, dp), (dp, dm)))
+    x = np.stack([-dm, np.zeros_like(dm), dp], axis=1)
+    y = fast_op(hxlib, cuda, op, x.reshape(-1), len(x))
+    live, want = slopes(x)
+    assert (y[~live] == 0.0).all() and rel(y[live], want[live]).max() <= 2.0 ** -41
+

@@ -673,33 +673,34 @@ template <class R> struct ScreenCell {
 
 // The Manning factor 2 / (1 + sqrt(1 + 4 dt g n^2 |u| / h^(4/3))) of a wet rough cell in float pairs (the FP64 fast
 // form; one-step FP64 reciprocals and roots before, 28 FP64 instructions and 2^-42): false, and no factor, where
-// |u| is not above tol12.  States past the pairs' range, and speeds at tol12 itself, take FP64.  (friction_far gives
-// 0 for no factor.)
+// |u| is not above tol12.  States, roughness and time steps past the pairs' range (the largest product is 2^115 within
+// the bounds below), and speeds at tol12 itself, take FP64.  (friction_far gives -1 for no factor.)
 static __device__ __noinline__ double friction_far(double h, double qx, double qy, double n, double dt) {
     const double modM = sqrt(qx * qx + qy * qy) / h;
-    if (modM <= Cst<double>::tol12) return 0.0;
+    if (modM <= Cst<double>::tol12) return -1.0;
     return 2.0 / (1.0 + sqrt(1.0 + 4.0 * (dt * Cst<double>::g * (n * n) * modM / (h * cbrt(h)))));
 }
 __device__ __forceinline__ bool friction_pair(double h, double qx, double qy, double n, double dt, double& fac,
                                               unsigned& pflags) {
-    const F2 H = f2_of(h), X = f2_of(qx), Y = f2_of(qy), N = f2_of(n);
+    const F2 H = f2_of(h), X = f2_of(qx), Y = f2_of(qy), N = f2_of(n), T = f2_of(dt);
     const F2 rh = f2_rcp(H);
     const F2 u = f2_mul(X, rh), v = f2_mul(Y, rh);
     const F2 m2 = f2_add(f2_mul_raw(u, u), f2_mul_raw(v, v));
     float r;
     const F2 modM = f2_sqrt(m2, r);
-    const bool in = (H.h < 0x1p32f) & (fabsf(u.h) < 0x1p24f) & (fabsf(v.h) < 0x1p24f) & (fabsf(N.h) < 0x1p24f);
+    const bool in = (H.h < 0x1p32f) & (fabsf(u.h) < 0x1p24f) & (fabsf(v.h) < 0x1p24f) & (fabsf(N.h) < 0x1p8f) &
+                    (T.h < 0x1p40f);
     if (in & (m2.h < 0.9e-24f)) return false;  // still water
     if (!(in & (m2.h > 1.1e-24f))) {
         fac = friction_far(h, qx, qy, n, dt);
-        if (fac == 0.0) return false;
+        if (fac == -1.0) return false;
         pflags |= 1u;
         return true;
     }
     pflags |= 1u;
     // 4 dt g n^2 |u| h^(-1/3) / h
     constexpr F2 k4g{39.24f, (float)(39.24 - (double)39.24f)};
-    const F2 t = f2_mul(f2_mul(f2_mul(f2_mul(k4g, f2_of(dt)), f2_mul(N, N)), modM), f2_mul(f2_rcbrt(H), rh));
+    const F2 t = f2_mul(f2_mul(f2_mul(f2_mul(k4g, T), f2_mul(N, N)), modM), f2_mul(f2_rcbrt(H), rh));
     const F2 ff = f2_sqrt(f2_add(F2{1.f, 0.f}, t), r);
     const F2 d = f2_add(F2{1.f, 0.f}, ff), q = f2_rcp(d);
     fac = f64_of(F2{q.h + q.h, q.l + q.l});

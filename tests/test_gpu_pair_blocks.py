@@ -107,3 +107,14 @@ def test_slopes_past_the_float_range(cuda, hxlib, op):
     live, want = slopes(x)
     assert (y[~live] == 0.0).all() and rel(y[live], want[live]).max() <= 2.0 ** -41
 
+
+def test_friction_past_the_float_range(cuda, hxlib):
+    """Time steps, roughness and speeds whose products pass a float's range: 2^-42, and 0 where n^2 is infinite."""
+    rng = np.random.default_rng(7)
+    n = 4096
+    h, u = wide_range(rng, n, 1e-6, 1e3, signed=False), wide_range(rng, n, 1e-6, 1e8)
+    x = np.stack([h, h * u, 0.0 * h, wide_range(rng, n, 1e-3, 1e9, signed=False), wide_range(rng, n, 1e-3, 1e60, signed=False)], axis=1)
+    y = fast_op(hxlib, cuda, capi.HX_FAST_OP_FRICTION, x.reshape(-1), n)
+    assert rel(y, friction(x)[1]).max() <= 2.0 ** -42
+    x = np.array([[1.0, 1.0, 0.0, 1e160, 1.0], [1.0, 1e-14, 0.0, 1e160, 1.0]])
+    assert fast_op(hxlib, cuda, capi.HX_FAST_OP_FRICTION, x.reshape(-1), 2).tolist() == [0.0, 1.0]

@@ -2411,7 +2411,10 @@ __device__ __forceinline__ int tag_screen(float gx, float gy, float ex, float ey
 }
 __device__ __forceinline__ float tag_f32(double x) { return f32_lead(x); }
 __device__ __forceinline__ float tag_f32(float x) { return x; }
-__device__ __forceinline__ bool tag_thin(double h) { return sbits(h) < 0x3EB0C6F7A0B5ED8Dll; }  // h < 1e-6
+// h < 1e-6, false for a NaN
+__device__ __forceinline__ bool tag_thin(double h) {
+    return (sbits(h) < 0x3EB0C6F7A0B5ED8Dll) & ((unsigned long long)sbits(h) <= 0xFFF0000000000000ull);
+}
 __device__ __forceinline__ bool tag_thin(float h) { return h < 1.0e-6f; }
 __device__ __forceinline__ bool bed_is(double z, double) { return sbits(z) == kNodataRoughBits; }  // z == -9999
 __device__ __forceinline__ bool bed_is(float z, float) { return z == -9999.0f; }

@@ -106,9 +106,11 @@ class BaseSolver:
         stencil reads follows the level's boundary rules (the reference reads
         whatever its MultiFab ghosts hold): each ghost holds its edge cell,
         a wall's up to a momentum sign that the tags do not depend on."""
-        if tuple(tags.shape[-2:]) != (geom.ny, geom.nx) or tags.numel() != geom.ny * geom.nx:
-            raise RuntimeError(f"tag_cells: tags of shape {tuple(tags.shape)} on a level of {geom.ny} x {geom.nx} cells")
-        tg = tags.to(device=U.device, dtype=torch.int8).contiguous()  # the tensor itself where it already is one
+        tg, shape = tags, (geom.ny, geom.nx)
+        if tags.shape != shape or tags.dtype != torch.int8 or tags.device != U.device or not tags.is_contiguous():
+            if tags.shape[-2:] != shape or tags.numel() != geom.ny * geom.nx:
+                raise RuntimeError(f"tag_cells: tags of shape {tuple(tags.shape)} on a level of {geom.ny} x {geom.nx} cells")
+            tg = tags.to(device=U.device, dtype=torch.int8).reshape(shape).contiguous()
         R = ctypes.c_double if U.dtype == torch.float64 else ctypes.c_float
         sfx = "f64" if U.dtype == torch.float64 else "f32"
         th = (phys_params.h_grad_thresh[lev], phys_params.umag_grad_thresh[lev], phys_params.z_grad_thresh[lev])
@@ -118,7 +120,7 @@ class BaseSolver:
             ctypes.byref(array4(tg)), box((0, 0), (geom.nx - 1, geom.ny - 1)), R(geom.dx), R(geom.dy),
             R(time), *(R(x) for x in th), set_value, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
         capi.check(rc, "hx_tag_level")
-        if tg is not tags:
+        if tg is not tags and tg.data_ptr() != tags.data_ptr():  # not a view of them
             tags.copy_(tg)
 
 

@@ -67,7 +67,7 @@ def test_tags_of_another_device_are_copied(call):
         call(torch.zeros((NY, NX), dtype=torch.int8, device="meta"), U, T)
 
 
-@pytest.mark.parametrize("shape", [(NY, NX), (1, NY, NX), (NY + 1, NX), (NY, NX + 3), (2, NY, NX), (NY, 1), (NX * NY,)])
+@pytest.mark.parametrize("shape", [(NY, NX), (1, NY, NX), (1, 1, NY, NX), (NY + 1, NX), (NY, NX + 3), (2, NY, NX), (NY, 1), (NX * NY,)])
 @pytest.mark.parametrize("dtype", [torch.int8, torch.int32])
 def test_tags_have_the_level_shape(call, shape, dtype):
     U, T = (torch.rand((k, NY, NX), dtype=torch.float64) for k in (3, 2))

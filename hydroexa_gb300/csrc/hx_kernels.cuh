@@ -1401,6 +1401,16 @@ template <int Y> struct WideTile {
     static constexpr int N = (Y * (TX + 2) + 31) / 32 * 32 + (Y + 2) * TX;  // slopes, more than faces
 };
 inline long long box_cells(const IBox& vb) { return (long long)(vb.hi0 - vb.lo0 + 1) * (long long)(vb.hi1 - vb.lo1 + 1); }
+// Whether an FP64 level or band of rows takes a persistent kernel: from kBigTileCells on, and without an epilogue (whose
+// block sums are laid out for the 32 x 8 tiles) from kPersistCells on, unless its tiles cover more than half as many rows
+// again as the 32 x 8 tiles do.  us per step, persistent kernel against those (exact / fast form): 300000 x 4 1554 / 725
+// against 800 / 325, 100000 x 10 719 / 291 against 684 / 253, 28500 x 33 617 / 219 against 580 / 206; but 200000 x 17
+// 1972 / 694 against 2192 / 762, 50000 x 65 1857 / 592 against 1841 / 625.
+inline bool persist_pays(const IBox& vb, bool epilogue = false) {
+    const long long cells = box_cells(vb), ny = vb.hi1 - vb.lo1 + 1;
+    return cells >= kBigTileCells ||
+           (!epilogue && cells >= kPersistCells && 2 * ((ny + 31) / 32 * 32) <= 3 * ((ny + 7) / 8 * 8));
+}
 template <class R> inline bool big_tile(const IBox& vb) { return BigTile<R>::Y != TY && box_cells(vb) >= kBigTileCells; }
 
 // EPI: the advance epilogue (eta and this tile's diagnostics partial, slot =
@@ -2761,8 +2771,7 @@ cudaError_t launch_hydro_k(const Src& src, const Cells3<R>& uo, const Plane<R>& 
     if constexpr (std::is_same_v<Src, LevelSrc<double>>) {
         // a whole level (or a band of its rows) on the big tile: the persistent kernel, when the stored state
         // and roughness are the level's own planes and no face arrays are asked for
-        // (with an epilogue from the size on that its block sums were laid out for)
-        if (box_cells(vb) >= (EPI ? kBigTileCells : kPersistCells) && !fo.on && !fo.mean && uo.p[0] == src.h &&
+        if (persist_pays(vb, EPI) && !fo.on && !fo.mean && uo.p[0] == src.h &&
             uo.p[1] == src.hu && uo.p[2] == src.hv && uo.js == src.pitch && uo.lo0 == 0 && uo.lo1 == 0 &&
             np.p == src.n && np.js == src.pitch && np.lo0 == 0 && np.lo1 == 0) {
             const dim3 tg = tile_grid(vb, kPX, kPY);
@@ -2915,7 +2924,7 @@ template <class R, bool FAST>
 cudaError_t launch_hydro_split(const LevelSrc<R>& src, const Cells3<R>& uo, const Plane<R>& np, const DivOut<R>& div,
                                const IBox& vb, R dx, R dy, cudaStream_t st) {
     if constexpr (std::is_same_v<R, double>) {
-        if (box_cells(vb) >= kPersistCells && uo.p[0] == src.h && uo.p[1] == src.hu && uo.p[2] == src.hv) {
+        if (persist_pays(vb) && uo.p[0] == src.h && uo.p[1] == src.hu && uo.p[2] == src.hv) {
             const dim3 tg = tile_grid(vb, kPX, kPY);
             const int ntiles = (int)(tg.x * tg.y);
             int dev = 0, sms = 0;

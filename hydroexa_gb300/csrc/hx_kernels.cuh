@@ -233,7 +233,8 @@ __device__ __forceinline__ RoePair roe_pair_state(F2 Hi, F2 Hj, F2 dh, F2 uni, F
     float r;
     const F2 si = f2_sqrt(Hi, r), sj = f2_sqrt(Hj, r);
     const F2 hs = f2_add(Hi, Hj);
-    const bool hmb = hs.h > 2e-6f;
+    constexpr F2 floor2{2e-6f, (float)(2e-6 - (double)2e-6f)};
+    const bool hmb = (hs.h > floor2.h) | ((hs.h == floor2.h) & (hs.l > floor2.l));
     // c^2 = g hm: (g / 2)(hi + hj), floored at g toldry
     F2 ghm = f2_mul(F2{4.905f, (float)(4.905 - (double)4.905f)}, hs);
     if (!hmb) ghm = F2{9.81e-6f, (float)(9.81e-6 - (double)9.81e-6f)};

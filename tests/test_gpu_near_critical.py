@@ -1,5 +1,5 @@
-"""The FP64 fast form's flux where one wave of a face stands still: |um| within 2e-7 of c, a depth jump and no entropy
-fix (a bore at rest), where the dissipation turns on the sign of um -+ c below a float's last place."""
+"""The FP64 fast form's flux where a decision falls below a float's last place: faces whose one wave stands still (|um|
+within 2e-7 of c, a depth jump and no entropy fix: a bore at rest), and mean depths at their floor."""
 import numpy as np
 import pytest
 
@@ -41,6 +41,25 @@ def test_standing_wave_faces_against_extended_precision(cuda, hxlib, ydir, sign)
     st = np.empty((n, 6))
     st[:, 0], st[:, 3] = hi, hj
     st[:, a], st[:, b], st[:, 3 + a], st[:, 3 + b] = hi * ui, hi * vi, hj * uj, hj * vj
+    normals = np.zeros((n, 2))
+    normals[:, int(ydir)] = 1.0
+    want = roe_long_double(st, normals[:, 1] != 0)
+    got = run_points(hxlib, 1, capi.HX_ARITH_FAST, st, normals, cuda).reshape(-1, 3)
+    err = (np.abs(got.astype(LD) - want) / term_scale(st)).max(axis=1)
+    assert err.max() <= 2.0 ** -42, (float(err.max()), int((err > 2.0 ** -42).sum()))
+
+
+@pytest.mark.parametrize("ydir", [False, True])
+def test_mean_depth_at_its_floor(cuda, hxlib, ydir):
+    """One wet side of about 2e-6 m, so that the mean depth passes its floor of 1e-6 m: the same bound."""
+    n = 40000
+    rng = np.random.default_rng(32)
+    st = np.zeros((n, 6))
+    h = 2e-6 * (1.0 + rng.choice([-1.0, 1.0], n) * 10.0 ** rng.uniform(-15.0, -7.0, n))
+    side = 3 * rng.integers(0, 2, n)
+    at = np.arange(n)
+    st[at, side] = h
+    st[at, side + 1], st[at, side + 2] = (h * rng.uniform(-0.01, 0.01, n) for _ in range(2))
     normals = np.zeros((n, 2))
     normals[:, int(ydir)] = 1.0
     want = roe_long_double(st, normals[:, 1] != 0)

@@ -687,12 +687,13 @@ def adjoint_summary(adj):
 
 
 def dominant_kernel(args, arith, cells):
-    """The kernel that advances the level in the timed loop: the persistent
-    32 x 32 kernel for FP64 hydrostatic levels of 933,888 cells and more, the
-    marching kernel for FP32 ones from 900,000 (fast) or 3 * 2^20 (exact)
-    cells, else the tile kernel of the method and precision."""
+    """The kernel that advances the (square) level in the timed loop: the
+    persistent 32 x 32 kernel for FP64 hydrostatic levels of 933,888 cells and
+    more (kPersistCells), the marching kernel for FP32 ones from 900,000 (fast)
+    or 3 * 2^20 (exact) cells (kMarchCells, kMarchCellsExact), else the tile
+    kernel of the method and precision."""
     form = "true" if arith else "false"
-    if (args.method, args.precision) == ("hydrostatic", "f64") and cells >= 6 * 152 * 1024:
+    if (args.method, args.precision) == ("hydrostatic", "f64") and cells >= 933888:
         return "k_hydro_persist<%s>" % form
     if (args.method, args.precision) == ("hydrostatic", "f32") and cells >= (900000 if arith else 3 << 20):
         return "k_hydro_march<float,%s>" % form

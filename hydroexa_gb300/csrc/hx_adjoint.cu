@@ -181,7 +181,7 @@ __device__ void roe_rev(double hi, double ui, double vi, double hj, double uj, d
     if (wj) { ghj += gHj; guj += gUj; gvj += gVj; }
 }
 
-// Fast form of roe_rev in FP64, for the faces that face_rev_pair leaves: roe_fwd_fast forms the quantities the
+// Fast form of roe_rev in FP64, for the faces that face_adjoint leaves: roe_fwd_fast forms the quantities the
 // reverse needs (taking the branches roe_hydrostatic_fast takes, every division of the reverse turned into a
 // product with one of five reciprocals 1/sden, 1/den, 1/cm, 1/si, 1/sj from a single rcp_nr of their product),
 // roe_rev_core runs the reverse.
@@ -714,7 +714,6 @@ __device__ __forceinline__ double vsub(double a, double b) { return a - b; }
 __device__ __forceinline__ F2 vsub(F2 a, F2 b) { return f2_sub(a, b); }
 __device__ __forceinline__ double vmul(double a, double b) { return a * b; }
 __device__ __forceinline__ F2 vmul(F2 a, F2 b) { return f2_mul(a, b); }
-template <class V> __device__ __forceinline__ V vzero() { return V{}; }
 // x 2^-k as a pair (the tile's lambda on the scale of its largest), 0 far below it.
 __device__ __forceinline__ F2 scaled_pair(double x, int k) {
     const int hi = __double2hiint(x), m = (hi & 0x7FFFFFFF) - (k << 20);

@@ -490,7 +490,7 @@ struct RoeRecVals {
     unsigned fl;
 };
 constexpr int NREC = 10;  // pairs of a RoeRecVals
-constexpr unsigned RR_WI = 1u, RR_WJ = 2u, RR_HM = 4u, RR_OTHER = 8u;
+constexpr unsigned RR_HM = 1u, RR_OTHER = 2u;
 
 // Fast form: inputs are the face depths and face velocities (the reference
 // rebuilds the velocity as (h u)/h, which equals u to an ulp).  In FP64 one

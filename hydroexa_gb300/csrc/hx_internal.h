@@ -31,13 +31,14 @@ struct IBox {
 // Boxes whose ghosts the caller fills, and the adjoint's forward steps, take the big FP64 tile kernel (32 x 32, one
 // block of 1024 threads per SM) from 2048 x 2048 cells.
 constexpr long long kBigTileCells = 1ll << 22;
-// Cells from which a level (or a band of its rows, or a multi-box level) takes a persistent kernel: six 32 x 32 tiles
-// for each of 152 SMs, below which the last round of tiles leaves too many SMs idle.  us per step, 32 x 8 tiles
-// against the persistent kernel (exact / fast form): 896^2 422 against 441 / 144 against 139, 1000^2 557 against
-// 517 / 183 against 162, 2047 x 1531 1688 against 1538 / 538 against 482.
-constexpr long long kPersistCells = 6ll * 152 * 32 * 32;
-// Cells from which an FP32 level takes the marching kernel, in the fast and the exact form: below, its strips
-// leave the GPU idle in part, and a strip's rows come one after another.  us per step, 32 x 8 tiles against it: fast 768^2 27.7 / 27.6, 1000^2 39.9 / 35.9, exact 1700 x 1500 204 / 214, 2500 x 2000 390 / 366.
+// Cells from which a level (or a band of its rows, or a multi-box level) takes a persistent kernel: measured on the 152
+// SMs of GB300, where they are six 32 x 32 tiles to an SM; below, the last round of tiles leaves too many SMs idle.
+// us per step, 32 x 8 tiles against the persistent kernel (exact / fast form): 896^2 422 against 441 / 144 against 139,
+// 1000^2 557 against 517 / 183 against 162, 2047 x 1531 1688 against 1538 / 538 against 482.
+constexpr long long kPersistCells = 933888;
+// Cells from which an FP32 level takes the marching kernel, in the fast and the exact form (measured there too): below,
+// its strips leave the GPU idle in part, and a strip's rows come one after another.  us per step, 32 x 8 tiles against
+// it: fast 768^2 27.7 / 27.6, 1000^2 39.9 / 35.9, exact 1700 x 1500 204 / 214, 2500 x 2000 390 / 366.
 constexpr long long kMarchCells = 900000, kMarchCellsExact = 3ll << 20;
 
 // Array4-like strided view: element (i, j, c) at p[(i-lo0) + (j-lo1)*js + c*ns].

@@ -354,8 +354,7 @@ __device__ __forceinline__ bool roe_hydrostatic_pair(double hi, F2 ui, F2 vi, do
         if constexpr (REC)
             *rv = RoeRecVals{si, sj, cm, q.rs, f2_half(rc), um, vm, f2_half(f2_sub(A, B)), f2_mul(mv, rc),
                              f2_half(f2_add(A, B)),
-                             (wi ? RR_WI : 0u) | (wj ? RR_WJ : 0u) | (q.hmb ? RR_HM : 0u) |
-                                 (q.rule0 & q.rule2 ? 0u : RR_OTHER)};
+                             (q.hmb ? RR_HM : 0u) | (q.rule0 & q.rule2 ? 0u : RR_OTHER)};
     }
     const F2 qi = f2_mul(Hi, uni), qj = f2_mul(Hj, unj);
     const F2 d0 = f2_sub(f2_half(f2_add(qi, qj)), w);
@@ -708,15 +707,6 @@ __device__ __forceinline__ bool friction_pair(double h, double qx, double qy, do
     return true;
 }
 
-template <class R> __device__ __forceinline__ R exact_quot(R a, R b) {
-    if constexpr (std::is_same_v<R, double>) return ieee_div(a, b);
-    else return a / b;
-}
-template <class R> __device__ __forceinline__ R exact_root(R x) {
-    if constexpr (std::is_same_v<R, double>) return ieee_sqrt(x);
-    else return sqrt(x);
-}
-
 template <class R, bool FAST, bool LINEAR, class NP = Plane<R>>
 __device__ __forceinline__ void step_cell(R o0, R o1, R o2, R dx0, R dx1, R dx2, R dy0, R dy1, R dy2, R cx, R cy,
                                           R dt, const NP& nplane, const Cells3W<R>& out, int gi, int gj,
@@ -749,15 +739,15 @@ __device__ __forceinline__ void step_cell(R o0, R o1, R o2, R dx0, R dx1, R dx2,
         if (rough) {  // the friction factor needs a rough bed
             const R qx = un[1], qy = un[2];
             if constexpr (!FAST) {
-                const R inv_h = exact_quot(R(1.0), hh);
+                const R inv_h = ieee_quot(R(1.0), hh);
                 const R uu = qx * inv_h, vv = qy * inv_h;
-                const R modM = exact_root(uu * uu + vv * vv);
+                const R modM = ieee_root(uu * uu + vv * vv);
                 if (modM > Cst<R>::tol12) {
                     pflags |= 1u;
                     const R h43 = hh * cbrt(hh);
-                    const R tt = exact_quot(dt * Cst<R>::g * nsq * modM, h43);
-                    const R ff = exact_root(R(1.0) + R(4.0) * tt);
-                    const R fac = exact_quot(R(2.0), R(1.0) + ff);
+                    const R tt = ieee_quot(dt * Cst<R>::g * nsq * modM, h43);
+                    const R ff = ieee_root(R(1.0) + R(4.0) * tt);
+                    const R fac = ieee_quot(R(2.0), R(1.0) + ff);
                     un[1] = qx * fac;
                     un[2] = qy * fac;
                 }

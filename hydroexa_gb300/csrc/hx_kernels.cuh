@@ -172,8 +172,7 @@ __device__ __forceinline__ void cell_velocity(double h, double qx, double qy, F2
 // own).  The lanes of a warp stay together (a branch per lane splits the warp, and what follows may then issue once for
 // each part).
 static __device__ __noinline__ double half_slope_far(double qm, double q, double qp) {
-    const double s = (q - qm) + (qp - q);
-    return pos_nan(s != s ? s : 0.5 * van_leer_slope<double, true>(qm, q, qp));
+    return 0.5 * van_leer_slope<double, true>(qm, q, qp);
 }
 static __device__ __noinline__ float2 half_slope_far(F2 qm, F2 q, F2 qp) {
     const F2 s = f2_any(half_slope_far(f64_any(qm), f64_any(q), f64_any(qp)));
@@ -398,8 +397,8 @@ __device__ __forceinline__ void hydro_face(bool wall, double zL, double zR, doub
         double F[4];
         hydro_face_far<DIR>(zL, zR, eL, eR, seL, seR, uL, uR, suL, suR, vL, vR, svL, svR, F);
         Fm = f2_any(F[0]);
-        Fl = pos_nan(F[1]);
-        Fr = pos_nan(F[2]);
+        Fl = F[1];
+        Fr = F[2];
         Ft = f2_any(F[3]);
         return;
     }
@@ -613,7 +612,7 @@ template <class R> __device__ __forceinline__ R flux_diff(R a, R b) { return a -
 // take from a cell what it does not give the next): the roundings of the low parts' sums go into the last places of
 // the double.  Nearly equal fluxes, where those could reach its leading places, subtract in FP64, exactly, and so do
 // fluxes past the float range (NaN here).
-static __device__ __noinline__ double flux_diff_close(F2 a, F2 b) { return pos_nan(f64_any(a) - f64_any(b)); }
+static __device__ __noinline__ double flux_diff_close(F2 a, F2 b) { return f64_any(a) - f64_any(b); }
 __device__ __forceinline__ double flux_diff(F2 a, F2 b) {
     const F2 s = f2_two_sum(a.h, -b.h), t = f2_two_sum(a.l, -b.l), v = f2_two_sum(s.l, t.h);
     const F2 n = f2_norm(s.h, v.h);

@@ -144,16 +144,11 @@ __device__ __forceinline__ F2 f2_of_rn(double x) {
     return r;
 }
 // Doubles past the float range in a pair's place (velocities, fluxes): a quiet NaN that holds the double's sign,
-// exponent and leading 43 bits of significand, so arithmetic on it gives NaN, and who meets a NaN takes FP64.  A NaN,
-// and one that arithmetic made (0x7FFFFFFF), reads as a positive NaN: comparisons of bit patterns take those for large.
-__device__ __forceinline__ double pos_nan(double x) {
-    const bool nan = ((unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull) > 0x7FF0000000000000ull;
-    return nan ? __hiloint2double(0x7FF80000, 0) : x;
-}
+// exponent and leading 43 bits of significand, so arithmetic on it gives NaN, and who meets a NaN takes FP64.  A NaN
+// keeps its sign, which comparisons of bit patterns go by; one that arithmetic made (0x7FFFFFFF) reads as a NaN too.
 __device__ __forceinline__ F2 f2_box(double x) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
-    if (b > 0x7FF0000000000000ull) return {__uint_as_float(0x7FFFFFFFu), __uint_as_float(0xFFFFFFFFu)};
-    const unsigned long long p = (b + 0x100ull) >> 9;
+    const unsigned long long p = (b > 0x7FF0000000000000ull ? 0x7FFFFFFFFFFFFFFFull : b + 0x100ull) >> 9;
     return {__uint_as_float(((unsigned)__double2hiint(x) & 0x80000000u) | 0x7FC00000u | (unsigned)(p >> 32)),
             __uint_as_float((unsigned)p)};
 }

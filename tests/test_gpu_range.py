@@ -101,3 +101,17 @@ def test_one_cell_beyond_the_float_range(cuda):
     b = lev.advance(capi.HX_METHOD_HYDROSTATIC_ROE, 1e-50, arith=FAST)
     assert torch.isfinite(a).all()
     assert (torch.abs(a - b).amax(dim=(1, 2)) <= 1e-12 * torch.abs(a).amax(dim=(1, 2))).all()
+
+
+@pytest.mark.parametrize("void", [np.inf, -np.inf, np.copysign(np.nan, -1.0)])
+@pytest.mark.parametrize("nx,ny", [(60, 40), (300, 290)])
+def test_bed_voids_that_are_not_numbers(cuda, void, nx, ny):
+    """An infinite bed (or a NaN as arithmetic makes it) under dry cells ends no run: the state stays finite, and away
+    from the voids it is the exact form's."""
+    f = scene(nx, ny, void)
+    lev = Level.from_numpy(Geometry(nx, ny, 0.1, 0.12, *SIDES), *f, device=cuda)
+    a, b = (lev.advance(capi.HX_METHOD_HYDROSTATIC_ROE, 2e-3, arith=arith) for arith in (EXACT, FAST))
+    assert torch.isfinite(a).all() and torch.isfinite(b).all() and lev.status.read() == 0
+    near = torch.nn.functional.max_pool2d(torch.from_numpy((~np.isfinite(f[3])).astype(np.float32))[None, None], 5, 1, 2)
+    away = (near[0, 0] == 0).to(cuda)
+    assert away.any() and torch.abs(a - b)[:, away].max() <= 1e-12 * torch.abs(a).max()

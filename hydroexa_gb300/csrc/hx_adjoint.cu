@@ -622,13 +622,15 @@ static __device__ __noinline__ void slope_rev_fix(unsigned which, const double* 
         const int qL = qi == 0 ? 0 : 2 + 2 * qi;
         const F2 gs2 = f2_sub(fl[qL * fs], fr[(qL + 1) * fs]);
         double x = 0.0, y = 0.0;
-        if (!abs_le_bits(dp, Cst<double>::tol12_bits)) {
+        if (gs2.h != 0.f && !abs_le_bits(dp, Cst<double>::tol12_bits)) {  // (a dry side's slope passes nothing on)
             if (dm == 0.0) {
                 x = 0.5;
-            } else if ((sbits(dm) ^ sbits(dp)) >= 0) {
-                const double rS = 1.0 / (dm + dp);
-                x = (dp * rS) * (dp * rS);
-                y = (dm * rS) * (dm * rS);
+            } else if (pos_i(dm * dp)) {
+                const double rS = 1.0 / (dm + dp);  // 0: an infinite difference, whose slope is a NaN on a dry side
+                if (rS != 0.0) {
+                    x = (dp * rS) * (dp * rS);
+                    y = (dm * rS) * (dm * rS);
+                }
             }
         }
         const F2 a = f2_neg(f2_mul(gs2, f2_of(x))), b = f2_mul(gs2, f2_of(y));

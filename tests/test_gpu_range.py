@@ -115,3 +115,15 @@ def test_bed_voids_that_are_not_numbers(cuda, void, nx, ny):
     near = torch.nn.functional.max_pool2d(torch.from_numpy((~np.isfinite(f[3])).astype(np.float32))[None, None], 5, 1, 2)
     away = (near[0, 0] == 0).to(cuda)
     assert away.any() and torch.abs(a - b)[:, away].max() <= 1e-12 * torch.abs(a).max()
+
+
+@pytest.mark.parametrize("every", [0, 2, -2])
+def test_gradient_beside_nan_voids_is_finite(cuda, every):
+    """A dry side's slope hands nothing on, whatever it is."""
+    nx, ny = 60, 40
+    h, hu, hv, z, n = (torch.from_numpy(a).to(cuda) for a in scene(nx, ny, np.copysign(np.nan, -1.0)))
+    at = (h.reshape(-1) > 0).nonzero()[::97, 0]
+    href = torch.ones((4, at.numel()), dtype=torch.float64, device=cuda)
+    p = GaugeProblem(Geometry(nx, ny, 0.1, 0.12, *SIDES), n, at, 4, 0.3, checkpoint_every=every, arith=FAST)
+    p.forward(z, h, hu, hv)
+    assert torch.isfinite(torch.stack(p.reverse(href))).all()

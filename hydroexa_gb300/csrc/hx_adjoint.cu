@@ -446,7 +446,7 @@ __device__ __forceinline__ void face_adjoint(const FaceIn<double>& f, const doub
 //
 // Of the reverse's 422 FP64 instructions per cell this leaves 64 (23% of the FP64 pipe; the block's phases and their
 // barriers bound it now).  Gradient of 90 steps on 512^2 cells, recompute and all: 51.4 -> 22.3 ms with this, 21.2 with
-// 20 warps to a tile.
+// 20 warps to a tile (22.1 with values past the float range followed).
 template <int DIR>
 __device__ __forceinline__ void face_adjoint(const FaceIn<F2>& f, const F2* lL, const F2* lR, FaceAdj<F2>& g,
                                              const RoeRecVals* rec = nullptr) {

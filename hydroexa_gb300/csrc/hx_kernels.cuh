@@ -276,10 +276,10 @@ __device__ __forceinline__ RoePair roe_pair_state(F2 Hi, F2 Hj, F2 dh, F2 uni, F
 // denominators si + sj and 2 c enter to first order: um = u (1 - tol12 / (si + sj)), 1 / (2 c + tol12) =
 // (1 - tol12 / (2 c)) / (2 c), the second order being below 1e-18.
 //
-// Measured on the 8192^2 FP64 level: 24.6 -> 8.8 ms a step (8.4 with the free-surface slopes and the friction in pairs
-// too), the FP64 instructions of a cell's update 190 -> 50; error of four steps against 64-bit arithmetic 8.9e-16 ->
-// 5.8e-16 (2-norm).  The entropy-fixed faces in pairs too
-// (in FP64 out of line at first: 9.2 ms).  A first version that kept the wave
+// Measured on the 8192^2 FP64 level: 24.6 -> 8.8 ms a step (with the free-surface slopes and the friction in pairs too, and
+// with flux differences rounded once), the FP64 instructions of a cell's update 190 -> 42; error of four steps against
+// 64-bit arithmetic 9.3e-16 -> 5.4e-16 (2-norm).  The entropy-fixed faces are in pairs too (FP64 out of line cost
+// 0.4 ms).  A first version that kept the wave
 // strengths l2 dh - d(hu), l0 dh - d(hu) in pairs lost 2^-48 (|u| / c)^2 of thin fast flow and was 5% slower.
 //
 // False, and no flux, for states beyond the pair form's range (depths from 2^32 m, speeds from 2^24 m/s, boxed ones, NaN
@@ -610,7 +610,8 @@ __device__ __forceinline__ double flux_of(F2 f) { return f64_any(f); }
 template <class R> __device__ __forceinline__ R flux_diff(R a, R b) { return a - b; }
 // Of two fluxes in pairs, rounded once, as an FP64 difference is (f2_sub loses 2^-49 of the fluxes, and one face would
 // take from a cell what it does not give the next): the roundings of the low parts' sums go into the last places of
-// the double.  Nearly equal fluxes, where those could reach its leading places, subtract in FP64, exactly, and so do
+// the double.  (8192^2: 8.47 -> 8.74 ms a step; storing doubles and subtracting those in FP64 took 9.13.)  Nearly equal
+// fluxes, where those could reach its leading places, subtract in FP64, exactly, and so do
 // fluxes past the float range (NaN here).
 static __device__ __noinline__ double flux_diff_close(F2 a, F2 b) { return f64_any(a) - f64_any(b); }
 __device__ __forceinline__ double flux_diff(F2 a, F2 b) {

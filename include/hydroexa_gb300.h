@@ -33,12 +33,14 @@
  * Precision: every entry has an _f64 form (the reference's DOUBLE build) and
  * an _f32 form (SINGLE build).  Arithmetic: HX_ARITH_EXACT repeats the
  * reference's operation order with no multiply-add contraction (bit-for-bit
- * the reference's host arithmetic up to cbrt); HX_ARITH_FAST shares
- * reciprocals and square roots between terms, takes them (and the Manning
- * factor's h^(-1/3)) from float seeds with one FP64 Newton step (within
- * 2^-42) and contracts multiply-adds,
- * agreeing with the exact form to a few 1e-15 relative per step (bound:
- * 1e-12 per step); its time step follows the exact form's to a few ulps.
+ * the reference's host arithmetic up to cbrt); HX_ARITH_FAST rearranges and
+ * contracts.  In FP64 it keeps the state, free surface, depths, their
+ * differences, the pressure and the update in doubles and computes
+ * velocities, slopes, Roe averages, dissipation and the Manning factor in
+ * pairs of floats (48 bits; states past a float's range in FP64), agreeing
+ * with the exact form to a few 1e-15 relative per step (bound: 1e-12 per
+ * step); its time step follows the exact form's to a few ulps.  Momenta below
+ * 2^-71 keep 24 bits in it.
  */
 #ifndef HYDROEXA_GB300_H
 #define HYDROEXA_GB300_H

@@ -3018,8 +3018,8 @@ cudaError_t launch_adj_forward_linear(const LevelSrc<double>& src, const Cells3<
 // which == 1) of n values, for checking them against IEEE division and sqrt.
 // The fast form's FP64 building blocks on n points: op 0 rcp_nr, 1 fast_sqrt,
 // 2 the van Leer slope of the triplet x[3i..3i+2], 3 rcp_fa, 4 fast_sqrt_fa, 5 rcbrt_nr; then those of the level step
-// in pairs: 6 f2_of_rn and back, 7 the velocity of (h, q), 8 and 9 the slopes of free surfaces and velocities,
-// 10 the Manning factor of (h, hu, hv, n, dt).
+// in pairs: 16 f2_of_rn and back, 17 the velocity of (h, q), 18 and 19 the slopes of free surfaces and velocities,
+// 20 the Manning factor of (h, hu, hv, n, dt).
 template <bool FAST> __global__ void k_rcp_probe(long n, const double* x, double* y, int which) {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -3030,15 +3030,15 @@ template <bool FAST> __global__ void k_rcp_probe(long n, const double* x, double
         case 3: y[i] = rcp_fa(x[i]); break;
         case 4: y[i] = fast_sqrt_fa(x[i]); break;
         case 5: y[i] = rcbrt_nr(x[i]); break;
-        case 6: y[i] = f64_of(f2_of_rn(x[i])); break;
-        case 7: {
+        case 16: y[i] = f64_of(f2_of_rn(x[i])); break;
+        case 17: {
             F2 u, v;
             cell_velocity(x[2 * i], x[2 * i + 1], 0.0, u, v);
             y[i] = f64_any(u);
             break;
         }
-        case 8: y[i] = 2.0 * half_slope(x[3 * i], x[3 * i + 1], x[3 * i + 2]); break;
-        case 9:
+        case 18: y[i] = 2.0 * half_slope(x[3 * i], x[3 * i + 1], x[3 * i + 2]); break;
+        case 19:
             y[i] = 2.0 * f64_any(half_slope(f2_any(x[3 * i]), f2_any(x[3 * i + 1]), f2_any(x[3 * i + 2])));
             break;
         default: {

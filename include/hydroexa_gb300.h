@@ -731,11 +731,11 @@ enum {
     HX_FAST_OP_RCP_FAITHFUL = 3,
     HX_FAST_OP_SQRT_FAITHFUL = 4,
     HX_FAST_OP_RCBRT = 5,
-    HX_FAST_OP_PAIR = 6,
-    HX_FAST_OP_VELOCITY = 7,
-    HX_FAST_OP_SURFACE_SLOPE = 8,
-    HX_FAST_OP_VELOCITY_SLOPE = 9,
-    HX_FAST_OP_FRICTION = 10
+    HX_FAST_OP_PAIR = 16,
+    HX_FAST_OP_VELOCITY = 17,
+    HX_FAST_OP_SURFACE_SLOPE = 18,
+    HX_FAST_OP_VELOCITY_SLOPE = 19,
+    HX_FAST_OP_FRICTION = 20
 };
 int hx_debug_fast_op_f64(int op, long n, const double* x, double* y, hx_stream_t stream);
 /* Test setting of the persistent level kernel's TMA staging: the next launches wait for this many bytes
